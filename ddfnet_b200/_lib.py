@@ -15,6 +15,7 @@ _lib = None
 
 F32, F16, BF16, F64 = 0, 1, 2, 3
 MUL, ADD = 0, 1
+E_TOO_LARGE = -9
 VARIANT_AUTO, VARIANT_GENERIC, VARIANT_STREAM = 0, 1, 2
 
 # every symbol include/ddf_b200.h declares

@@ -1,6 +1,8 @@
 """Builds libddf_b200.so from the CUDA sources in this directory with nvcc for
 sm_100a (cross-compiles without a GPU).  The library links the CUDA runtime
 statically and has no other dependency, so it loads in any process.
+Then builds _native.so (native.cpp, g++ against the installed torch): the host
+path of the Python operator.
 
     python -m ddfnet_b200.csrc.build [--force] [-DNAME=VALUE ...] [--out NAME]
 """
@@ -80,6 +82,36 @@ def build(force: bool = False, defines: list[str] | None = None,
     return out
 
 
+def build_native(force: bool = False) -> str:
+    """Compiles native.cpp into ddfnet_b200/_native.so."""
+    import sysconfig
+
+    import torch
+    src, out = os.path.join(HERE, "native.cpp"), os.path.join(PKG, "_native.so")
+    root = os.path.dirname(os.path.abspath(torch.__file__))
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-I{root}/include", f"-I{root}/include/torch/csrc/api/include", f"-I{cuda}/include",
+           f"-I{sysconfig.get_paths()['include']}", src, "-o", out + ".tmp", f"-L{root}/lib",
+           "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", f"-Wl,-rpath,{root}/lib"]
+    h = hashlib.sha256((" ".join(cmd) + torch.__version__).encode())
+    for p in (src, os.path.join(os.path.dirname(PKG), "include", "ddf_b200.h")):
+        with open(p, "rb") as f:
+            h.update(f.read())
+    stamp = out + ".stamp"
+    if not force and os.path.exists(out) and os.path.exists(stamp):
+        with open(stamp) as f:
+            if f.read() == h.hexdigest():
+                return out
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed on native.cpp:\n{r.stderr}")
+    os.replace(out + ".tmp", out)
+    with open(stamp, "w") as f:
+        f.write(h.hexdigest())
+    return out
+
+
 if __name__ == "__main__":
     args = sys.argv[1:]
     force = "--force" in args
@@ -89,3 +121,4 @@ if __name__ == "__main__":
     if "--out" in args:
         name = args[args.index("--out") + 1]
     print(build(force=force, defines=defs, out_name=name, verbose=verbose))
+    print(build_native(force=force))

@@ -1,0 +1,16 @@
+// Host-side entries of the band filter gradients (band_bwd.cuh).
+#pragma once
+
+#include "common.cuh"
+
+namespace ddf {
+
+// Scratch bytes of the filter gradients (0 is possible); false when the band form is not built for p.
+bool band_filters_workspace(const Problem& p, int sm_count, size_t* bytes);
+
+// kNotHandled: not built, or a tensor is not aligned for bulk copies.  `workspace` holds what
+// band_filters_workspace says.
+int band_filters(const Problem& p, const void* go, const void* x, const void* cf, const void* sf, void* gcf, void* gsf,
+                 void* workspace, int sm_count, int* fault, int device, cudaStream_t st, int* launches);
+
+}  // namespace ddf

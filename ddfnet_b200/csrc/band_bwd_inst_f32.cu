@@ -1,0 +1,3 @@
+// Band filter-gradient kernel instantiations for float elements.
+#define DDF_INST_T float
+#include "band_bwd_inst.inc"

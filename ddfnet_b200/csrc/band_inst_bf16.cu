@@ -1,0 +1,3 @@
+// Band kernel instantiations for __nv_bfloat16 elements.
+#define DDF_INST_T __nv_bfloat16
+#include "band_inst.inc"

@@ -1,6 +1,7 @@
 // Streaming filter-gradient kernels: host-side entry (see bwd_stream.cuh).
 #include <atomic>
 
+#include "band.cuh"
 #include "bwd_stream.cuh"
 
 #include "bwd_stream_impl.cuh"
@@ -149,7 +150,16 @@ int ddf_b200_backward_noalloc(const void* go, const void* x, const void* cf, con
                                 reinterpret_cast<cudaStream_t>(stream), &launches);
         if (rc != kNotHandled) return rc;
     }
-    // Outside the streaming kernel's range: the generic kernels use no scratch at all.
+    // Outside the streaming kernel's range: the band kernel where its scratch fits the array, else the
+    // generic kernels, which use no scratch at all.
+    size_t band = 0;
+    if (band_filters_workspace(p, sm_count, &band) && band <= kStaticScratchBytes) {
+        void* scratch = nullptr;
+        rc = static_scratch_address(index, &scratch);
+        if (rc) return rc;
+        return ddf_b200_backward(go, x, cf, sf, nullptr, gcf, gsf, scratch, kStaticScratchBytes, B, C, H, W, k, d, s,
+                                 combine, dtype, DDF_B200_VARIANT_AUTO, stream);
+    }
     return ddf_b200_backward(go, x, cf, sf, nullptr, gcf, gsf, nullptr, 0, B, C, H, W, k, d, s,
                              combine, dtype, DDF_B200_VARIANT_GENERIC, stream);
 }

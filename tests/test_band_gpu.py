@@ -1,0 +1,104 @@
+"""The band kernels (planes of any height and width): forward and the three gradients against the float64
+oracle at the edges of their ranges -- one row, one column, widths around a warp and at the widest band,
+a last band of one row, channel counts that the planes of a pass do not divide, H and W that the stride
+does not divide -- and non-finite values next to the padding."""
+import pytest
+import torch
+
+from tests.util import DTYPES, check_close, make_inputs, oracle_backward, oracle_forward
+
+pytestmark = pytest.mark.gpu
+
+# (B, C, H, W, k, d, s).  The gradients take the band form at any size, the forward from about three
+# million tap products up.
+SHAPES = [
+    (1, 3, 1, 9, 3, 1, 1), (2, 5, 9, 1, 3, 1, 1), (1, 300, 5, 7, 3, 1, 1), (3, 37, 9, 11, 3, 2, 1),
+    (2, 19, 5, 33, 5, 1, 1), (2, 7, 13, 31, 5, 2, 1), (1, 9, 7, 11, 3, 1, 2), (2, 33, 15, 29, 3, 1, 2),
+    (1, 8, 201, 320, 3, 1, 1),   # the widest band, a last band of one row
+    (1, 8, 200, 321, 3, 1, 1),   # wider: the generic kernels
+    (1, 70, 101, 75, 3, 2, 1), (3, 67, 50, 67, 3, 1, 1), (2, 131, 101, 75, 3, 1, 2), (1, 24, 61, 99, 5, 1, 1),
+    (1, 24, 63, 101, 5, 2, 1), (1, 40, 30, 167, 5, 2, 1), (40, 75, 17, 13, 3, 1, 1),
+]
+
+
+def _inputs(shape, dt, seed):
+    B, C, H, W, k, d, s = shape
+    dev = torch.device("cuda:0")
+    cpu = make_inputs(B, C, H, W, k, s, DTYPES[dt], seed)
+    return cpu, [t.to(dev) for t in cpu]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("dt", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("mode", ["mul", "add"])
+def test_matches_oracle(shape, dt, mode):
+    from ddfnet_b200 import _lib, ddf
+    k, d, s = shape[4:]
+    (x, cf, sf, go), dev = _inputs(shape, dt, 50 + sum(shape))
+    ts = [t.requires_grad_() for t in dev[:3]]
+    out = ddf(*ts, k, d, s, mode)
+    check_close(out, oracle_forward(x, cf, sf, k, d, s, mode), DTYPES[dt], f"forward {shape} {dt} {mode}")
+    got = torch.autograd.grad(out, ts, dev[3])
+    want = oracle_backward(go, x, cf, sf, k, d, s, mode)
+    for name, g, w in zip(("grad_x", "grad_cf", "grad_sf"), got, want):
+        check_close(g, w, DTYPES[dt], f"{name} {shape} {dt} {mode}", reduction=name != "grad_x")
+    assert _lib.load().ddf_b200_take_fault() == 0
+
+
+@pytest.mark.parametrize("shape", [(1, 70, 101, 75, 3, 2, 1), (1, 24, 63, 101, 5, 1, 1), (2, 131, 51, 75, 3, 1, 2)])
+@pytest.mark.parametrize("which", [0, 1, 2, 3])
+@pytest.mark.parametrize("dt", ["f32", "bf16"])
+def test_padding_is_skipped_not_multiplied(shape, which, dt):
+    """An infinity in one operand reaches exactly the results it reaches in the generic kernels, which
+    skip taps outside the plane."""
+    from ddfnet_b200 import ddf
+    k, d, s = shape[4:]
+    for mode in ("mul", "add"):
+        _, t = _inputs(shape, dt, 9)
+        t[which].view(-1)[::37] = float("inf")
+        res = []
+        for version in ("", "o"):
+            ts = [v.clone().requires_grad_() for v in t[:3]]
+            out = ddf(*ts, k, d, s, mode, version)
+            res.append((out, *torch.autograd.grad(out, ts, t[3])))
+        for name, a, b in zip(("out", "grad_x", "grad_cf", "grad_sf"), *res):
+            assert torch.equal(torch.isfinite(a), torch.isfinite(b)), f"{name} {mode}"
+
+
+def test_spatial_norm_inside_the_kernel():
+    from ddfnet_b200.op import ddf_sfnorm, spatial_filter_norm
+    shape = (1, 70, 101, 75, 3, 1, 1)
+    (x, cf, raw, _), dev = _inputs(shape, "f32", 3)
+    out = ddf_sfnorm(*dev[:3], 3, 1, 1, "mul", 0.7)
+    want = oracle_forward(x, cf, spatial_filter_norm(raw.double(), 3, 0.7), 3, 1, 1, "mul")
+    check_close(out, want, torch.float32, "sfnorm")
+
+
+@pytest.mark.parametrize("shape", [(4, 60, 50, 67, 3, 1, 1), (16, 75, 9, 11, 3, 1, 2)])
+def test_no_scratch_and_built_in_scratch(shape):
+    """Without a workspace the generic kernels run, as for every problem that they cover; the entry point
+    with built-in scratch gives the regular one's results."""
+    from ddfnet_b200 import _lib
+    L = _lib.load()
+    B, C, H, W, k, d, s = shape
+    (x, cf, sf, go), dev = _inputs(shape, "f32", 4)
+    want = oracle_backward(go, x, cf, sf, k, d, s, "mul")
+    xd, cfd, sfd, god = dev
+    st = torch.cuda.current_stream().cuda_stream
+    need = int(L.ddf_b200_backward_workspace(B, C, H, W, k, d, s, 0, 0, _lib.VARIANT_AUTO))
+    assert need > 0
+    ws = torch.empty(need, dtype=torch.uint8, device=xd.device)
+    got = []
+    for ptr, n in ((ws.data_ptr(), need), (None, 0)):
+        g = [torch.empty_like(t) for t in dev[:3]]
+        assert L.ddf_b200_backward(god.data_ptr(), xd.data_ptr(), cfd.data_ptr(), sfd.data_ptr(), *(t.data_ptr() for t in g),
+                                   ptr, n, B, C, H, W, k, d, s, 0, 0, _lib.VARIANT_AUTO, st) == 0
+        got.append(g)
+    g = [torch.empty_like(t) for t in dev[:3]]
+    assert L.ddf_b200_backward_noalloc(god.data_ptr(), xd.data_ptr(), cfd.data_ptr(), sfd.data_ptr(),
+                                       *(t.data_ptr() for t in g), B, C, H, W, k, d, s, 0, 0, st) == 0
+    got.append(g)
+    for gs in got:
+        for name, a, w in zip(("grad_x", "grad_cf", "grad_sf"), gs, want):
+            check_close(a, w, torch.float32, name, reduction=name != "grad_x")
+    assert all(torch.equal(a, b) for a, b in zip(got[0], got[2]))

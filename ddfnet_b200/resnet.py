@@ -18,6 +18,7 @@ import torch.nn as nn
 
 from .layout import to_channels_last
 from .modules import DDFPack, _derived
+from .nhwc import StemMaxPool
 
 
 class DDFBottleneck(nn.Module):
@@ -96,7 +97,7 @@ class DDFResNet(nn.Module):
         self.conv1 = nn.Conv2d(3, 64, 7, stride=2, padding=3, bias=False)
         self.bn1 = nn.BatchNorm2d(64)
         self.act1 = nn.ReLU(inplace=True)
-        self.maxpool = nn.MaxPool2d(3, stride=2, padding=1)
+        self.maxpool = StemMaxPool()
         self.layer1 = self._make_layer(64, layers[0], 1, kernel_combine, se_ratio)
         self.layer2 = self._make_layer(128, layers[1], 2, kernel_combine, se_ratio)
         self.layer3 = self._make_layer(256, layers[2], 2, kernel_combine, se_ratio)

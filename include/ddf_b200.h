@@ -319,6 +319,14 @@ int ddf_b200_channel_filter(const float* pooled, int n_partials, float pool_scal
                             int dtype, void* stream);
 
 /*
+ * 3 x 3 / stride 2 / padding 1 max-pooling of a channels_last tensor, x (B,H,W,C) -> y (B,(H-1)/2+1,
+ * (W-1)/2+1,C): the stem's pooling of the DDF ResNets (the reference's models use torch's).  As
+ * torch's max_pool2d, a NaN in a window is its result.  dtype F32, F16 or BF16; 16 bytes must divide
+ * a pixel's C values, x and y must be 16-byte aligned (DDF_B200_E_UNSUPPORTED otherwise).
+ */
+int ddf_b200_maxpool_nhwc(const void* x, void* y, int B, int C, int H, int W, int dtype, void* stream);
+
+/*
  * Reads and clears the per-device fault word that the streaming kernels set
  * when one of their bounded waits runs out (they then stop instead of spinning).
  * Synchronises the device.  0 = no fault recorded; otherwise a positive code

@@ -114,7 +114,7 @@ template <typename T>
 static int generic_grad_x_launch(const Problem& p, const void* go, const void* cf, const void* sf,
                                  void* gx, int sm_count, cudaStream_t st) {
     // the down-sampling layers' case has a kernel of its own (no per-tap divisions)
-    if (p.k == 3 && p.d == 1 && p.s == 2 && p.H == 2 * p.OH && p.W == 2 * p.OW && p.B <= 65535) {
+    if (p.k == 3 && p.d == 1 && p.s == 2 && p.B <= 65535) {
         constexpr int CH = 16;
         dim3 grid((unsigned)((p.OH * p.OW + 255) / 256), (unsigned)((p.C + CH - 1) / CH), (unsigned)p.B);
         if (grid.y <= 65535u) {

@@ -74,8 +74,7 @@ generic_forward(const T* __restrict__ x, const T* __restrict__ cf, const T* __re
     }
 }
 
-// grad-x for k = 3, dilation 1, stride 2, even H and W (H = 2*OH, W = 2*OW): the case of the
-// down-sampling layers.  A thread owns one OUTPUT pixel q = (qy, qx) of a sample and walks a
+// grad-x for k = 3, dilation 1, stride 2: the case of the down-sampling layers.  A thread owns one OUTPUT pixel q = (qy, qx) of a sample and walks a
 // chunk of channels; per channel it writes the 2 x 2 input pixels (2qy.., 2qx..).  With stride
 // 2 each input pixel receives only the taps whose offset has its parity -- 1, 2, 2 and 4 of
 // the nine -- so the four results need exactly nine products, and the nine spatial-filter
@@ -86,7 +85,9 @@ generic_forward(const T* __restrict__ x, const T* __restrict__ cf, const T* __re
 //   gx[2qy+1][2qx  ] = go[q]*w7[q]  + go[q+y]*w1[q+y]
 //   gx[2qy+1][2qx+1] = go[q]*w8[q]  + go[q+x]*w6[q+x] + go[q+y]*w2[q+y] + go[q+x+y]*w0[q+x+y]
 // (w_t[q] = cf[c,t] (.) sf[t,q]; neighbours outside the plane contribute nothing).
-// Same arithmetic as generic_grad_x, without its per-tap divisions and parity tests.
+// The last row of an odd H and the last column of an odd W are read by no tap: their gradient is zero.
+// Same arithmetic as generic_grad_x, without its per-tap divisions and parity tests:
+// (16,128,101x75) f32 20 us against 392.
 template <typename T, int MODE, int CH>
 __global__ void __launch_bounds__(256)
 grad_x_k3s2(const T* __restrict__ go, const T* __restrict__ cf, const T* __restrict__ sf,
@@ -98,6 +99,7 @@ grad_x_k3s2(const T* __restrict__ go, const T* __restrict__ cf, const T* __restr
     const int qy = q / p.OW, qx = q - qy * p.OW;
     const long long b = blockIdx.z;
     const bool has_x = qx + 1 < p.OW, has_y = qy + 1 < p.OH;
+    const bool odd_x = !has_x && (p.W & 1), odd_y = !has_y && (p.H & 1);
     const T* sfb = sf + b * 9 * (long long)opl + q;
     auto sfv = [&](int t, int off, bool ok) -> A { return ok ? (A)Elem<T>::load(sfb + (long long)t * opl + off) : (A)0; };
     const A s4 = sfv(4, 0, true), s5 = sfv(5, 0, true), s7 = sfv(7, 0, true), s8 = sfv(8, 0, true);
@@ -128,6 +130,15 @@ grad_x_k3s2(const T* __restrict__ go, const T* __restrict__ cf, const T* __restr
         Elem<T>::store(o + 1, r01);
         Elem<T>::store(o + p.W, r10);
         Elem<T>::store(o + p.W + 1, r11);
+        if (odd_x) {
+            Elem<T>::store(o + 2, (A)0);
+            Elem<T>::store(o + p.W + 2, (A)0);
+        }
+        if (odd_y) {
+            Elem<T>::store(o + 2 * p.W, (A)0);
+            Elem<T>::store(o + 2 * p.W + 1, (A)0);
+            if (odd_x) Elem<T>::store(o + 2 * p.W + 2, (A)0);
+        }
     }
 }
 

@@ -278,15 +278,6 @@ static bool stream_worthwhile(const Problem& p, int sm_count) {
     return planes >= sm_count && bytes >= (256ll << 10);
 }
 
-// AUTO's next choice, the band kernel, starts slower than the generic forward (barriers, filters into
-// registers, first copy: 5 us against 4 us in a graph) and runs several times faster: (4,64,57x75) f16 at
-// stride 2, 2.4M tap products: 9.4 us against 8.6; (3,256,14x14) f16 at k = 5, 3.8M: 5.0 against 10.0;
-// (2,256,200x300) f32, 276M: 85 against 655.  Against the generic gradients it wins from the smallest
-// problems on ((1,16,7x7): grad-x 5.1 us against 5.6, filters 8.0 against 11.4).
-static bool band_worthwhile(const Problem& p) {
-    return (long long)p.B * p.C * p.OH * p.OW * p.k * p.k >= 3000000ll;
-}
-
 // Forward for a checked problem: the streaming kernel where it applies, else the generic one.
 static int forward_impl(const Problem& p, const void* x, const void* cf, const void* sf, void* out,
                         int variant, void* stream) {
@@ -313,10 +304,12 @@ static int forward_impl(const Problem& p, const void* x, const void* cf, const v
             if (rc != kNotHandled) return rc;
         }
         if (variant == DDF_B200_VARIANT_STREAM) return DDF_B200_E_UNSUPPORTED;
-        if (band_worthwhile(p)) {
-            rc = run_band(BandArgs{x, cf, sf, out, p, false, di->sm_count, di->fault, di->index}, st);
-            if (rc != kNotHandled) return rc;
-        }
+        // AUTO's next choice wins over the generic kernel at every size measured, in a graph: (1,16,7x7)
+        // f16 3.6 us against 3.9, (1,256,14x14) f16 3.7 against 4.4, (2,64,29x31) f32 4.1 against 5.3,
+        // (1,16,33x31) f16 at k = 5 5.3 against 7.8, (2,256,200x300) f32 80 against 655; its gradients
+        // likewise ((1,16,7x7) f16: grad-x 4.2 against 5.3, filters 7.7 against 11.3).
+        rc = run_band(BandArgs{x, cf, sf, out, p, false, di->sm_count, di->fault, di->index}, st);
+        if (rc != kNotHandled) return rc;
     }
     return run_generic_forward(p, x, cf, sf, out, di->sm_count, st);
 }

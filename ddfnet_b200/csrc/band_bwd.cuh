@@ -96,16 +96,21 @@ band_filters_kernel(const __grid_constant__ BandBwdPlan pl) {
     const int c_hi = c_lo + pl.chunk < pl.C ? c_lo + pl.chunk : pl.C;
     const int npass = (c_hi - c_lo + G - 1) / G;
     const int y_lo = band_row<D, PH>(band * pl.groups);
-    const int y_next = band_row<D, PH>((band + 1) * pl.groups);
-    const int y_hi = y_next < pl.OH ? y_next : pl.OH;
-    const int iy_lo = y_lo * S - R * D > 0 ? y_lo * S - R * D : 0;
+    const int y_next = y_lo + band_rows<D, PH>(pl.groups);
+    int y_hi = y_next < pl.OH ? y_next : pl.OH;
+    int iy_lo = y_lo * S - R * D > 0 ? y_lo * S - R * D : 0;
     const int iy_end = (y_hi - 1) * S + R * D + 1;
-    const int iy_hi = iy_end < pl.H ? iy_end : pl.H;
+    int iy_hi = iy_end < pl.H ? iy_end : pl.H;
+    int go_row = y_lo;
+    if (D > 1 && y_lo >= pl.OH) {  // the plane ends before this group: any row will do
+        iy_lo = go_row = 0;
+        iy_hi = y_hi = 1;
+    }
     const unsigned long long xplane = (unsigned long long)pl.H * pl.W * ES;
     const unsigned long long gplane = (unsigned long long)pl.OH * pl.OW * ES;
     const unsigned long long first_plane = (unsigned long long)b * pl.C + c_lo;
     const unsigned long long x_first = first_plane * xplane + (unsigned long long)iy_lo * pl.W * ES;
-    const unsigned long long go_first = first_plane * gplane + (unsigned long long)y_lo * pl.OW * ES;
+    const unsigned long long go_first = first_plane * gplane + (unsigned long long)go_row * pl.OW * ES;
 
     if (warp == NW) {
         // ------------------------------------------------------------- producer
@@ -122,7 +127,7 @@ band_filters_kernel(const __grid_constant__ BandBwdPlan pl) {
                 const Span sx = span_prepare(BAND_DATA(slot), pl.x, x0,
                                              x0 + more * xplane + (unsigned long long)(iy_hi - iy_lo) * pl.W * ES, pl.x_total);
                 const Span sg = span_prepare(BAND_DATA(slot) + pl.go_off, pl.go, g0,
-                                             g0 + more * gplane + (unsigned long long)(y_hi - y_lo) * pl.OW * ES, pl.go_total);
+                                             g0 + more * gplane + (unsigned long long)(y_hi - go_row) * pl.OW * ES, pl.go_total);
                 mbar_arrive_expect_tx(BAND_FULL(slot), sx.bytes + sg.bytes);
                 span_issue(sx, BAND_FULL(slot));
                 span_issue(sg, BAND_FULL(slot));
@@ -195,14 +200,16 @@ band_filters_kernel(const __grid_constant__ BandBwdPlan pl) {
     unsigned long long sf2[MUL ? KK : 1][HP];  // [column-major tap][pair]
     if constexpr (MUL) {
         const T* sfb = reinterpret_cast<const T*>(pl.sf) + (long long)b * KK * opl;
+        const T* at[PH];  // a clamped address and values dropped after: see band_kernel
+#pragma unroll
+        for (int p = 0; p < PH; ++p) at[p] = p < rows_left ? sfb + (y0 + p * D) * pl.OW + x : sfb;
 #pragma unroll
         for (int t = 0; t < KK; ++t) {
             float v[PH];
 #pragma unroll
-            for (int p = 0; p < PH; ++p) {  // from a clamped address: see band_kernel
-                const bool ok = p < rows_left;
-                const float w = Elem<T>::load(sfb + (ok ? t * opl + (long long)(y0 + p * D) * pl.OW + x : 0ll));
-                v[p] = ok ? w : 0.f;
+            for (int p = 0; p < PH; ++p) {
+                const float w = Elem<T>::load(at[p] + t * opl);
+                v[p] = p < rows_left ? w : 0.f;
             }
 #pragma unroll
             for (int q = 0; q < HP; ++q) sf2[(t % K) * K + t / K][q] = f2_pack(v[q], v[q + HP]);
@@ -468,7 +475,8 @@ inline bool band_filters_split(const Problem& p, int sm_count, BandBwdSplit& s) 
     }
     if ((long long)p.B * s.bands * s.chunks > (1ll << 30)) return false;
     const int es = p.dtype == DDF_B200_F32 ? 4 : 2;
-    const long long rows = (long long)(s.groups * PH - 1) * p.s + (p.k - 1) * p.d + 1;
+    const int out_rows = s.groups % p.d == 0 ? s.groups * PH : p.d * (PH - 1) + 1;
+    const long long rows = (long long)(out_rows - 1) * p.s + (p.k - 1) * p.d + 1;
     const long long run = ((s.planes - 1) * (long long)p.H + (rows < p.H ? rows : p.H)) * p.W * es;
     return run <= (64 << 10);
 }
@@ -515,8 +523,8 @@ int band_filters_launch(const BandBwdArgs& a, cudaStream_t stream, int* launches
     pl.x_total = (unsigned long long)p.B * p.C * p.H * p.W * ES;
     pl.go_total = (unsigned long long)p.B * p.C * p.OH * p.OW * ES;
     pl.fault = a.fault;
-    const long long rows = (long long)(sp.groups * PH - 1) * S + (K - 1) * D + 1;
-    const long long grows = (long long)sp.groups * PH;
+    const long long rows = (long long)(band_rows<D, PH>(sp.groups) - 1) * S + (K - 1) * D + 1;
+    const long long grows = band_rows<D, PH>(sp.groups);
     const uint32_t xrun = (uint32_t)(((sp.planes - 1) * (long long)p.H + (rows < p.H ? rows : p.H)) * p.W * ES);
     const uint32_t grun = (uint32_t)(((sp.planes - 1) * (long long)p.OH + (grows < p.OH ? grows : p.OH)) * p.OW * ES);
     pl.off_cf = round_up(16u * kBandSlots, 128);

@@ -16,6 +16,12 @@
 // filter values stay in registers, paired (p, p + PH/2) for the two-wide FMA.  A column of the window is
 // loaded once and serves k taps of PH pixels.
 //
+// What bounds it: instruction issue and the latency of a pass at 20 warps per SM (57% of issue slots busy,
+// DRAM at 21%, shared loads at 31%), and on small problems the filters' way into registers: one pointer per
+// pixel instead of an address per value took (4,128,50x67) f16 from 17.7 to 11.3 us.  (2,256,200x300) f32:
+// 80 us, 3.1 TB/s; the generic kernel 655.  Eight pixels per thread instead of four (half the CTAs fit): 97;
+// scalar instead of two-wide FMAs: 93 (k = 5, (8,96,75x101): 50 against 58 before the pointers, 48 after).
+//
 // Zero padding.  Rows outside the plane are read from a zeroed spot of the slot (their offset is a
 // per-thread constant), columns outside are masked.  A zero times an infinite filter value would be
 // NaN where the definition skips the tap: while the filters hold anything not below kBandFilterMax
@@ -47,7 +53,7 @@ struct BandPlan {
     int planes;               // planes per unit (> 1 only when a band is the whole plane)
     int passes;               // units per (sample, band) = ceil(C / planes)
     int stage_passes;         // units whose channel filters are staged together
-    long long units;
+    int units;
     int n_slots, n_warps;
     int bwdx, norm;
     float sf_scale;
@@ -109,6 +115,11 @@ template <int K> constexpr int kBandRegs = K == 3 ? 80 : 168;
 template <int D, int PH>
 __device__ __forceinline__ int band_row(int group) { return D == 1 ? group * PH : (group / D) * (PH * D) + group % D; }
 
+// Output rows from a band's first to its last.  Bands hold whole blocks of D groups, or, where the D groups
+// of a wide plane would need more threads than a CTA has, one group.
+template <int D, int PH>
+__host__ __device__ __forceinline__ int band_rows(int groups) { return groups % D == 0 ? groups * PH : D * (PH - 1) + 1; }
+
 template <typename T, int K, int D, int S, int PH, int MODE>
 __global__ void __launch_bounds__(kBandThreads<K>, kBandCtas<K>)
 band_kernel(const __grid_constant__ BandPlan pl) {
@@ -142,21 +153,25 @@ band_kernel(const __grid_constant__ BandPlan pl) {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
-    const long long u_lo = (pl.units * (long long)blockIdx.x) / gridDim.x;
-    const long long u_hi = (pl.units * (long long)(blockIdx.x + 1)) / gridDim.x;
+    const int u_lo = (int)(((unsigned long long)pl.units * blockIdx.x) / gridDim.x);
+    const int u_hi = (int)(((unsigned long long)pl.units * (blockIdx.x + 1)) / gridDim.x);
     const unsigned long long plane_bytes = (unsigned long long)pl.H * pl.W * ES;
     // a (sample, band)'s rows
     struct Rows { int b, y_lo, iy_lo, iy_hi; };
-    auto rows_of = [&](long long seg) {
+    auto rows_of = [&](int seg) {
         Rows r;
-        r.b = (int)(seg / pl.bands);
-        const int band = (int)(seg - (long long)r.b * pl.bands);
+        r.b = seg / pl.bands;
+        const int band = seg - r.b * pl.bands;
         r.y_lo = band_row<D, PH>(band * pl.groups);
-        const int y_next = band_row<D, PH>((band + 1) * pl.groups);
+        const int y_next = r.y_lo + band_rows<D, PH>(pl.groups);
         const int y_hi = y_next < pl.OH ? y_next : pl.OH;
         r.iy_lo = r.y_lo * S - R * D > 0 ? r.y_lo * S - R * D : 0;
         const int iy_end = (y_hi - 1) * S + R * D + 1;
         r.iy_hi = iy_end < pl.H ? iy_end : pl.H;
+        if (D > 1 && r.y_lo >= pl.OH) {  // the plane ends before this group: any row will do
+            r.iy_lo = 0;
+            r.iy_hi = 1;
+        }
         return r;
     };
     auto run_start = [&](const Rows& r, int c) {
@@ -166,10 +181,10 @@ band_kernel(const __grid_constant__ BandPlan pl) {
     if (warp == NW) {
         // ------------------------------------------------------------- producer
         if (lane != 0) return;
-        long long seg = u_lo / pl.passes;
-        int pass = (int)(u_lo - seg * pl.passes);
+        int seg = u_lo / pl.passes;
+        int pass = u_lo - seg * pl.passes;
         Rows r = rows_of(seg);
-        const int n = (int)(u_hi - u_lo);
+        const int n = u_hi - u_lo;
         int issued = 0;
         bool ok = true;
         for (; issued < n; ++issued) {
@@ -214,12 +229,13 @@ band_kernel(const __grid_constant__ BandPlan pl) {
         cmask[j] = Masked<T>::mask(ix >= 0 && ix < pl.W);
     }
     const long long out_plane = (long long)pl.OH * pl.OW;
+    const int row_step = D * pl.OW;
     const uint32_t g_step = (uint32_t)((unsigned long long)G * plane_bytes);
 
     int slot = -1;
     uint32_t ph = 1;
-    long long seg = u_lo / pl.passes;
-    int pass = (int)(u_lo - seg * pl.passes);
+    int seg = u_lo / pl.passes;
+    int pass = u_lo - seg * pl.passes;
     bool dead = false;
     bool fresh = true;  // the next unit starts another (sample, band)
     Rows rw = rows_of(seg);
@@ -227,9 +243,9 @@ band_kernel(const __grid_constant__ BandPlan pl) {
     uint32_t rowoff[NR];
     unsigned long long sf2[KK][HP];  // spatial filters of this thread's pixels, [column-major tap][pair]
     int y0 = 0, rows_left = 0;
-    for (long long u = u_lo; u < u_hi;) {
+    for (int u = u_lo; u < u_hi;) {
         int npass = pl.passes - pass;
-        if (npass > u_hi - u) npass = (int)(u_hi - u);
+        if (npass > u_hi - u) npass = u_hi - u;
         if (npass > pl.stage_passes) npass = pl.stage_passes;
         const int c_lo = pass * G;
         const int c_hi = c_lo + npass * G < pl.C ? c_lo + npass * G : pl.C;
@@ -245,23 +261,38 @@ band_kernel(const __grid_constant__ BandPlan pl) {
                                 ? (uint32_t)pip * (uint32_t)plane_bytes + (uint32_t)(((iy - rw.iy_lo) * pl.W + x * S) * ES)
                                 : pl.zero_off + 16u;
             }
+            // Loads from clamped addresses and values dropped after: a load behind a branch would wait for
+            // the one before.
             const T* sfb = reinterpret_cast<const T*>(pl.sf) + (long long)rw.b * KK * out_plane;
-            big_sf = 0;
+            float sum_abs = 0.f;
 #pragma unroll
             for (int q = 0; q < HP; ++q) {
                 float v[2][KK];
-                // all loads first, from a clamped address: a load behind a branch would wait for the one before
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    const int y = y0 + D * (q + h * HP);
+                    const int p = q + h * HP;
+                    if (!pl.bwdx) {
+                        const bool ok = p < rows_left;
+                        const T* at = ok ? sfb + (y0 + D * p) * pl.OW + x : sfb;
 #pragma unroll
-                    for (int t = 0; t < KK; ++t) {
-                        const int yy = pl.bwdx ? y + D * (t / K - R) : y;
-                        const int xx = pl.bwdx ? x + D * (t % K - R) : x;
-                        const int ft = pl.bwdx ? KK - 1 - t : t;
-                        const bool ok = active && yy >= 0 && yy < pl.OH && xx >= 0 && xx < pl.OW;
-                        const float w = Elem<T>::load(sfb + (ok ? ft * out_plane + (long long)yy * pl.OW + xx : 0ll));
-                        v[h][t] = ok ? w : 0.f;
+                        for (int t = 0; t < KK; ++t) v[h][t] = Elem<T>::load(at + t * out_plane);
+                        if (!ok) {
+#pragma unroll
+                            for (int t = 0; t < KK; ++t) v[h][t] = 0.f;
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < K; ++i) {
+                            const int yy = y0 + D * (p + i - R);
+                            const bool row = p < rows_left && yy >= 0 && yy < pl.OH;
+                            const T* at = row ? sfb + (KK - 1 - i * K) * out_plane + yy * pl.OW + x : sfb;
+#pragma unroll
+                            for (int j = 0; j < K; ++j) {
+                                const bool ok = row && x + D * (j - R) >= 0 && x + D * (j - R) < pl.OW;
+                                const float w = Elem<T>::load(ok ? at + (D * (j - R) - j * out_plane) : sfb);
+                                v[h][i * K + j] = ok ? w : 0.f;
+                            }
+                        }
                     }
                 }
 #pragma unroll
@@ -282,11 +313,12 @@ band_kernel(const __grid_constant__ BandPlan pl) {
                         for (int t = 0; t < KK; ++t) v[h][t] *= inv;
                     }
 #pragma unroll
-                    for (int t = 0; t < KK; ++t) big_sf |= !(fabsf(v[h][t]) < kBandFilterMax);
+                    for (int t = 0; t < KK; ++t) sum_abs += fabsf(v[h][t]);
                 }
 #pragma unroll
                 for (int t = 0; t < KK; ++t) sf2[(t % K) * K + t / K][q] = f2_pack(v[0][t], v[1][t]);
             }
+            big_sf = !(sum_abs < kBandFilterMax);
         }
         // Channel filters of the next units as (c, c) pairs, one column of taps after the other; grad-x
         // pairs window tap (i, j) with the mirrored filter tap.
@@ -375,12 +407,14 @@ band_kernel(const __grid_constant__ BandPlan pl) {
             __syncwarp();
             if (lane == 0) mbar_arrive(BAND_EMPTY(slot));
             if (left > 0) {
+                T* o = outp;
+                float res[PH];
 #pragma unroll
-                for (int q = 0; q < HP; ++q) {
-                    float lo, hi;
-                    f2_unpack(acc2[q], lo, hi);
-                    if (q < rows_left) Elem<T>::store(outp + (long long)(q * D) * pl.OW, lo);
-                    if (q + HP < rows_left) Elem<T>::store(outp + (long long)((q + HP) * D) * pl.OW, hi);
+                for (int q = 0; q < HP; ++q) f2_unpack(acc2[q], res[q], res[q + HP]);
+#pragma unroll
+                for (int p = 0; p < PH; ++p) {
+                    if (p < rows_left) Elem<T>::store(o, res[p]);
+                    o += row_step;
                 }
             }
             outp += G * out_plane;
@@ -422,14 +456,15 @@ struct BandSplit {
 // `whole_warps`: a plane's positions are padded to whole warps.
 inline bool band_split(int B, int C, int OH, int OW, int D, int PH, int max_threads, bool whole_warps, BandSplit& s) {
     const int max_pos = max_threads - 32;  // one warp is the producer
-    if (OW < 1 || OW > max_pos / D) return false;
+    if (OW < 1 || OW > max_pos) return false;
+    const int step = OW > max_pos / D ? 1 : D;
     const int total = (OH + PH * D - 1) / (PH * D) * D;  // column groups of a plane
     // Groups per band: the fewest warps over all bands (a short last band and a half-empty last warp
     // both cost whole warps), the bigger band where equal.
-    int best = D;
+    int best = step;
     long long best_cost = -1;
-    for (int n = D; n * OW <= max_pos && n <= total; n += D) {
-        if (n * OW > 288 && n > D) break;  // two or three CTAs per SM hide one another's start
+    for (int n = step; n * OW <= max_pos && n <= total; n += D) {
+        if (n * OW > 288 && n > step) break;  // two or three CTAs per SM hide one another's start
         const int bands = (total + n - 1) / n;
         const long long cost = (long long)bands * ((n * OW + 31) / 32);
         if (best_cost < 0 || cost <= best_cost) { best = n; best_cost = cost; }
@@ -471,14 +506,16 @@ int band_launch(const BandArgs& a, cudaStream_t stream) {
     if (!band_split(p.B, p.C, p.OH, p.OW, D, PH, kBandThreads<K>, false, sp)) return kNotHandled;
     pl.bands = sp.bands; pl.groups = sp.groups; pl.planes = sp.planes; pl.n_warps = sp.warps;
     pl.passes = (p.C + sp.planes - 1) / sp.planes;
-    pl.units = (long long)p.B * sp.bands * pl.passes;
+    const long long units = (long long)p.B * sp.bands * pl.passes;
+    if (units > (1ll << 30)) return kNotHandled;
+    pl.units = (int)units;
     pl.stage_passes = kBandStage / sp.planes > 1 ? kBandStage / sp.planes : 1;
     if (pl.stage_passes > pl.passes) pl.stage_passes = pl.passes;
     pl.bwdx = a.bwdx; pl.norm = p.sf_norm; pl.sf_scale = (float)p.sf_scale;
     pl.in_total = (unsigned long long)p.B * p.C * pl.H * pl.W * ES;
     pl.fault = a.fault;
     const long long plane_bytes = (long long)pl.H * pl.W * ES;
-    const long long rows = (long long)(sp.groups * PH - 1) * S + 2 * R * D + 1;
+    const long long rows = (long long)(band_rows<D, PH>(sp.groups) - 1) * S + 2 * R * D + 1;
     const long long run = (sp.planes - 1) * plane_bytes + (rows < pl.H ? rows : pl.H) * (long long)pl.W * ES;
     if (run > (100 << 10)) return kNotHandled;
     pl.off_cf = round_up(16u * kBandSlots, 128);
@@ -494,8 +531,7 @@ int band_launch(const BandArgs& a, cudaStream_t stream) {
         if (pl.n_slots >= 3 || (ctas == 1 && pl.n_slots == 2)) break;
     }
     const long long most = (long long)ctas * a.sm_count;
-    const long long grid = pl.units < most ? pl.units : most;
-    if (pl.units / grid > (1ll << 30)) return kNotHandled;
+    const long long grid = units < most ? units : most;
     const uint32_t smem = pl.off_slot0 + (uint32_t)pl.n_slots * pl.slot_stride;
     auto kern = band_kernel<T, K, D, S, PH, MODE>;
     static std::atomic<unsigned long long> opted_in{0};

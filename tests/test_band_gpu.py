@@ -9,13 +9,14 @@ from tests.util import DTYPES, check_close, make_inputs, oracle_backward, oracle
 
 pytestmark = pytest.mark.gpu
 
-# (B, C, H, W, k, d, s).  The gradients take the band form at any size, the forward from about three
-# million tap products up.
+# (B, C, H, W, k, d, s)
 SHAPES = [
     (1, 3, 1, 9, 3, 1, 1), (2, 5, 9, 1, 3, 1, 1), (1, 300, 5, 7, 3, 1, 1), (3, 37, 9, 11, 3, 2, 1),
     (2, 19, 5, 33, 5, 1, 1), (2, 7, 13, 31, 5, 2, 1), (1, 9, 7, 11, 3, 1, 2), (2, 33, 15, 29, 3, 1, 2),
     (1, 8, 201, 320, 3, 1, 1),   # the widest band, a last band of one row
     (1, 8, 200, 321, 3, 1, 1),   # wider: the generic kernels
+    (2, 5, 33, 200, 3, 2, 1), (1, 5, 19, 299, 5, 2, 1),   # dilated, too wide for both residues in a band
+    (1, 3, 9, 320, 3, 2, 1),     # ... and a band beyond the plane's last row
     (1, 70, 101, 75, 3, 2, 1), (3, 67, 50, 67, 3, 1, 1), (2, 131, 101, 75, 3, 1, 2), (1, 24, 61, 99, 5, 1, 1),
     (1, 24, 63, 101, 5, 2, 1), (1, 40, 30, 167, 5, 2, 1), (40, 75, 17, 13, 3, 1, 1),
 ]

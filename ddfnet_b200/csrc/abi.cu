@@ -507,7 +507,7 @@ int ddf_b200_backward(const void* go, const void* x, const void* cf, const void*
         // the band form; a caller without scratch for it gets the generic kernels, which need none
         size_t band = 0;
         if (!done && allow_stream && band_filters_workspace(p, di->sm_count, &band) &&
-            (band == 0 || (workspace && workspace_bytes >= band && (reinterpret_cast<uintptr_t>(workspace) & 3u) == 0))) {
+            (band == 0 || (workspace && workspace_bytes >= band && (reinterpret_cast<uintptr_t>(workspace) & 7u) == 0))) {
             int launches = 0;
             rc = band_filters(p, go, x, cf, sf, gcf, gsf, workspace, di->sm_count, di->fault, di->index, st, &launches);
             if (rc == 0) {

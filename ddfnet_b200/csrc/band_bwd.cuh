@@ -11,7 +11,10 @@
 // there is one partial, the CTA rounds it.
 //
 // The sums over channels are compensated for float tensors, as in the generic kernels this one stands in
-// for; for the 2-byte types the final rounding is 2^13 (f16) or 2^16 (bf16) times a float's.
+// for, and their partials are doubles: relative error of gsf against 64 bits at (4,128,50x67) 4.4e-8, as the
+// generic kernel's; Kahan sums and float partials gave 5.4e-8 (and 256 us instead of 300 at (2,256,200x300);
+// the generic kernels 3230).  For the 2-byte types the final rounding is 2^13 (f16) or 2^16 (bf16) times a
+// float's, and the sums are plain: 180 us there, bound by issue as the forward is.
 //
 // Padding.  Taps outside the plane contribute nothing, whatever the other factors hold: gsf of such a tap
 // is zero by definition and stored as such; a gcf partial that is not finite in a warp at the plane's edge
@@ -33,6 +36,8 @@ template <int K> constexpr int kBandBwdChunk = K == 3 ? 64 : 24;
 template <int K> constexpr int kBandBwdPixels = K == 3 ? 4 : 2;
 constexpr int kBandBwdParts = 32;  // gsf partials per element at most (unless the chunk limit asks for more)
 
+template <typename T> using BandPart = std::conditional_t<sizeof(T) == 4, double, float>;
+
 struct BandBwdPlan {
     const void* go;
     const void* x;
@@ -40,7 +45,7 @@ struct BandBwdPlan {
     const void* sf;
     void* gcf;         // may be null
     void* gsf;         // may be null
-    float* part_sf;    // [b][chunk][t][pixel]; null: one chunk, rounded here
+    void* part_sf;     // [b][chunk][t][pixel], BandPart<T>; null: one chunk, rounded here
     float* part_cf;    // [b][band][c][t]; null likewise
     int C, H, W, OH, OW;
     int bands, groups, chunk, chunks, planes;
@@ -286,11 +291,13 @@ band_filters_kernel(const __grid_constant__ BandBwdPlan pl) {
                         for (int q = 0; q < HP; ++q) {
                             const unsigned long long prod2 = f2_mul(g2[q], f2_pack(v[S * q + k], v[S * (q + HP) + k]));
                             if constexpr (COMP) {
-                                unsigned long long y2;
-                                if constexpr (MUL) y2 = f2_fma(prod2, cp[k], lost2[t][q]);
-                                else y2 = f2_add(prod2, lost2[t][q]);
-                                const unsigned long long t2 = f2_add(gsf2[t][q], y2);
-                                lost2[t][q] = f2_fma(f2_fma(gsf2[t][q], minus1, t2), minus1, y2);
+                                // the exact error of each addition is summed apart
+                                unsigned long long v2 = prod2;
+                                if constexpr (MUL) v2 = f2_mul(prod2, cp[k]);
+                                const unsigned long long t2 = f2_add(gsf2[t][q], v2);
+                                const unsigned long long d2 = f2_fma(gsf2[t][q], minus1, t2);
+                                const unsigned long long e2 = f2_fma(f2_fma(d2, minus1, t2), minus1, gsf2[t][q]);
+                                lost2[t][q] = f2_add(lost2[t][q], f2_add(e2, f2_fma(d2, minus1, v2)));
                                 gsf2[t][q] = t2;
                             } else {
                                 if constexpr (MUL) gsf2[t][q] = f2_fma(prod2, cp[k], gsf2[t][q]);
@@ -363,35 +370,34 @@ band_filters_kernel(const __grid_constant__ BandBwdPlan pl) {
         }
     }
     if (pl.gsf != nullptr) {
-        float* ps = pl.part_sf == nullptr ? nullptr : pl.part_sf + ((long long)b * pl.chunks + chunk_i) * KK * opl;
+        using P = BandPart<T>;
+        P* ps = pl.part_sf == nullptr
+                    ? nullptr
+                    : reinterpret_cast<P*>(pl.part_sf) + ((long long)b * pl.chunks + chunk_i) * KK * opl;
         T* os = reinterpret_cast<T*>(pl.gsf) + (long long)b * KK * opl;
-        auto put = [&](long long o, float v) {
+        auto put = [&](long long o, P v) {
             if (ps != nullptr) ps[o] = v;
-            else Elem<T>::store(os + o, v);
+            else Elem<T>::store(os + o, (float)v);
         };
         // Several planes per pass: a band is then the whole plane, and the planes' sums meet in the slots
         // (every copy has landed and been read).
-        const uint32_t meet = BAND_DATA(0) + 4u * (uint32_t)(pip * KK * (int)opl);
+        P* meet = reinterpret_cast<P*>(smem_raw + pl.off_slot0 + kBandGuard);
 #pragma unroll
         for (int t = 0; t < KK; ++t) {  // column-major tap
             const int ft = (t % K) * K + t / K;
 #pragma unroll
             for (int q = 0; q < HP; ++q) {
-                float v[2];
-                f2_unpack(gsf2[t][q], v[0], v[1]);
-                if constexpr (COMP) {
-                    float l0, l1;
-                    f2_unpack(lost2[t][q], l0, l1);
-                    v[0] += l0;
-                    v[1] += l1;
-                }
+                float v0, v1, l0 = 0.f, l1 = 0.f;
+                f2_unpack(gsf2[t][q], v0, v1);
+                if constexpr (COMP) f2_unpack(lost2[t][q], l0, l1);
+                const P v[2] = {(P)v0 + (P)l0, (P)v1 + (P)l1};
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int p = q + h * HP;
                     if (p < rows_left) {
                         const long long o = ft * opl + (long long)(y0 + p * D) * pl.OW + x;
-                        const float r = inside(t / K, t % K, p) ? v[h] : 0.f;
-                        if (G > 1) sts32(meet + 4u * (uint32_t)o, __float_as_uint(r));
+                        const P r = inside(t / K, t % K, p) ? v[h] : (P)0;
+                        if (G > 1) meet[pip * KK * (int)opl + (int)o] = r;
                         else put(o, r);
                     }
                 }
@@ -401,8 +407,8 @@ band_filters_kernel(const __grid_constant__ BandBwdPlan pl) {
             band_sync(NW * 32);
             const int n = KK * (int)opl;
             for (int e = tid; e < n; e += NW * 32) {
-                CompSum<float> tot;
-                for (int g = 0; g < G; ++g) tot.add(ldsf(BAND_DATA(0) + 4u * (uint32_t)(g * n + e)));
+                CompSum<P> tot;
+                for (int g = 0; g < G; ++g) tot.add(meet[g * n + e]);
                 put(e, tot.value());
             }
         }
@@ -412,34 +418,36 @@ band_filters_kernel(const __grid_constant__ BandBwdPlan pl) {
 #undef BAND_DATA
 }
 
-// out[s][e] = sum over the partials part[s][0 .. n_part-1][e], fixed order, compensated; the first
-// `sf_blocks` blocks do gsf, the others gcf.
-template <typename T>
-__global__ void __launch_bounds__(256)
-band_reduce_kernel(const float* __restrict__ part_sf, T* __restrict__ gsf, int n_sf, long long sf_size,
-                   const float* __restrict__ part_cf, T* __restrict__ gcf, int n_cf, long long cf_size, int B,
-                   int sf_blocks) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const bool sf = (int)blockIdx.x < sf_blocks;
-    const float* part = sf ? part_sf : part_cf;
-    T* out = sf ? gsf : gcf;
-    const int n = sf ? n_sf : n_cf;
-    const long long size = sf ? sf_size : cf_size;
-    const long long first = ((long long)blockIdx.x - (sf ? 0 : sf_blocks)) * 256 + threadIdx.x;
-    const long long step = (long long)(sf ? sf_blocks : gridDim.x - sf_blocks) * 256;
+// out[s][e] = sum over the partials part[s][0 .. n-1][e], fixed order, compensated, from element `first` on.
+template <typename T, typename P>
+__device__ __forceinline__ void band_reduce(const P* __restrict__ part, T* __restrict__ out, int n, long long size, int B,
+                                            long long first, long long step) {
     for (long long e = first; e < size * B; e += step) {
         const long long s = e / size;
-        const float* src = part + s * n * size + (e - s * size);
-        CompSum<float> tot;
+        const P* src = part + s * n * size + (e - s * size);
+        CompSum<P> tot;
         for (int j0 = 0; j0 < n; j0 += 8) {  // eight loads in flight
-            float v[8];
+            P v[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = j0 + u < n ? __ldg(src + (long long)(j0 + u) * size) : 0.f;
+            for (int u = 0; u < 8; ++u) v[u] = j0 + u < n ? __ldg(src + (long long)(j0 + u) * size) : (P)0;
 #pragma unroll
             for (int u = 0; u < 8; ++u) tot.add(v[u]);
         }
-        Elem<T>::store(out + e, tot.value());
+        Elem<T>::store(out + e, (float)tot.value());
     }
+}
+
+// The first `sf_blocks` blocks add up gsf, the others gcf.
+template <typename T>
+__global__ void __launch_bounds__(256)
+band_reduce_kernel(const BandPart<T>* part_sf, T* gsf, int n_sf, long long sf_size, const float* part_cf, T* gcf, int n_cf,
+                   long long cf_size, int B, int sf_blocks) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int block = (int)blockIdx.x - sf_blocks;
+    if (block < 0)
+        band_reduce(part_sf, gsf, n_sf, sf_size, B, blockIdx.x * 256ll + threadIdx.x, sf_blocks * 256ll);
+    else
+        band_reduce(part_cf, gcf, n_cf, cf_size, B, block * 256ll + threadIdx.x, (gridDim.x - sf_blocks) * 256ll);
 }
 
 // ------------------------------------------------------------------------ host side
@@ -481,9 +489,9 @@ inline bool band_filters_split(const Problem& p, int sm_count, BandBwdSplit& s) 
     return run <= (64 << 10);
 }
 
-// Floats of gsf / gcf partials (0: none needed).
+// Floats that gsf / gcf partials take (0: none needed).
 inline size_t band_part_sf(const Problem& p, const BandBwdSplit& s) {
-    return s.chunks > 1 ? (size_t)p.B * s.chunks * p.k * p.k * p.OH * p.OW : 0;
+    return s.chunks > 1 ? (size_t)p.B * s.chunks * p.k * p.k * p.OH * p.OW * (p.dtype == DDF_B200_F32 ? 2 : 1) : 0;
 }
 inline size_t band_part_cf(const Problem& p, const BandBwdSplit& s) {
     return s.bands > 1 ? (size_t)p.B * s.bands * p.C * p.k * p.k : 0;
@@ -542,7 +550,7 @@ int band_filters_launch(const BandBwdArgs& a, cudaStream_t stream, int* launches
     if (pl.n_slots < 2) return kNotHandled;
     uint32_t smem = pl.off_slot0 + (uint32_t)pl.n_slots * pl.slot_stride;
     if (sp.planes > 1) {  // room for the planes' sums to meet
-        const uint32_t meet = pl.off_slot0 + kBandGuard + (uint32_t)(sp.planes * K * K * p.OH * p.OW) * 4u;
+        const uint32_t meet = pl.off_slot0 + kBandGuard + (uint32_t)(sp.planes * K * K * p.OH * p.OW) * (uint32_t)sizeof(BandPart<T>);
         if (smem < meet) smem = meet;
         if (smem > kSmemBudget) return kNotHandled;
     }
@@ -566,7 +574,7 @@ int band_filters_launch(const BandBwdArgs& a, cudaStream_t stream, int* launches
         };
         const int nb_sf = pl.part_sf ? blocks(sf_size * p.B) : 0, nb_cf = pl.part_cf ? blocks(cf_size * p.B) : 0;
         e = launch_overlapped(band_reduce_kernel<T>, dim3((unsigned)(nb_sf + nb_cf)), dim3(256), 0, stream, true,
-                              (const float*)pl.part_sf, reinterpret_cast<T*>(a.gsf), sp.chunks, sf_size,
+                              (const BandPart<T>*)pl.part_sf, reinterpret_cast<T*>(a.gsf), sp.chunks, sf_size,
                               (const float*)pl.part_cf, reinterpret_cast<T*>(a.gcf), sp.bands, cf_size, p.B, nb_sf);
         if (e != cudaSuccess) return (int)e;
         ++*launches;

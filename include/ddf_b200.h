@@ -182,12 +182,15 @@ int ddf_b200_rate_probe(int mode, void* scratch, size_t scratch_bytes, int iters
 
 /* Which variant (GENERIC or STREAM) AUTO resolves to for this problem; pointers
  * are assumed 16-byte aligned.  `backward` = 0 for the forward, 1 for the backward.
- * Returns a DDF_B200_VARIANT_* value, or a negative status. */
+ * Returns a DDF_B200_VARIANT_* value, or a negative status.  GENERIC covers the band
+ * kernels too, which AUTO prefers to the generic ones where they are built. */
 int ddf_b200_plan(int B, int C, int H, int W, int k, int d, int s,
                   int combine, int dtype, int backward);
 
 /*
- * Bytes of scratch the backward needs for this problem (0 is possible).
+ * Bytes of scratch the backward needs for this problem (0 is possible).  Where
+ * ddf_b200_plan says GENERIC, less scratch (or none) is no error: the filter
+ * gradients then run on the generic kernels instead of the band kernels.
  * The reference makes its caller allocate three zero-filled scratch tensors
  * (ddf/ddf.py:106-108, resized in ddf/src/cuda/ddf_mul_cuda.cpp:85-87); here the
  * caller provides one untyped block, 256-byte aligned, which need not be zeroed.
@@ -227,9 +230,10 @@ int ddf_b200_backward(const void* go, const void* x, const void* cf, const void*
  * ddf_b200_backward_noalloc_limit() bytes (16 MiB), held by every GPU that
  * loads the library until the process exits.
  *
- *   - Problems whose scratch need (what ddf_b200_backward_workspace reports)
- *     exceeds that limit are refused with DDF_B200_E_SCRATCH_LIMIT before
- *     anything is launched.
+ *   - Problems of the plane-streaming kernels (ddf_b200_plan says STREAM) whose
+ *     scratch need (what ddf_b200_backward_workspace reports) exceeds that limit
+ *     are refused with DDF_B200_E_SCRATCH_LIMIT before anything is launched; any
+ *     other problem runs, on the generic kernels where the array is too small.
  *   - The call itself performs no cudaMalloc / cudaFree and uses no allocating
  *     library routine.
  *   - The first call on each device looks up the array's device address (one

@@ -118,10 +118,11 @@ static int generic_grad_x_launch(const Problem& p, const void* go, const void* c
         constexpr int CH = 16;
         dim3 grid((unsigned)((p.OH * p.OW + 255) / 256), (unsigned)((p.C + CH - 1) / CH), (unsigned)p.B);
         if (grid.y <= 65535u) {
-            if (p.combine == DDF_B200_MUL)
-                grad_x_k3s2<T, DDF_B200_MUL, CH><<<grid, 256, 0, st>>>((const T*)go, (const T*)cf, (const T*)sf, (T*)gx, p);
-            else
-                grad_x_k3s2<T, DDF_B200_ADD, CH><<<grid, 256, 0, st>>>((const T*)go, (const T*)cf, (const T*)sf, (T*)gx, p);
+            const bool odd = (p.H & 1) || (p.W & 1) || (reinterpret_cast<uintptr_t>(gx) & (2 * sizeof(T) - 1)) != 0;
+            auto kern = p.combine == DDF_B200_MUL
+                            ? (odd ? grad_x_k3s2<T, DDF_B200_MUL, CH, true> : grad_x_k3s2<T, DDF_B200_MUL, CH, false>)
+                            : (odd ? grad_x_k3s2<T, DDF_B200_ADD, CH, true> : grad_x_k3s2<T, DDF_B200_ADD, CH, false>);
+            kern<<<grid, 256, 0, st>>>((const T*)go, (const T*)cf, (const T*)sf, (T*)gx, p);
             g_launches.fetch_add(1, std::memory_order_relaxed);
             return (int)cudaGetLastError();
         }

@@ -88,7 +88,9 @@ generic_forward(const T* __restrict__ x, const T* __restrict__ cf, const T* __re
 // The last row of an odd H and the last column of an odd W are read by no tap: their gradient is zero.
 // Same arithmetic as generic_grad_x, without its per-tap divisions and parity tests:
 // (16,128,101x75) f32 20 us against 392.
-template <typename T, int MODE, int CH>
+// ODD: H or W is odd, or gx is not aligned to two elements; otherwise a row's two results leave as one store.
+// (64,128,56x56) bf16: 24 us; two stores per row 28, and 32 with the tests for odd edges beside them.
+template <typename T, int MODE, int CH, bool ODD>
 __global__ void __launch_bounds__(256)
 grad_x_k3s2(const T* __restrict__ go, const T* __restrict__ cf, const T* __restrict__ sf,
             T* __restrict__ gx, Problem p) {
@@ -99,7 +101,7 @@ grad_x_k3s2(const T* __restrict__ go, const T* __restrict__ cf, const T* __restr
     const int qy = q / p.OW, qx = q - qy * p.OW;
     const long long b = blockIdx.z;
     const bool has_x = qx + 1 < p.OW, has_y = qy + 1 < p.OH;
-    const bool odd_x = !has_x && (p.W & 1), odd_y = !has_y && (p.H & 1);
+    const bool odd_x = ODD && !has_x && (p.W & 1), odd_y = ODD && !has_y && (p.H & 1);
     const T* sfb = sf + b * 9 * (long long)opl + q;
     auto sfv = [&](int t, int off, bool ok) -> A { return ok ? (A)Elem<T>::load(sfb + (long long)t * opl + off) : (A)0; };
     const A s4 = sfv(4, 0, true), s5 = sfv(5, 0, true), s7 = sfv(7, 0, true), s8 = sfv(8, 0, true);
@@ -126,10 +128,18 @@ grad_x_k3s2(const T* __restrict__ go, const T* __restrict__ cf, const T* __restr
         const A r11 = g00 * combine_w<MODE, A>(w[8], s8) + g01 * combine_w<MODE, A>(w[6], s6) +
                       g10 * combine_w<MODE, A>(w[2], s2) + g11 * combine_w<MODE, A>(w[0], s0);
         T* o = gx + plane * ipl + (long long)(2 * qy) * p.W + 2 * qx;
-        Elem<T>::store(o, r00);
-        Elem<T>::store(o + 1, r01);
-        Elem<T>::store(o + p.W, r10);
-        Elem<T>::store(o + p.W + 1, r11);
+        if constexpr (!ODD && sizeof(T) == 2) {
+            *reinterpret_cast<uint32_t*>(o) = Word<T>::put(r00, r01);
+            *reinterpret_cast<uint32_t*>(o + p.W) = Word<T>::put(r10, r11);
+        } else if constexpr (!ODD && sizeof(T) == 4) {
+            *reinterpret_cast<float2*>(o) = make_float2(r00, r01);
+            *reinterpret_cast<float2*>(o + p.W) = make_float2(r10, r11);
+        } else {
+            Elem<T>::store(o, r00);
+            Elem<T>::store(o + 1, r01);
+            Elem<T>::store(o + p.W, r10);
+            Elem<T>::store(o + p.W + 1, r11);
+        }
         if (odd_x) {
             Elem<T>::store(o + 2, (A)0);
             Elem<T>::store(o + p.W + 2, (A)0);

@@ -4,9 +4,12 @@
 // for most shapes up to a few hundred microseconds of device work; the same call here costs a few
 // microseconds, most of it the launch itself.
 //
-// Semantics are those of the reference's autograd function (ddf/ddf.py:27-122).  Every argument
-// that does not pass the checks below goes to the Python function `explain` (op.py), which raises
-// the reference's assertion or this framework's error; there is one set of error texts.
+// Semantics are those of the reference's autograd function (ddf/ddf.py:27-122).  This path takes the
+// ordinary call: arguments that pass the checks below, plain tensors, nothing that watches or
+// transforms the program.  Every other call goes to the Python function `general` (op.py), the same
+// operator as a torch.autograd.Function: it raises the reference's assertions and this framework's
+// errors, and torch handles it under jit tracing (a node past the tracer would leave the traced
+// batch's output in the graph as a constant), functorch transforms, dispatch modes and forward mode.
 //
 // The library's entry points are bound by address (bind()), so DDF_B200_LIB keeps working.
 #include <Python.h>
@@ -14,6 +17,8 @@
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAGraphsUtils.cuh>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -21,6 +26,7 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include <cstring>
 #include <string>
@@ -42,7 +48,7 @@ struct Library {
     decltype(&ddf_b200_take_fault) take_fault = nullptr;
 } lib;
 PyObject* g_error_class = nullptr;  // _lib.DDFError
-PyObject* g_explain = nullptr;      // op.explain
+PyObject* g_general = nullptr;      // op._general
 PyObject* g_load = nullptr;         // op._bind_native: loads the library and calls bind()
 bool g_debug = false;
 
@@ -178,7 +184,7 @@ bool plain_int(PyObject* o, int& v) {
 
 bool text_is(PyObject* o, const char* s) { return PyUnicode_Check(o) && PyUnicode_CompareWithASCIIString(o, s) == 0; }
 
-// The reference's argument checks (ddf/ddf.py:32-65); false: `explain` finds out which one failed.
+// The reference's argument checks (ddf/ddf.py:32-65); false: `general` finds out which one failed.
 bool parse(PyObject* const* args, Py_ssize_t n, bool norm, Params& p, const Tensor*& x, const Tensor*& cf,
            const Tensor*& sf, at::ScalarType& dt) {
     if (n < 3 || n > (norm ? 9 : 8)) return false;
@@ -222,23 +228,29 @@ bool parse(PyObject* const* args, Py_ssize_t n, bool norm, Params& p, const Tens
     return dtype_code(dt) >= 0;
 }
 
+// Nothing watches or transforms the program (see the head of this file).
+bool ordinary(const Tensor& x, const Tensor& cf, const Tensor& sf) {
+    if (torch::jit::tracer::isTracing() || c10::impl::TorchDispatchModeTLS::any_modes_set() ||
+        c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode))
+        return false;
+    for (const Tensor* t : {&x, &cf, &sf})  // wrappers hold no storage of their own
+        if (!t->has_storage() || torch::autograd::isFwGradDefined(*t)) return false;
+    return true;
+}
+
 PyObject* call(PyObject* const* args, Py_ssize_t n, bool norm) {
     HANDLE_TH_ERRORS
     Params p;
     const Tensor *x, *cf, *sf;
     at::ScalarType dt;
-    if (!parse(args, n, norm, p, x, cf, sf, dt)) {
+    if (!parse(args, n, norm, p, x, cf, sf, dt) || !ordinary(*x, *cf, *sf)) {
         PyObject* list = PyTuple_New(n + 1);
         if (!list) return nullptr;
         PyTuple_SET_ITEM(list, 0, PyBool_FromLong(norm));
         for (Py_ssize_t i = 0; i < n; ++i) PyTuple_SET_ITEM(list, i + 1, Py_NewRef(args[i]));
-        PyObject* r = PyObject_CallObject(g_explain, list);
+        PyObject* r = PyObject_CallObject(g_general, list);
         Py_DECREF(list);
-        if (r) {
-            Py_DECREF(r);
-            PyErr_SetString(PyExc_TypeError, "ddf: unsupported arguments");
-        }
-        return nullptr;
+        return r;
     }
     if (C10_UNLIKELY(lib.forward == nullptr)) {
         PyObject* r = PyObject_CallNoArgs(g_load);
@@ -246,9 +258,6 @@ PyObject* call(PyObject* const* args, Py_ssize_t n, bool norm) {
         Py_DECREF(r);
     }
     const bool grad = at::GradMode::is_enabled() && (x->requires_grad() || cf->requires_grad() || sf->requires_grad());
-    TORCH_CHECK_NOT_IMPLEMENTED(!torch::autograd::isFwGradDefined(*x) && !torch::autograd::isFwGradDefined(*cf) &&
-                                    !torch::autograd::isFwGradDefined(*sf),
-                                "ddf: forward-mode differentiation is not implemented");
     Tensor out;
     {
         pybind11::gil_scoped_release no_gil;
@@ -289,12 +298,12 @@ PyObject* call(PyObject* const* args, Py_ssize_t n, bool norm) {
 PyObject* py_ddf(PyObject*, PyObject* const* args, Py_ssize_t n) { return call(args, n, false); }
 PyObject* py_ddf_sfnorm(PyObject*, PyObject* const* args, Py_ssize_t n) { return call(args, n, true); }
 
-// hooks(error_class, explain, load): the Python side's callables, set when the package is imported.
+// hooks(error_class, general, load): the Python side's callables, set when the package is imported.
 PyObject* py_hooks(PyObject*, PyObject* args) {
     PyObject *e, *x, *l;
     if (!PyArg_ParseTuple(args, "OOO", &e, &x, &l)) return nullptr;
     Py_XSETREF(g_error_class, Py_NewRef(e));
-    Py_XSETREF(g_explain, Py_NewRef(x));
+    Py_XSETREF(g_general, Py_NewRef(x));
     Py_XSETREF(g_load, Py_NewRef(l));
     Py_RETURN_NONE;
 }

@@ -74,8 +74,9 @@ generic_forward(const T* __restrict__ x, const T* __restrict__ cf, const T* __re
     }
 }
 
-// grad-x for k = 3, dilation 1, stride 2: the case of the down-sampling layers.  A thread owns one OUTPUT pixel q = (qy, qx) of a sample and walks a
-// chunk of channels; per channel it writes the 2 x 2 input pixels (2qy.., 2qx..).  With stride
+// grad-x for k = 3, dilation 1, stride 2: the case of the down-sampling layers.  A thread owns one
+// OUTPUT pixel q = (qy, qx) of a sample and walks a chunk of channels; per channel it writes the
+// 2 x 2 input pixels (2qy.., 2qx..).  With stride
 // 2 each input pixel receives only the taps whose offset has its parity -- 1, 2, 2 and 4 of
 // the nine -- so the four results need exactly nine products, and the nine spatial-filter
 // values they use (at q and its right / lower / lower-right neighbours) stay in registers for
@@ -84,7 +85,8 @@ generic_forward(const T* __restrict__ x, const T* __restrict__ cf, const T* __re
 //   gx[2qy  ][2qx+1] = go[q]*w5[q]  + go[q+x]*w3[q+x]
 //   gx[2qy+1][2qx  ] = go[q]*w7[q]  + go[q+y]*w1[q+y]
 //   gx[2qy+1][2qx+1] = go[q]*w8[q]  + go[q+x]*w6[q+x] + go[q+y]*w2[q+y] + go[q+x+y]*w0[q+x+y]
-// (w_t[q] = cf[c,t] (.) sf[t,q]; neighbours outside the plane contribute nothing).
+// (w_t[q] = cf[c,t] (.) sf[t,q]; terms of neighbours outside the plane are left out, not multiplied by
+// zero: cf may hold an infinity).
 // The last row of an odd H and the last column of an odd W are read by no tap: their gradient is zero.
 // Same arithmetic as generic_grad_x, without its per-tap divisions and parity tests:
 // (16,128,101x75) f32 20 us against 392.
@@ -123,10 +125,17 @@ grad_x_k3s2(const T* __restrict__ go, const T* __restrict__ cf, const T* __restr
         const A g10 = has_y ? (A)Elem<T>::load(gop + p.OW) : (A)0;
         const A g11 = (has_x && has_y) ? (A)Elem<T>::load(gop + p.OW + 1) : (A)0;
         const A r00 = g00 * combine_w<MODE, A>(w[4], s4);
-        const A r01 = g00 * combine_w<MODE, A>(w[5], s5) + g01 * combine_w<MODE, A>(w[3], s3);
-        const A r10 = g00 * combine_w<MODE, A>(w[7], s7) + g10 * combine_w<MODE, A>(w[1], s1);
-        const A r11 = g00 * combine_w<MODE, A>(w[8], s8) + g01 * combine_w<MODE, A>(w[6], s6) +
-                      g10 * combine_w<MODE, A>(w[2], s2) + g11 * combine_w<MODE, A>(w[0], s0);
+        A r01 = g00 * combine_w<MODE, A>(w[5], s5), r10 = g00 * combine_w<MODE, A>(w[7], s7);
+        A r11 = g00 * combine_w<MODE, A>(w[8], s8);
+        if (has_x) {
+            r01 += g01 * combine_w<MODE, A>(w[3], s3);
+            r11 += g01 * combine_w<MODE, A>(w[6], s6);
+        }
+        if (has_y) {
+            r10 += g10 * combine_w<MODE, A>(w[1], s1);
+            r11 += g10 * combine_w<MODE, A>(w[2], s2);
+        }
+        if (has_x && has_y) r11 += g11 * combine_w<MODE, A>(w[0], s0);
         T* o = gx + plane * ipl + (long long)(2 * qy) * p.W + 2 * qx;
         if constexpr (!ODD && sizeof(T) == 2) {
             *reinterpret_cast<uint32_t*>(o) = Word<T>::put(r00, r01);

@@ -3,7 +3,7 @@
 import pytest
 import torch
 
-from tests.util import DTYPES, check_close, make_inputs, oracle_backward
+from tests.util import DTYPES, check_close, check_extremes, make_inputs, oracle_backward
 
 pytestmark = pytest.mark.gpu
 
@@ -143,3 +143,19 @@ def test_gradcheck_float64(shape, s, m):
         sf = torch.randn(B, k * k, H // s, W // s, generator=g, dtype=torch.float64).to(dev).requires_grad_()
         assert torch.autograd.gradcheck(lambda a, b, c: ddf(a, b, c, k, d, s, m), (x, cf, sf),
                                         eps=1e-3, atol=1e-5)
+
+
+@pytest.mark.parametrize("plane", [(8, 10), (9, 10), (8, 11), (9, 11), (2, 3), (35, 37)])
+@pytest.mark.parametrize("version", ["", "o"])
+@pytest.mark.parametrize("dt", ["f32", "f64", "f16", "bf16"])
+@pytest.mark.parametrize("mode", ["mul", "add"])
+def test_stride2_grad_x_leaves_out_the_padding(plane, version, dt, mode):
+    """Infinite channel-filter values: a tap whose output pixel lies outside the plane is skipped."""
+    from ddfnet_b200 import ddf
+    dtype = DTYPES[dt]
+    x, cf, sf, go = make_inputs(2, 19, *plane, 3, 2, dtype, seed=91)
+    cf.view(-1)[::5] = float("inf")
+    cf.view(-1)[2::31] = float("-inf")
+    ts = [t.cuda().requires_grad_() for t in (x, cf, sf)]
+    gx, = torch.autograd.grad(ddf(*ts, 3, 1, 2, mode, version), ts[:1], go.cuda())
+    check_extremes(gx, oracle_backward(go, x, cf, sf, 3, 1, 2, mode)[0], dtype, f"grad_x {plane} {mode}")

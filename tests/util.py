@@ -89,3 +89,13 @@ def check_close(actual, expected64, dtype, what="", reduction=False):
         b_rounded = b.to(dtype).to(torch.float64)
         rel_l2 = ((a - b_rounded).pow(2).sum() / b.pow(2).sum().clamp_min(1e-30)).sqrt().item()
         assert rel_l2 <= 2e-3, f"{what}: relative L2 distance {rel_l2:.3e} > 2e-3"
+
+
+def check_extremes(actual, want64, dtype, what, reduction=False):
+    """As check_close where the oracle is finite; elsewhere NaN for NaN and infinities of the same sign."""
+    a, fin = actual.detach().cpu().double(), torch.isfinite(want64)
+    assert torch.equal(torch.isfinite(a), fin), f"{what}: other values are finite"
+    assert torch.equal(a.isnan(), want64.isnan()), f"{what}: NaN and infinity mixed up"
+    assert torch.equal(a.nan_to_num(0.0).sign()[~fin], want64.nan_to_num(0.0).sign()[~fin]), f"{what}: an infinity's sign"
+    zero = torch.zeros((), dtype=torch.float64)
+    check_close(torch.where(fin, a, zero), torch.where(fin, want64, zero), dtype, what, reduction)

@@ -116,13 +116,14 @@ struct DDFBackward : public torch::autograd::Node {
         torch::autograd::variable_list out(3);
         std::lock_guard<std::mutex> lock(mutex_);
         TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
-        if (!grads[0].defined()) return out;
         const bool need_x = task_should_compute_output(0), need_cf = task_should_compute_output(1),
                    need_sf = task_should_compute_output(2);
         const Tensor x = x_.unpack(), cf = cf_.unpack(), sf = sf_.unpack();
         at::NoGradGuard no_grad;
         const at::ScalarType dt = x.scalar_type();
-        Tensor go = grads[0];
+        // a gradient that never reached the output is zero, as torch.autograd.Function has it
+        Tensor go = grads[0].defined() ? grads[0]
+                                       : at::zeros({x.size(0), x.size(1), x.size(2) / p.s, x.size(3) / p.s}, x.options());
         TORCH_CHECK(go.is_cuda(), "the gradient of the op's output must be a CUDA tensor");
         if (go.scalar_type() != dt) go = go.to(dt);
         go = go.contiguous();

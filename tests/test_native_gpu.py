@@ -59,3 +59,19 @@ def test_transforms_are_refused_as_for_any_autograd_function():
         torch.func.grad(lambda x: f(x, *a[1:]).sum())(a[0])
     with forward_ad.dual_level(), pytest.raises(RuntimeError):
         f(forward_ad.make_dual(a[0], torch.ones_like(a[0])), *a[1:])
+
+
+@pytest.mark.parametrize("fused", [False, True])
+def test_a_gradient_that_does_not_arrive_is_zero(fused):
+    class Drop(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, y):
+            return y.clone()
+
+        @staticmethod
+        def backward(ctx, g):
+            return None
+
+    ts = _inputs(5, grad=True)[:3]
+    Drop.apply(_entry(fused)(*ts)).sum().backward()
+    assert all(t.grad is not None and not t.grad.any() for t in ts)

@@ -15,8 +15,10 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/SequenceNumber.h>
 #include <ATen/cuda/CUDAGraphsUtils.cuh>
 #include <ATen/cuda/EmptyTensor.h>
+#include <ATen/record_function.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -259,6 +261,16 @@ PyObject* call(PyObject* const* args, Py_ssize_t n, bool norm) {
         Py_DECREF(r);
     }
     const bool grad = at::GradMode::is_enabled() && (x->requires_grad() || cf->requires_grad() || sf->requires_grad());
+    // the range that a profiler shows for an autograd function's forward
+    at::RecordFunction range(at::RecordScope::FUNCTION);
+    if (C10_UNLIKELY(range.isActive())) {
+        const char* name = norm ? "DDFSpatialNormFunction" : "DDFFunction";
+        const c10::IValue inputs[] = {*x, *cf, *sf};
+        if (range.needsInputs())
+            range.before(name, c10::ArrayRef<const c10::IValue>(inputs), at::sequence_number::peek());
+        else
+            range.before(name, at::sequence_number::peek());
+    }
     Tensor out;
     {
         pybind11::gil_scoped_release no_gil;

@@ -75,3 +75,12 @@ def test_a_gradient_that_does_not_arrive_is_zero(fused):
     ts = _inputs(5, grad=True)[:3]
     Drop.apply(_entry(fused)(*ts)).sum().backward()
     assert all(t.grad is not None and not t.grad.any() for t in ts)
+
+
+@pytest.mark.parametrize("fused,name", [(False, "DDFFunction"), (True, "DDFSpatialNormFunction")])
+def test_a_profiler_shows_the_call_and_its_backward(fused, name):
+    ts = _inputs(6, grad=True)[:3]
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+        _entry(fused)(*ts).sum().backward()
+    seen = {e.key for e in prof.key_averages()}
+    assert {name, name + "Backward"} <= seen

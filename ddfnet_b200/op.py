@@ -21,20 +21,19 @@ The arithmetic runs in hand-written CUDA kernels reached through the C ABI of
 libddf_b200.so; there is no CPU path.  The host side of a call -- argument checks, output
 allocation, autograd node, launch -- is csrc/native.cpp for the calls that are ordinary (see there);
 every other call takes the autograd functions of this file: refused arguments, whose error they
-raise, tracing, functorch transforms, forward-mode tensors, dispatch modes.
+raise, tracing, functorch transforms, forward-mode tensors, dispatch modes.  Where csrc/native.cpp
+has not been built, every call takes them.
 """
 from __future__ import annotations
 
 import ctypes
+import importlib
+import warnings
 
 import torch
 from torch.autograd import Function
 
 from . import _lib
-try:
-    from . import _native
-except ImportError:  # not built: importing works, calling the op raises
-    _native = None
 
 _DTYPES = {torch.float32: _lib.F32, torch.float16: _lib.F16, torch.bfloat16: _lib.BF16,
            torch.float64: _lib.F64}
@@ -259,6 +258,30 @@ def _general(norm, *args):
     return super(cls, cls).apply(*args)
 
 
+_native = None  # csrc/native.cpp, once it could be imported
+_asked = False  # ... and whether its absence has been reported
+
+
+def _import_native():
+    """Imports the C++ host path.  It may be built after this package was imported, so a call that does
+    not have it yet asks again."""
+    global _native, _asked
+    if _native is None:
+        importlib.invalidate_caches()
+        try:
+            module = importlib.import_module("._native", __package__)
+        except ImportError as e:
+            if not _asked:
+                _asked = True
+                what = "is not built" if isinstance(e, ModuleNotFoundError) else f"failed to load ({e})"
+                warnings.warn(f"ddfnet_b200/_native.so {what}: calls of ddf take the slower Python host path.  "
+                              "Build it:  python -m ddfnet_b200.csrc.build", RuntimeWarning, stacklevel=3)
+            return False
+        module.hooks(_lib.DDFError, _general, _bind_native)
+        _native = module
+    return True
+
+
 def _bind_native():
     """Hands the library's entry points to the native module (the first call does this)."""
     lib = _lib.load()
@@ -267,12 +290,17 @@ def _bind_native():
     _native.bind({n: ctypes.cast(getattr(lib, n), ctypes.c_void_p).value for n in names}, _lib._DEBUG)
 
 
-def _not_built(*_args):
-    raise RuntimeError("ddfnet_b200/_native.so not found. The DDF op has no Python fallback; build it first:  "
-                       "python -m ddfnet_b200.csrc.build")
+def _until_built(name, norm):
+    def call(*args):
+        return getattr(_native, name)(*args) if _import_native() else _general(norm, *args)
+    call.__name__ = name
+    return call
 
 
-if _native is not None:
+try:
+    from . import _native
+except ImportError:
+    ddf, ddf_sfnorm = _until_built("ddf", False), _until_built("ddf_sfnorm", True)
+else:
     _native.hooks(_lib.DDFError, _general, _bind_native)
-ddf = _native.ddf if _native is not None else _not_built
-ddf_sfnorm = _native.ddf_sfnorm if _native is not None else _not_built
+    ddf, ddf_sfnorm = _native.ddf, _native.ddf_sfnorm

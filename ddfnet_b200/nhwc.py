@@ -6,7 +6,7 @@ from __future__ import annotations
 
 import torch
 
-from . import _lib
+from . import _lib, op
 from .op import _DTYPES
 
 
@@ -44,22 +44,13 @@ class StemMaxPool(torch.nn.MaxPool2d):
         super().__init__(3, stride=2, padding=1)
 
     def forward(self, x):
-        if (type(x) not in (torch.Tensor, torch.nn.Parameter) or not x.is_cuda or torch.is_grad_enabled() and x.requires_grad
-                or torch.compiler.is_compiling() or torch._C._functorch.is_functorch_wrapped_tensor(x)
-                or x.dtype not in (torch.float16, torch.bfloat16, torch.float32) or not _is_cl(x) or x.is_contiguous()
-                or x.numel() == 0 or x.shape[2] * x.shape[3] > 1 << 30
-                or x.shape[1] * x.element_size() % 16 != 0 or x.data_ptr() % 16 != 0
-                or (self.kernel_size, self.stride, self.padding, self.dilation, self.ceil_mode, self.return_indices)
-                != (3, 2, 1, 1, False, False) or torch.jit.is_tracing()
-                or torch.autograd.forward_ad.unpack_dual(x).tangent is not None):
-            return super().forward(x)
-        b, c, h, w = x.shape
-        out = torch.empty((b, c, (h - 1) // 2 + 1, (w - 1) // 2 + 1), dtype=x.dtype, device=x.device,
-                          memory_format=torch.channels_last)
-        with torch.cuda.device(x.device):
-            _lib.check(_lib.load().ddf_b200_maxpool_nhwc(x.data_ptr(), out.data_ptr(), b, c, h, w, _DTYPES[x.dtype],
-                                                         torch.cuda.current_stream().cuda_stream))
-        return out
+        if (op._native is not None and not torch.compiler.is_compiling()
+                and (self.kernel_size, self.stride, self.padding, self.dilation, self.ceil_mode, self.return_indices)
+                == (3, 2, 1, 1, False, False)):
+            out = op._native.stem_maxpool(x)
+            if out is not None:
+                return out
+        return super().forward(x)
 
 
 def ddf_nhwc(x: torch.Tensor, channel_filter: torch.Tensor, spatial_filter: torch.Tensor,

@@ -286,7 +286,7 @@ def _bind_native():
     """Hands the library's entry points to the native module (the first call does this)."""
     lib = _lib.load()
     names = ("ddf_b200_forward", "ddf_b200_forward_sfnorm", "ddf_b200_backward_workspace", "ddf_b200_backward",
-             "ddf_b200_sfnorm", "ddf_b200_sfnorm_backward", "ddf_b200_take_fault")
+             "ddf_b200_sfnorm", "ddf_b200_sfnorm_backward", "ddf_b200_take_fault", "ddf_b200_maxpool_nhwc")
     _native.bind({n: ctypes.cast(getattr(lib, n), ctypes.c_void_p).value for n in names}, _lib._DEBUG)
 
 

@@ -36,3 +36,11 @@ def test_gradients_stay_with_torch():
     x = torch.randn(2, 16, 9, 9, device="cuda").contiguous(memory_format=torch.channels_last).requires_grad_()
     StemMaxPool()(x).sum().backward()
     assert x.grad is not None
+
+
+def test_a_traced_pooling_runs_on_new_inputs():
+    from ddfnet_b200.nhwc import StemMaxPool
+    a, b = (torch.randn(2, 16, 9, 11, device="cuda").contiguous(memory_format=torch.channels_last) for _ in range(2))
+    with torch.no_grad():
+        traced = torch.jit.trace(StemMaxPool(), (a,), check_trace=False)
+        assert torch.equal(traced(b), F.max_pool2d(b, 3, 2, 1))

@@ -403,6 +403,37 @@ int ddf_b200_forward_waitlimit(const void* x, const void* cf, const void* sf, vo
     return rc == kNotHandled ? DDF_B200_E_UNSUPPORTED : rc;
 }
 
+int ddf_b200_band_waitlimit(const void* go, const void* x, const void* cf, const void* sf, void* out, void* gcf,
+                            void* gsf, void* workspace, size_t workspace_bytes, int B, int C, int H, int W, int k,
+                            int d, int s, int combine, int dtype, long long wait_cycles, int starve, void* stream) {
+    Problem p;
+    int rc = check_problem(B, C, H, W, k, d, s, combine, dtype, DDF_B200_VARIANT_AUTO, p);
+    if (rc) return rc;
+    if (!x || !cf || !sf || (!go && (gcf || gsf))) return DDF_B200_E_NULL;
+    if (wait_cycles < 1) return DDF_B200_E_SHAPE;
+    DeviceInfo* di = nullptr;
+    rc = device_info(di);
+    if (rc) return rc;
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    const uint32_t skew = starve ? 16u : 0u;
+    if (out) {
+        rc = run_band(BandArgs{x, cf, sf, out, p, false, di->sm_count, di->fault, di->index, wait_cycles, skew}, st);
+        if (rc) return rc == kNotHandled ? DDF_B200_E_UNSUPPORTED : rc;
+    }
+    if (gcf || gsf) {
+        size_t need = 0;
+        if (!band_filters_workspace(p, di->sm_count, &need)) return DDF_B200_E_UNSUPPORTED;
+        if (need > 0 && (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 7u) != 0))
+            return DDF_B200_E_WORKSPACE;
+        int launches = 0;
+        rc = band_filters(p, go, x, cf, sf, gcf, gsf, workspace, di->sm_count, di->fault, di->index, st, &launches,
+                          wait_cycles, skew);
+        g_launches.fetch_add((unsigned long long)launches, std::memory_order_relaxed);
+        if (rc) return rc == kNotHandled ? DDF_B200_E_UNSUPPORTED : rc;
+    }
+    return 0;
+}
+
 int ddf_b200_forward_sfnorm(const void* x, const void* cf, const void* sf_raw, void* out, int B,
                             int C, int H, int W, int k, int d, int s, int combine, int dtype,
                             int variant, double sf_scale, void* stream) {

@@ -13,9 +13,10 @@ bool band_filters_workspace(const Problem& p, int sm_count, size_t* bytes) {
 }
 
 int band_filters(const Problem& p, const void* go, const void* x, const void* cf, const void* sf, void* gcf, void* gsf,
-                 void* workspace, int sm_count, int* fault, int device, cudaStream_t st, int* launches) {
+                 void* workspace, int sm_count, int* fault, int device, cudaStream_t st, int* launches,
+                 long long wait_cycles, uint32_t tx_skew) {
     *launches = 0;
-    const BandBwdArgs a{go, x, cf, sf, gcf, gsf, workspace, p, sm_count, fault, device};
+    const BandBwdArgs a{go, x, cf, sf, gcf, gsf, workspace, p, sm_count, fault, device, wait_cycles, tx_skew};
     switch (p.dtype) {
         case DDF_B200_F32: return band_filters_dispatch<float>(a, st, launches);
         case DDF_B200_F16: return band_filters_dispatch<__half>(a, st, launches);

@@ -11,6 +11,7 @@ bool band_filters_workspace(const Problem& p, int sm_count, size_t* bytes);
 // kNotHandled: not built, or a tensor is not aligned for bulk copies.  `workspace` holds what
 // band_filters_workspace says.
 int band_filters(const Problem& p, const void* go, const void* x, const void* cf, const void* sf, void* gcf, void* gsf,
-                 void* workspace, int sm_count, int* fault, int device, cudaStream_t st, int* launches);
+                 void* workspace, int sm_count, int* fault, int device, cudaStream_t st, int* launches,
+                 long long wait_cycles = kWaitCycles, uint32_t tx_skew = 0);
 
 }  // namespace ddf

@@ -53,6 +53,8 @@ struct BandBwdPlan {
     unsigned long long x_total, go_total;
     uint32_t off_cf, off_part, off_slot0, slot_stride, zero_off, go_off;  // zero_off, go_off: from a slot's data
     int* fault;
+    long long wait_cycles;
+    uint32_t tx_skew;  // see BandPlan
 };
 
 template <typename T, int K, int D, int S, int PH, int MODE>
@@ -120,11 +122,10 @@ band_filters_kernel(const __grid_constant__ BandBwdPlan pl) {
     if (warp == NW) {
         // ------------------------------------------------------------- producer
         if (lane == 0) {
-            bool ok = true;
             int issued = 0;
             for (; issued < npass; ++issued) {
                 const int slot = issued % NST;
-                if (issued >= NST && !mbar_wait(BAND_EMPTY(slot), (uint32_t)((issued / NST - 1) & 1))) { ok = false; break; }
+                if (!band_slot_free(BAND_EMPTY(slot), issued, NST, pl.wait_cycles, pl.tx_skew)) break;
                 const int left = c_hi - c_lo - issued * G;
                 const unsigned long long more = (unsigned long long)((left < G ? left : G) - 1);
                 const unsigned long long x0 = x_first + (unsigned long long)issued * G * xplane;
@@ -133,17 +134,11 @@ band_filters_kernel(const __grid_constant__ BandBwdPlan pl) {
                                              x0 + more * xplane + (unsigned long long)(iy_hi - iy_lo) * pl.W * ES, pl.x_total);
                 const Span sg = span_prepare(BAND_DATA(slot) + pl.go_off, pl.go, g0,
                                              g0 + more * gplane + (unsigned long long)(y_hi - go_row) * pl.OW * ES, pl.go_total);
-                mbar_arrive_expect_tx(BAND_FULL(slot), sx.bytes + sg.bytes);
+                mbar_arrive_expect_tx(BAND_FULL(slot), sx.bytes + sg.bytes + pl.tx_skew);
                 span_issue(sx, BAND_FULL(slot));
                 span_issue(sg, BAND_FULL(slot));
             }
-            if (!ok) {
-                atomicCAS(pl.fault, 0, (int)kFaultService);
-                bool drained = true;
-                for (int j = issued - NST; j < issued; ++j)
-                    drained &= mbar_wait(BAND_FULL(j % NST), (uint32_t)((j / NST) & 1));
-                if (!drained) atomicExch(pl.fault, (int)kFaultDrain);
-            }
+            band_leave(BAND_FULL(0), issued, npass, NST, pl.wait_cycles, pl.tx_skew, pl.fault);
         }
         return;
     }
@@ -238,17 +233,15 @@ band_filters_kernel(const __grid_constant__ BandBwdPlan pl) {
     uint32_t cf_s = sbase + pl.off_cf + (uint32_t)pip * CFB;
     uint32_t part_s = sbase + pl.off_part + 4u * (uint32_t)((pip * pl.plane_warps + wip) * KK);
     int left = c_hi - c_lo - pip;
-    bool dead = false;
 
     int slot = -1;
     uint32_t ph = 1;
     for (int i = 0; i < npass; ++i) {
         if (++slot == NST) slot = 0;
         if (slot == 0) ph ^= 1u;
-        // a warp whose wait ran out stays for the barriers of the others, without waiting again
-        if (!dead && !mbar_wait(BAND_FULL(slot), ph)) {
+        if (ph < kBandDead && !mbar_wait_for(BAND_FULL(slot), ph, pl.wait_cycles)) {
             atomicCAS(pl.fault, 0, (int)kFaultConsumerFull);
-            dead = true;
+            ph |= kBandDead;
         }
         if (left > 0) {  // this warp's plane of the pass exists
             const uint32_t xbase = BAND_DATA(slot) + (x_lo & 15u);
@@ -345,14 +338,14 @@ band_filters_kernel(const __grid_constant__ BandBwdPlan pl) {
             }
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(BAND_EMPTY(slot));
+        if (lane == 0 && ph < kBandDead) mbar_arrive(BAND_EMPTY(slot));
         x_lo += x_step;
         go_lo += go_step;
         cf_s += (uint32_t)G * CFB;
         part_s += 4u * (uint32_t)(NW * KK);
         left -= G;
     }
-    if (band_sync_or(NW * 32, dead ? 1 : 0)) return;  // a fault is recorded; copies may still be in flight
+    if (band_sync_or(NW * 32, ph >= kBandDead ? 1 : 0)) return;  // a fault is recorded, and there are no whole sums
 
     if (pl.gcf != nullptr) {  // this band's share of gcf: the plane's warps added up; taps back in row order
         const int n = (c_hi - c_lo) * KK;
@@ -509,6 +502,8 @@ struct BandBwdArgs {
     int sm_count;
     int* fault;
     int device;
+    long long wait_cycles = kWaitCycles;
+    uint32_t tx_skew = 0;
 };
 
 template <typename T, int K, int D, int S, int MODE>
@@ -530,7 +525,7 @@ int band_filters_launch(const BandBwdArgs& a, cudaStream_t stream, int* launches
     pl.plane_warps = sp.warps / sp.planes;
     pl.x_total = (unsigned long long)p.B * p.C * p.H * p.W * ES;
     pl.go_total = (unsigned long long)p.B * p.C * p.OH * p.OW * ES;
-    pl.fault = a.fault;
+    pl.fault = a.fault; pl.wait_cycles = a.wait_cycles; pl.tx_skew = a.tx_skew;
     const long long rows = (long long)(band_rows<D, PH>(sp.groups) - 1) * S + (K - 1) * D + 1;
     const long long grows = band_rows<D, PH>(sp.groups);
     const uint32_t xrun = (uint32_t)(((sp.planes - 1) * (long long)p.H + (rows < p.H ? rows : p.H)) * p.W * ES);

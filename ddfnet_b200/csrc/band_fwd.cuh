@@ -27,7 +27,9 @@
 // NaN where the definition skips the tap: while the filters hold anything not below kBandFilterMax
 // in magnitude (so that cf * sf is finite too) a CTA takes a plain loop that skips those taps.
 //
-// Every mbarrier wait is bounded (fault word, drain), as in the other streaming kernels.
+// Every mbarrier wait is bounded by the plan's wait_cycles.  A thread whose wait ran out records a fault,
+// stays for the barriers of the others, and neither stores nor hands slots back: the producer's own wait
+// then runs out and it issues no more.  The producer leaves, always, after the last copies have landed.
 #pragma once
 
 #include <atomic>
@@ -42,6 +44,7 @@ constexpr int kBandStage = 64;       // channels whose filters are staged togeth
 constexpr float kBandFilterMax = 1e18f;
 constexpr uint32_t kBandGuard = 32;  // readable bytes before a slot's data (left halo of its first row)
 constexpr uint32_t kBandZero = 80;   // zeroed bytes after it
+constexpr uint32_t kBandDead = 2;    // bit of a compute thread's ring phase: one of its waits ran out
 
 struct BandPlan {
     const void* in;
@@ -60,7 +63,24 @@ struct BandPlan {
     unsigned long long in_total;
     uint32_t off_cf, off_slot0, slot_stride, zero_off;  // zero_off: from a slot's data start
     int* fault;
+    long long wait_cycles;    // limit of every mbarrier wait, in SM clocks
+    uint32_t tx_skew;         // self-test: bytes announced beyond what is copied, so that no stage completes
 };
+
+// Ring hand-over of the band kernels' producer lane: its wait for a free slot, and, before it leaves, the
+// waits for the last copies (the block's shared memory must not go while they are in flight).
+__device__ __forceinline__ bool band_slot_free(uint32_t bar_empty, int issued, int nst, long long wait_cycles, uint32_t skew) {
+    // with the self-test's skew the compute warps, whose limit is shorter, report first
+    return issued < nst || mbar_wait_for(bar_empty, (uint32_t)((issued / nst - 1) & 1), skew ? 2 * wait_cycles : wait_cycles);
+}
+__device__ __forceinline__ void band_leave(uint32_t bar_full0, int issued, int n, int nst, long long wait_cycles, uint32_t skew,
+                                           int* fault) {
+    if (issued < n) atomicCAS(fault, 0, (int)kFaultService);
+    bool landed = true;
+    for (int j = issued > nst ? issued - nst : 0; j < issued; ++j)
+        landed &= mbar_wait_for(bar_full0 + 8u * (uint32_t)(j % nst), (uint32_t)((j / nst) & 1), wait_cycles);
+    if (!landed && skew == 0) atomicExch(fault, (int)kFaultDrain);
+}
 
 // Element loads with a per-thread column mask folded into the conversion.
 template <typename T> struct Masked;
@@ -186,10 +206,9 @@ band_kernel(const __grid_constant__ BandPlan pl) {
         Rows r = rows_of(seg);
         const int n = u_hi - u_lo;
         int issued = 0;
-        bool ok = true;
         for (; issued < n; ++issued) {
             const int slot = issued % NST;
-            if (issued >= NST && !mbar_wait(BAND_EMPTY(slot), (uint32_t)((issued / NST - 1) & 1))) { ok = false; break; }
+            if (!band_slot_free(BAND_EMPTY(slot), issued, NST, pl.wait_cycles, pl.tx_skew)) break;
             const int c = pass * G;
             const int count = pl.C - c < G ? pl.C - c : G;
             const unsigned long long g0 = run_start(r, c);
@@ -197,20 +216,14 @@ band_kernel(const __grid_constant__ BandPlan pl) {
                                          g0 + (unsigned long long)(count - 1) * plane_bytes +
                                              (unsigned long long)(r.iy_hi - r.iy_lo) * pl.W * ES,
                                          pl.in_total);
-            mbar_arrive_expect_tx(BAND_FULL(slot), sp.bytes);
+            mbar_arrive_expect_tx(BAND_FULL(slot), sp.bytes + pl.tx_skew);
             span_issue(sp, BAND_FULL(slot));
             if (++pass == pl.passes) {
                 pass = 0;
                 r = rows_of(++seg);
             }
         }
-        if (!ok) {
-            atomicCAS(pl.fault, 0, (int)kFaultService);
-            bool drained = true;
-            for (int j = issued - NST; j < issued; ++j)
-                drained &= mbar_wait(BAND_FULL(j % NST), (uint32_t)((j / NST) & 1));
-            if (!drained) atomicExch(pl.fault, (int)kFaultDrain);
-        }
+        band_leave(BAND_FULL(0), issued, n, NST, pl.wait_cycles, pl.tx_skew, pl.fault);
         return;
     }
 
@@ -236,7 +249,6 @@ band_kernel(const __grid_constant__ BandPlan pl) {
     uint32_t ph = 1;
     int seg = u_lo / pl.passes;
     int pass = u_lo - seg * pl.passes;
-    bool dead = false;
     bool fresh = true;  // the next unit starts another (sample, band)
     Rows rw = rows_of(seg);
     int big_sf = 0;     // a spatial-filter value too large for products with padding zeros (or NaN)
@@ -346,10 +358,9 @@ band_kernel(const __grid_constant__ BandPlan pl) {
         for (int i = 0; i < npass; ++i) {
             if (++slot == NST) slot = 0;
             if (slot == 0) ph ^= 1u;
-            // a warp whose wait ran out stays for the barriers of the others, without waiting again
-            if (!dead && !mbar_wait(BAND_FULL(slot), ph)) {
+            if (ph < kBandDead && !mbar_wait_for(BAND_FULL(slot), ph, pl.wait_cycles)) {
                 atomicCAS(pl.fault, 0, (int)kFaultConsumerFull);
-                dead = true;
+                ph |= kBandDead;
             }
             const uint32_t base = BAND_DATA(slot) + (g_lo & 15u);
             unsigned long long acc2[HP];
@@ -405,8 +416,8 @@ band_kernel(const __grid_constant__ BandPlan pl) {
             }
             // the slot is handed back before the stores: nothing below reads it
             __syncwarp();
-            if (lane == 0) mbar_arrive(BAND_EMPTY(slot));
-            if (left > 0) {
+            if (lane == 0 && ph < kBandDead) mbar_arrive(BAND_EMPTY(slot));
+            if (left > 0 && ph < kBandDead) {
                 T* o = outp;
                 float res[PH];
 #pragma unroll
@@ -446,6 +457,8 @@ struct BandArgs {
     int sm_count;
     int* fault;
     int device;
+    long long wait_cycles = kWaitCycles;
+    uint32_t tx_skew = 0;
 };
 
 // Bands of a problem; shared with the filter-gradient form.
@@ -513,7 +526,7 @@ int band_launch(const BandArgs& a, cudaStream_t stream) {
     if (pl.stage_passes > pl.passes) pl.stage_passes = pl.passes;
     pl.bwdx = a.bwdx; pl.norm = p.sf_norm; pl.sf_scale = (float)p.sf_scale;
     pl.in_total = (unsigned long long)p.B * p.C * pl.H * pl.W * ES;
-    pl.fault = a.fault;
+    pl.fault = a.fault; pl.wait_cycles = a.wait_cycles; pl.tx_skew = a.tx_skew;
     const long long plane_bytes = (long long)pl.H * pl.W * ES;
     const long long rows = (long long)(band_rows<D, PH>(sp.groups) - 1) * S + 2 * R * D + 1;
     const long long run = (sp.planes - 1) * plane_bytes + (rows < pl.H ? rows : pl.H) * (long long)pl.W * ES;

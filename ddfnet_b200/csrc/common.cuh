@@ -94,22 +94,22 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Bounded wait: gives up after about a second (kWaitCycles SM clocks).  Returns
-// false when the limit ran out (the caller records a fault and leaves); never
-// spins forever.  mbarrier.try_wait without a time hint blocks for a short,
-// hardware-chosen time and returns as soon as the phase completes; the hinted form
-// compiles to sleep loops that add microseconds to every stage hand-over.
-constexpr long long kWaitCycles = 2000000000ll;
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+// Bounded wait: gives up after `limit` SM clocks.  Returns false when the limit ran out (the caller
+// records a fault and leaves); never spins forever.  mbarrier.try_wait without a time hint blocks for
+// a short, hardware-chosen time and returns as soon as the phase completes; the hinted form compiles
+// to sleep loops that add microseconds to every stage hand-over.
+__device__ __forceinline__ bool mbar_wait_for(uint32_t bar, uint32_t parity, long long limit) {
     if (mbar_test(bar, parity)) return true;
     const long long t0 = clock64();
     for (;;) {
 #pragma unroll 1
         for (int i = 0; i < 32; ++i)
             if (mbar_test(bar, parity)) return true;
-        if (clock64() - t0 > kWaitCycles) return false;
+        if (clock64() - t0 > limit) return false;
     }
 }
+constexpr long long kWaitCycles = 2000000000ll;  // about a second
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) { return mbar_wait_for(bar, parity, kWaitCycles); }
 
 // Bulk asynchronous copy global -> shared (TMA, untiled).  dst, src 16-byte
 // aligned, bytes a multiple of 16.  Completion is counted on `bar`.

@@ -249,20 +249,6 @@ __device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 
-// Bounded wait.  mbarrier.try_wait without a time hint blocks for a hardware-chosen short
-// time and returns as soon as the phase completes (the hinted form compiles to sleep
-// loops that add microseconds to every stage hand-over).
-__device__ __forceinline__ bool mbar_wait_for(uint32_t bar, uint32_t parity, long long limit) {
-    if (mbar_test(bar, parity)) return true;
-    const long long t0 = clock64();
-    for (;;) {
-#pragma unroll 1
-        for (int i = 0; i < 32; ++i)
-            if (mbar_test(bar, parity)) return true;
-        if (clock64() - t0 > limit) return false;
-    }
-}
-
 constexpr int kRingMaxSlots = 12;
 
 // 25 compute warps + the producer warp: 7 warps on one SM sub-partition at most, i.e. up to 72

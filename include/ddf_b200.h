@@ -119,6 +119,16 @@ int ddf_b200_forward_waitlimit(const void* x, const void* cf, const void* sf, vo
                                void* stream);
 
 /*
+ * The same for the band kernels: the forward into `out`, then the filter gradients into `gcf` / `gsf`
+ * (NULL: not run; `go` and the workspace are needed for them only, sized by ddf_b200_backward_workspace).
+ * DDF_B200_E_UNSUPPORTED where a band kernel is not built for the problem.
+ */
+int ddf_b200_band_waitlimit(const void* go, const void* x, const void* cf, const void* sf, void* out,
+                            void* gcf, void* gsf, void* workspace, size_t workspace_bytes,
+                            int B, int C, int H, int W, int k, int d, int s, int combine, int dtype,
+                            long long wait_cycles, int starve, void* stream);
+
+/*
  * The spatial FilterNorm on its own, for the backward of ddf_b200_forward_sfnorm.
  * ddf_b200_sfnorm writes the normalised filter (same shape and type as `raw`,
  * (B,k*k,H',W')) that ddf_b200_backward takes as `sf`; ddf_b200_sfnorm_backward turns the

@@ -103,3 +103,37 @@ def test_no_scratch_and_built_in_scratch(shape):
         for name, a, w in zip(("grad_x", "grad_cf", "grad_sf"), gs, want):
             check_close(a, w, torch.float32, name, reduction=name != "grad_x")
     assert all(torch.equal(a, b) for a, b in zip(got[0], got[2]))
+
+
+@pytest.mark.parametrize("shape", [(2, 150, 33, 45, 3, 1, 1), (3, 37, 9, 11, 3, 2, 1), (2, 60, 31, 29, 5, 1, 1), (2, 64, 50, 67, 3, 1, 2)])
+@pytest.mark.parametrize("dt", ["f32", "bf16"])
+def test_wait_limit_reports_a_fault_and_the_context_survives(shape, dt):
+    """Every stage is announced 16 bytes larger than what is copied, so that none completes: with a limit of
+    about a millisecond the compute warps give up, the kernels return, the fault word reads 1 and the next
+    calls give their results."""
+    from ddfnet_b200 import _lib
+    L = _lib.load()
+    B, C, H, W, k, d, s = shape
+    dc = {"f32": _lib.F32, "bf16": _lib.BF16}[dt]
+    (x, cf, sf, go), dev = _inputs(shape, dt, 6)
+    xd, cfd, sfd, god = dev
+    out, gcf, gsf = torch.empty_like(god), torch.empty_like(cfd), torch.empty_like(sfd)
+    ws = torch.empty(64 << 20, dtype=torch.uint8, device=xd.device)
+
+    def call(o, filters, limit, starve):
+        return L.ddf_b200_band_waitlimit(god.data_ptr(), xd.data_ptr(), cfd.data_ptr(), sfd.data_ptr(), o,
+                                         *([gcf.data_ptr(), gsf.data_ptr()] if filters else [None, None]),
+                                         ws.data_ptr(), ws.numel(), B, C, H, W, k, d, s, _lib.MUL, dc, limit, starve,
+                                         torch.cuda.current_stream().cuda_stream)
+
+    assert L.ddf_b200_take_fault() == 0
+    for o, filters in ((out.data_ptr(), False), (None, True)):
+        assert call(o, filters, 2_000_000, 1) == 0
+        assert L.ddf_b200_take_fault() == 1
+        assert L.ddf_b200_take_fault() == 0
+    assert call(out.data_ptr(), True, 2_000_000_000, 0) == 0
+    check_close(out, oracle_forward(x, cf, sf, k, d, s, "mul"), DTYPES[dt], "forward after a starved launch")
+    _, wcf, wsf = oracle_backward(go, x, cf, sf, k, d, s, "mul")
+    check_close(gcf, wcf, DTYPES[dt], "grad_cf after a starved launch", reduction=True)
+    check_close(gsf, wsf, DTYPES[dt], "grad_sf after a starved launch", reduction=True)
+    assert L.ddf_b200_take_fault() == 0

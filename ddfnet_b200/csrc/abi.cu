@@ -421,13 +421,13 @@ int ddf_b200_band_waitlimit(const void* go, const void* x, const void* cf, const
         if (rc) return rc == kNotHandled ? DDF_B200_E_UNSUPPORTED : rc;
     }
     if (gcf || gsf) {
-        size_t need = 0;
-        if (!band_filters_workspace(p, di->sm_count, &need)) return DDF_B200_E_UNSUPPORTED;
-        if (need > 0 && (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 7u) != 0))
+        size_t need = 0, least = 0;
+        if (!band_filters_workspace(p, di->sm_count, &need, &least)) return DDF_B200_E_UNSUPPORTED;
+        if (least > 0 && (!workspace || workspace_bytes < least || (reinterpret_cast<uintptr_t>(workspace) & 7u) != 0))
             return DDF_B200_E_WORKSPACE;
         int launches = 0;
-        rc = band_filters(p, go, x, cf, sf, gcf, gsf, workspace, di->sm_count, di->fault, di->index, st, &launches,
-                          wait_cycles, skew);
+        rc = band_filters(p, go, x, cf, sf, gcf, gsf, workspace, workspace_bytes, di->sm_count, di->fault, di->index,
+                          st, &launches, wait_cycles, skew);
         g_launches.fetch_add((unsigned long long)launches, std::memory_order_relaxed);
         if (rc) return rc == kNotHandled ? DDF_B200_E_UNSUPPORTED : rc;
     }
@@ -456,9 +456,9 @@ size_t ddf_b200_backward_workspace(int B, int C, int H, int W, int k, int d, int
     int sm = 148;
     if (device_info(di) == 0) sm = di->sm_count;
     // one call takes one of the two forms; AUTO may take either
-    size_t need = bwd_stream_supported(p) ? bwd_stream_workspace(p, sm) : 0, band = 0;
+    size_t need = bwd_stream_supported(p) ? bwd_stream_workspace(p, sm) : 0, band = 0, least = 0;
     if (variant == DDF_B200_VARIANT_AUTO && !(need > 0 && stream_worthwhile(p, sm)) &&
-        band_filters_workspace(p, sm, &band) && band > need)
+        band_filters_workspace(p, sm, &band, &least) && band > need)
         need = band;
     return need;
 }
@@ -537,11 +537,12 @@ int ddf_b200_backward(const void* go, const void* x, const void* cf, const void*
         }
         if (!done && variant == DDF_B200_VARIANT_STREAM) return DDF_B200_E_UNSUPPORTED;
         // the band form; a caller without scratch for it gets the generic kernels, which need none
-        size_t band = 0;
-        if (!done && allow_stream && band_filters_workspace(p, di->sm_count, &band) &&
-            (band == 0 || (workspace && workspace_bytes >= band && (reinterpret_cast<uintptr_t>(workspace) & 7u) == 0))) {
+        size_t band = 0, least = 0;
+        if (!done && allow_stream && band_filters_workspace(p, di->sm_count, &band, &least) &&
+            (least == 0 || (workspace && workspace_bytes >= least && (reinterpret_cast<uintptr_t>(workspace) & 7u) == 0))) {
             int launches = 0;
-            rc = band_filters(p, go, x, cf, sf, gcf, gsf, workspace, di->sm_count, di->fault, di->index, st, &launches);
+            rc = band_filters(p, go, x, cf, sf, gcf, gsf, workspace, workspace_bytes, di->sm_count, di->fault, di->index,
+                              st, &launches);
             if (rc == 0) {
                 done = true;
                 g_launches.fetch_add((unsigned long long)launches, std::memory_order_relaxed);

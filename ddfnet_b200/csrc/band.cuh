@@ -5,13 +5,14 @@
 
 namespace ddf {
 
-// Scratch bytes of the filter gradients (0 is possible); false when the band form is not built for p.
-bool band_filters_workspace(const Problem& p, int sm_count, size_t* bytes);
+// Scratch bytes of the filter gradients: what they take, and the least that they run with (0 is possible);
+// false when the band form is not built for p.
+bool band_filters_workspace(const Problem& p, int sm_count, size_t* bytes, size_t* least);
 
-// kNotHandled: not built, or a tensor is not aligned for bulk copies.  `workspace` holds what
-// band_filters_workspace says.
+// kNotHandled: not built, or a tensor is not aligned for bulk copies.  `workspace` holds at
+// least what band_filters_workspace says, aligned to 8 bytes; the results do not depend on how much.
 int band_filters(const Problem& p, const void* go, const void* x, const void* cf, const void* sf, void* gcf, void* gsf,
-                 void* workspace, int sm_count, int* fault, int device, cudaStream_t st, int* launches,
+                 void* workspace, size_t workspace_bytes, int sm_count, int* fault, int device, cudaStream_t st, int* launches,
                  long long wait_cycles = kWaitCycles, uint32_t tx_skew = 0);
 
 }  // namespace ddf

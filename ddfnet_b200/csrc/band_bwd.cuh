@@ -40,6 +40,10 @@ constexpr int kBandBwdThreads = 352;
 template <int K> constexpr int kBandBwdChunk = K == 3 ? 64 : 24;
 template <int K> constexpr int kBandBwdPixels = K == 3 ? 4 : 2;
 constexpr int kBandBwdParts = 32;  // gsf partials per element at most (unless the chunk limit asks for more)
+// Scratch asked for at most, unless one sample needs more: the partials can be several times x's bytes (k = 5,
+// 24 channels a chunk: twice), so a large batch goes through the scratch in slices of
+// samples.  A slice of this size is still some 3000 CTAs, ten waves.
+constexpr size_t kBandBwdScratch = 256u << 20;
 
 template <typename T> using BandPart = std::conditional_t<sizeof(T) == 4, double, float>;
 
@@ -53,6 +57,7 @@ struct BandBwdPlan {
     void* part_sf;     // [b][chunk][t][pixel], BandPart<T>; null: one chunk, rounded here
     float* part_cf;    // [b][band][c][t]; null likewise
     int C, H, W, OH, OW;
+    int b0;            // the slice's first sample
     int bands, groups, chunk, chunks, planes;
     int n_slots, n_warps, plane_warps;
     unsigned long long x_total, go_total;
@@ -103,7 +108,8 @@ band_filters_kernel(const __grid_constant__ BandBwdPlan pl) {
     const int band = item % pl.bands;
     item /= pl.bands;
     const int chunk_i = item % pl.chunks;
-    const int b = item / pl.chunks;
+    const int bs = item / pl.chunks;  // sample within the slice
+    const int b = pl.b0 + bs;
     const int c_lo = chunk_i * pl.chunk;
     const int c_hi = c_lo + pl.chunk < pl.C ? c_lo + pl.chunk : pl.C;
     const int npass = (c_hi - c_lo + G - 1) / G;
@@ -370,7 +376,7 @@ band_filters_kernel(const __grid_constant__ BandBwdPlan pl) {
             CompSum<float> tot;
             for (int w = 0; w < pl.plane_warps; ++w) tot.add(ldsf(src + 4u * (uint32_t)(w * KK)));
             if (pl.part_cf != nullptr)
-                pl.part_cf[(((long long)b * pl.bands + band) * pl.C + c_lo) * KK + e] = tot.value();
+                pl.part_cf[(((long long)bs * pl.bands + band) * pl.C + c_lo) * KK + e] = tot.value();
             else
                 Elem<T>::store(reinterpret_cast<T*>(pl.gcf) + (long long)first_plane * KK + e, tot.value());
         }
@@ -379,7 +385,7 @@ band_filters_kernel(const __grid_constant__ BandBwdPlan pl) {
         using P = BandPart<T>;
         P* ps = pl.part_sf == nullptr
                     ? nullptr
-                    : reinterpret_cast<P*>(pl.part_sf) + ((long long)b * pl.chunks + chunk_i) * KK * opl;
+                    : reinterpret_cast<P*>(pl.part_sf) + ((long long)bs * pl.chunks + chunk_i) * KK * opl;
         T* os = reinterpret_cast<T*>(pl.gsf) + (long long)b * KK * opl;
         auto put = [&](long long o, P v) {
             if (ps != nullptr) ps[o] = v;
@@ -495,12 +501,13 @@ inline bool band_filters_split(const Problem& p, int sm_count, BandBwdSplit& s) 
     return run <= (64 << 10);
 }
 
-// Floats that gsf / gcf partials take (0: none needed).
+// Bytes that one sample's gsf / gcf partials take (0: none needed).
 inline size_t band_part_sf(const Problem& p, const BandBwdSplit& s) {
-    return s.chunks > 1 ? (size_t)p.B * s.chunks * p.k * p.k * p.OH * p.OW * (p.dtype == DDF_B200_F32 ? 2 : 1) : 0;
+    return s.chunks > 1 ? (size_t)s.chunks * p.k * p.k * p.OH * p.OW *
+                              (p.dtype == DDF_B200_F32 ? sizeof(double) : sizeof(float)) : 0;
 }
 inline size_t band_part_cf(const Problem& p, const BandBwdSplit& s) {
-    return s.bands > 1 ? (size_t)p.B * s.bands * p.C * p.k * p.k : 0;
+    return s.bands > 1 ? (size_t)s.bands * p.C * p.k * p.k * sizeof(float) : 0;
 }
 
 struct BandBwdArgs {
@@ -511,6 +518,7 @@ struct BandBwdArgs {
     void* gcf;
     void* gsf;
     void* workspace;
+    size_t workspace_bytes;
     Problem p;
     int sm_count;
     int* fault;
@@ -528,10 +536,14 @@ int band_filters_launch(const BandBwdArgs& a, cudaStream_t stream, int* launches
     if (!band_filters_split(p, a.sm_count, sp)) return kNotHandled;
     BandBwdPlan pl;
     pl.go = a.go; pl.x = a.x; pl.cf = a.cf; pl.sf = a.sf; pl.gcf = a.gcf; pl.gsf = a.gsf;
+    // samples per slice: what the scratch holds
     const size_t n_sf = band_part_sf(p, sp), n_cf = band_part_cf(p, sp);
-    float* ws = reinterpret_cast<float*>(a.workspace);
+    const size_t fit = n_sf + n_cf > 0 ? a.workspace_bytes / (n_sf + n_cf) : (size_t)p.B;
+    if (fit < 1) return DDF_B200_E_WORKSPACE;
+    const int samples = fit < (size_t)p.B ? (int)fit : p.B;
+    char* ws = reinterpret_cast<char*>(a.workspace);
     pl.part_sf = a.gsf && n_sf ? ws : nullptr;
-    pl.part_cf = a.gcf && n_cf ? ws + n_sf : nullptr;
+    pl.part_cf = a.gcf && n_cf ? reinterpret_cast<float*>(ws + n_sf * (size_t)samples) : nullptr;
     pl.C = p.C; pl.H = p.H; pl.W = p.W; pl.OH = p.OH; pl.OW = p.OW;
     pl.bands = sp.bands; pl.groups = sp.groups; pl.chunk = sp.chunk; pl.chunks = sp.chunks; pl.planes = sp.planes;
     pl.n_warps = sp.warps;
@@ -570,20 +582,25 @@ int band_filters_launch(const BandBwdArgs& a, cudaStream_t stream, int* launches
         if (e != cudaSuccess) return (int)e;
         opted_in.fetch_or(bit, std::memory_order_release);
     }
-    cudaError_t e = launch_overlapped(kern, dim3((unsigned)(p.B * sp.bands * sp.chunks)),
-                                      dim3((unsigned)(sp.warps + 1) * 32), smem, stream, true, pl);
-    if (e != cudaSuccess) return (int)e;
-    ++*launches;
-    if (pl.part_sf || pl.part_cf) {
-        const long long sf_size = (long long)K * K * p.OH * p.OW, cf_size = (long long)p.C * K * K;
+    const long long sf_size = (long long)K * K * p.OH * p.OW, cf_size = (long long)p.C * K * K;
+    for (int b0 = 0; b0 < p.B; b0 += samples) {
+        const int nb = p.B - b0 < samples ? p.B - b0 : samples;
+        pl.b0 = b0;
+        cudaError_t e = launch_overlapped(kern, dim3((unsigned)(nb * sp.bands * sp.chunks)),
+                                          dim3((unsigned)(sp.warps + 1) * 32), smem, stream, true, pl);
+        if (e != cudaSuccess) return (int)e;
+        ++*launches;
+        if (!pl.part_sf && !pl.part_cf) continue;
         auto blocks = [&](long long n) {
             const long long most = 4ll * a.sm_count;
             return (int)((n + 255) / 256 < most ? (n + 255) / 256 : most);
         };
-        const int nb_sf = pl.part_sf ? blocks(sf_size * p.B) : 0, nb_cf = pl.part_cf ? blocks(cf_size * p.B) : 0;
+        const int nb_sf = pl.part_sf ? blocks(sf_size * nb) : 0, nb_cf = pl.part_cf ? blocks(cf_size * nb) : 0;
+        T* gsf = pl.part_sf ? reinterpret_cast<T*>(a.gsf) + b0 * sf_size : nullptr;
+        T* gcf = pl.part_cf ? reinterpret_cast<T*>(a.gcf) + b0 * cf_size : nullptr;
         e = launch_overlapped(band_reduce_kernel<T>, dim3((unsigned)(nb_sf + nb_cf)), dim3(256), 0, stream, true,
-                              (const BandPart<T>*)pl.part_sf, reinterpret_cast<T*>(a.gsf), sp.chunks, sf_size,
-                              (const float*)pl.part_cf, reinterpret_cast<T*>(a.gcf), sp.bands, cf_size, p.B, nb_sf);
+                              (const BandPart<T>*)pl.part_sf, gsf, sp.chunks, sf_size, (const float*)pl.part_cf, gcf, sp.bands,
+                              cf_size, nb, nb_sf);
         if (e != cudaSuccess) return (int)e;
         ++*launches;
     }

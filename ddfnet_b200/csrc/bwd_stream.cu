@@ -150,10 +150,10 @@ int ddf_b200_backward_noalloc(const void* go, const void* x, const void* cf, con
                                 reinterpret_cast<cudaStream_t>(stream), &launches);
         if (rc != kNotHandled) return rc;
     }
-    // Outside the streaming kernel's range: the band kernel where its scratch fits the array, else the
-    // generic kernels, which use no scratch at all.
-    size_t band = 0;
-    if (band_filters_workspace(p, sm_count, &band) && band <= kStaticScratchBytes) {
+    // Outside the streaming kernel's range: the band kernel where the array holds its scratch for one sample,
+    // else the generic kernels, which use no scratch at all.
+    size_t band = 0, least = 0;
+    if (band_filters_workspace(p, sm_count, &band, &least) && least <= kStaticScratchBytes) {
         void* scratch = nullptr;
         rc = static_scratch_address(index, &scratch);
         if (rc) return rc;

@@ -199,8 +199,9 @@ int ddf_b200_plan(int B, int C, int H, int W, int k, int d, int s,
 
 /*
  * Bytes of scratch the backward needs for this problem (0 is possible).  Where
- * ddf_b200_plan says GENERIC, less scratch (or none) is no error: the filter
- * gradients then run on the generic kernels instead of the band kernels.
+ * ddf_b200_plan says GENERIC it is at most 256 MiB, unless a single sample needs more,
+ * and less scratch (or none) is no error: the filter gradients then take fewer samples
+ * at a time, with the same results, or, without room for one, the generic kernels.
  * The reference makes its caller allocate three zero-filled scratch tensors
  * (ddf/ddf.py:106-108, resized in ddf/src/cuda/ddf_mul_cuda.cpp:85-87); here the
  * caller provides one untyped block, 256-byte aligned, which need not be zeroed.
@@ -243,7 +244,8 @@ int ddf_b200_backward(const void* go, const void* x, const void* cf, const void*
  *   - Problems of the plane-streaming kernels (ddf_b200_plan says STREAM) whose
  *     scratch need (what ddf_b200_backward_workspace reports) exceeds that limit
  *     are refused with DDF_B200_E_SCRATCH_LIMIT before anything is launched; any
- *     other problem runs, on the generic kernels where the array is too small.
+ *     other problem runs, on the generic kernels where the array is too small for
+ *     one sample.
  *   - The call itself performs no cudaMalloc / cudaFree and uses no allocating
  *     library routine.
  *   - The first call on each device looks up the array's device address (one

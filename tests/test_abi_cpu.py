@@ -112,3 +112,12 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(lib, "_lib", None)
     with pytest.raises(RuntimeError, match="no CPU or PyTorch fallback"):
         lib.load()
+
+
+def test_the_band_kernels_scratch_is_bounded(L):
+    """Several times x's size if all samples were in flight (k = 5, few channels a chunk)."""
+    B, C, H, W = 64, 500, 150, 151
+    for dtype in (0, 1, 2):
+        one = L.ddf_b200_backward_workspace(1, C, H, W, 5, 1, 1, 0, dtype, 0)
+        need = L.ddf_b200_backward_workspace(B, C, H, W, 5, 1, 1, 0, dtype, 0)
+        assert 0 < need <= max(256 << 20, one)

@@ -158,3 +158,27 @@ def test_filter_gradients_are_as_exact_as_the_generic_kernels(shape, dt, mode):
         err[version] = [((g.double() - w).norm() / w.norm()).item() for g, w in zip(got, want)]
     for a, b in zip(err[""], err["o"]):
         assert a <= b * (1.03 if dt == "f32" else 1.0001), err
+
+
+@pytest.mark.parametrize("shape,dt", [((5, 60, 50, 67, 3, 1, 1), "f32"), ((3, 75, 31, 29, 5, 1, 1), "bf16"), ((7, 75, 33, 31, 3, 1, 2), "f16")])
+def test_less_scratch_gives_the_same_bits(shape, dt):
+    """The samples go through the scratch in slices of what it holds, down to one."""
+    from ddfnet_b200 import _lib
+    L = _lib.load()
+    B, C, H, W, k, d, s = shape
+    dc = {"f32": _lib.F32, "f16": _lib.F16, "bf16": _lib.BF16}[dt]
+    _, dev = _inputs(shape, dt, 8)
+    need = int(L.ddf_b200_backward_workspace(B, C, H, W, k, d, s, _lib.ADD, dc, _lib.VARIANT_AUTO))
+    assert need > 0 and need % B == 0
+    ws, got = torch.empty(need, dtype=torch.uint8, device="cuda"), []
+    for samples in (B, B - 1, 2, 1):
+        ws.fill_(0xff)
+        g = [torch.empty_like(t) for t in dev[1:3]]
+        before = L.ddf_b200_launch_count()
+        assert L.ddf_b200_backward(dev[3].data_ptr(), *(t.data_ptr() for t in dev[:3]), None, *(t.data_ptr() for t in g),
+                                   ws.data_ptr(), need // B * samples, B, C, H, W, k, d, s, _lib.ADD, dc,
+                                   _lib.VARIANT_AUTO, torch.cuda.current_stream().cuda_stream) == 0
+        assert L.ddf_b200_launch_count() - before == 2 * -(-B // samples)
+        got.append(g)
+    for g in got[1:]:
+        assert torch.equal(g[0], got[0][0]) and torch.equal(g[1], got[0][1])

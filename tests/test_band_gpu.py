@@ -5,7 +5,7 @@ does not divide -- and non-finite values next to the padding."""
 import pytest
 import torch
 
-from tests.util import DTYPES, check_close, make_inputs, oracle_backward, oracle_forward
+from tests.util import DTYPES, check_close, check_extremes, make_inputs, oracle_backward, oracle_forward
 
 pytestmark = pytest.mark.gpu
 
@@ -17,6 +17,9 @@ SHAPES = [
     (1, 8, 200, 321, 3, 1, 1),   # wider: the generic kernels
     (2, 5, 33, 200, 3, 2, 1), (1, 5, 19, 299, 5, 2, 1),   # dilated, too wide for both residues in a band
     (1, 3, 9, 320, 3, 2, 1),     # ... and a band beyond the plane's last row
+    # k = 5: the widest band of the filter gradients and of the other two, and one column more
+    (1, 3, 9, 320, 5, 1, 1), (1, 3, 9, 321, 5, 2, 1), (1, 3, 13, 352, 5, 1, 1), (1, 3, 9, 353, 5, 1, 1),
+    (1, 3, 11, 640, 3, 1, 2), (1, 3, 10, 641, 3, 1, 2), (1, 3, 11, 642, 3, 1, 2),   # the widest at stride 2, and wider
     (1, 70, 101, 75, 3, 2, 1), (3, 67, 50, 67, 3, 1, 1), (2, 131, 101, 75, 3, 1, 2), (1, 24, 61, 99, 5, 1, 1),
     (1, 24, 63, 101, 5, 2, 1), (1, 40, 30, 167, 5, 2, 1), (40, 75, 17, 13, 3, 1, 1),
 ]
@@ -46,24 +49,83 @@ def test_matches_oracle(shape, dt, mode):
     assert _lib.load().ddf_b200_take_fault() == 0
 
 
-@pytest.mark.parametrize("shape", [(1, 70, 101, 75, 3, 2, 1), (1, 24, 63, 101, 5, 1, 1), (2, 131, 51, 75, 3, 1, 2)])
+EXTREME = [(1, 70, 101, 75, 3, 2, 1), (1, 24, 63, 101, 5, 1, 1), (2, 131, 51, 75, 3, 1, 2)]
+
+
+@pytest.mark.parametrize("shape", EXTREME)
 @pytest.mark.parametrize("which", [0, 1, 2, 3])
 @pytest.mark.parametrize("dt", ["f32", "bf16"])
-def test_padding_is_skipped_not_multiplied(shape, which, dt):
-    """An infinity in one operand reaches exactly the results it reaches in the generic kernels, which
-    skip taps outside the plane."""
+@pytest.mark.parametrize("version", ["", "o"])
+def test_padding_is_skipped_not_multiplied(shape, which, dt, version):
+    """An infinity in one operand reaches exactly the results it reaches in the oracle, which skips taps
+    outside the plane, and leaves the others as they are.  (The filter gradients' compensated sums make NaN of
+    an infinity; their other values are compared.)"""
     from ddfnet_b200 import ddf
     k, d, s = shape[4:]
     for mode in ("mul", "add"):
-        _, t = _inputs(shape, dt, 9)
-        t[which].view(-1)[::37] = float("inf")
-        res = []
-        for version in ("", "o"):
-            ts = [v.clone().requires_grad_() for v in t[:3]]
-            out = ddf(*ts, k, d, s, mode, version)
-            res.append((out, *torch.autograd.grad(out, ts, t[3])))
-        for name, a, b in zip(("out", "grad_x", "grad_cf", "grad_sf"), *res):
-            assert torch.equal(torch.isfinite(a), torch.isfinite(b)), f"{name} {mode}"
+        cpu, t = _inputs(shape, dt, 9)
+        for v in (cpu[which], t[which]):
+            v.view(-1)[::37] = float("inf")
+            v.view(-1)[5::411] = float("-inf")
+        x, cf, sf, go = cpu
+        ts = [v.clone().requires_grad_() for v in t[:3]]
+        out = ddf(*ts, k, d, s, mode, version)
+        gx, gcf, gsf = torch.autograd.grad(out, ts, t[3])
+        wx, wcf, wsf = oracle_backward(go, x, cf, sf, k, d, s, mode)
+        check_extremes(out, oracle_forward(x, cf, sf, k, d, s, mode), DTYPES[dt], f"out {mode}")
+        check_extremes(gx, wx, DTYPES[dt], f"grad_x {mode}")
+        for name, g, w in (("grad_cf", gcf, wcf), ("grad_sf", gsf, wsf)):
+            fin = torch.isfinite(w)
+            assert torch.equal(torch.isfinite(g).cpu(), fin), f"{name} {mode}"
+            zero = torch.zeros((), dtype=torch.float64)
+            check_close(torch.where(fin, g.cpu().double(), zero), torch.where(fin, w, zero), DTYPES[dt], f"{name} {mode}",
+                        reduction=True)
+
+
+@pytest.mark.parametrize("shape", EXTREME + [(3, 37, 9, 11, 3, 1, 1), (1, 24, 63, 101, 5, 2, 1)])
+@pytest.mark.parametrize("which", [1, 2])
+@pytest.mark.parametrize("dt", ["f32", "bf16"])
+@pytest.mark.parametrize("mode", ["mul", "add"])
+def test_large_filter_values(shape, which, dt, mode):
+    """Filter values from 1e18 on, whose products with padding zeros would be no safe zeros, take the loop that
+    skips the padding: every value of it.  At most one such value in a window, so that none cancels; the filter
+    gradients, sums of several, are held in the 2-norm."""
+    from ddfnet_b200 import ddf
+    k, d, s = shape[4:]
+    cpu, t = _inputs(shape, dt, 10)
+    for v in (cpu[which], t[which]):
+        v.view(-1)[:: (211 if which == 1 else 1009)] = 2e18
+    x, cf, sf, go = cpu
+    ts = [v.clone().requires_grad_() for v in t[:3]]
+    out = ddf(*ts, k, d, s, mode)
+    gx, *filters = torch.autograd.grad(out, ts, t[3])
+    wx, *want = oracle_backward(go, x, cf, sf, k, d, s, mode)
+    check_close(out, oracle_forward(x, cf, sf, k, d, s, mode), DTYPES[dt], "out")
+    check_close(gx, wx, DTYPES[dt], "grad_x")
+    for g, w in zip(filters, want):
+        assert (g.cpu().double() - w).norm() <= (1e-6 if dt == "f32" else 4e-3) * w.norm()
+
+
+@pytest.mark.parametrize("shape", [(2, 300, 60, 63, 3, 1, 1), (300, 40, 14, 13, 3, 2, 1), (2, 300, 45, 47, 5, 1, 1), (4, 200, 61, 63, 3, 1, 2),
+                                   (1, 96, 75, 301, 5, 2, 1)])
+@pytest.mark.parametrize("dt", ["f32", "bf16"])
+@pytest.mark.parametrize("mode", ["mul", "add"])
+def test_results_do_not_change_between_runs(shape, dt, mode):
+    """Every CTA walks several times more stages than its ring has slots: a value read after its slot was handed
+    back would show as a difference between runs (there are no atomics: equal inputs give equal bits)."""
+    from ddfnet_b200 import _lib, ddf
+    k, d, s = shape[4:]
+    _, t = _inputs(shape, dt, 11)
+    ts = [v.requires_grad_() for v in t[:3]]
+
+    def results():
+        out = ddf(*ts, k, d, s, mode)
+        return [out, *torch.autograd.grad(out, ts, t[3])]
+
+    first = results()
+    for _ in range(30):
+        assert all(torch.equal(a, b) for a, b in zip(results(), first))
+    assert _lib.load().ddf_b200_take_fault() == 0
 
 
 def test_spatial_norm_inside_the_kernel():

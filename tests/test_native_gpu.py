@@ -84,3 +84,93 @@ def test_a_profiler_shows_the_call_and_its_backward(fused, name):
         _entry(fused)(*ts).sum().backward()
     seen = {e.key for e in prof.key_averages()}
     assert {name, name + "Backward"} <= seen
+
+
+def _gradients(ts, go, **kw):
+    out = _entry(False)(*ts)
+    return torch.autograd.grad(out, ts, go, **kw)
+
+
+def test_backward_on_another_stream_and_in_two_threads():
+    import threading
+    B, C, H, W = SHAPE
+    sets = [_inputs(20 + i, "f16", grad=True) for i in range(2)]
+    want = [_gradients(s[:3], s[3]) for s in sets]
+    torch.cuda.synchronize()
+    got, errors = [None, None], []
+
+    def work(i):
+        try:
+            stream = torch.cuda.Stream()
+            with torch.cuda.stream(stream):
+                for _ in range(50):
+                    got[i] = _gradients(sets[i][:3], sets[i][3])
+            stream.synchronize()
+        except Exception as e:  # a thread's exception would be lost
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
+    for g, w in zip(got, want):
+        assert all(torch.equal(a, b) for a, b in zip(g, w))
+
+
+def test_gradients_have_their_inputs_types():
+    x, cf, sf, go = _inputs(7)
+    ts = [x.half().requires_grad_(), cf.requires_grad_(), sf.half().requires_grad_()]
+    out = _entry(False)(*ts)
+    assert out.dtype == torch.float32
+    got = torch.autograd.grad(out, ts, go)
+    want = _gradients([t.detach().float().requires_grad_() for t in ts], go)
+    for g, t, w in zip(got, ts, want):
+        assert g.dtype == t.dtype and torch.equal(g, w.to(t.dtype))
+
+
+@pytest.mark.parametrize("need", [(1, 0, 0), (0, 1, 0), (0, 0, 1), (1, 0, 1)])
+def test_only_the_gradients_that_are_asked_for(need):
+    ts = _inputs(8)
+    full = _gradients([t.detach().requires_grad_() for t in ts[:3]], ts[3])
+    some = [t.detach().requires_grad_(bool(n)) for t, n in zip(ts[:3], need)]
+    _entry(False)(*some).backward(ts[3])
+    for t, n, f in zip(some, need, full):
+        assert (t.grad is None) == (not n) and (not n or torch.equal(t.grad, f))
+
+
+def test_saved_tensors_pass_through_hooks():
+    ts = _inputs(9, grad=True)
+    want, packed = _gradients(ts[:3], ts[3]), []
+
+    def pack(t):
+        packed.append(t.shape)
+        return t.cpu()
+
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t.cuda()):
+        out = _entry(False)(*ts[:3])
+    assert len(packed) == 3
+    assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(out, ts[:3], ts[3]), want))
+
+
+def test_changed_inputs_and_a_second_backward_are_noticed():
+    ts = _inputs(10, grad=True)
+    out = _entry(False)(*ts[:3])
+    with torch.no_grad():
+        ts[1].mul_(2)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        out.sum().backward()
+    out = _entry(False)(*ts[:3])
+    out.sum().backward()
+    with pytest.raises(RuntimeError, match="second time"):
+        out.sum().backward()
+
+
+def test_no_history_without_a_gradient_to_record():
+    ts = _inputs(11, grad=True)
+    with torch.no_grad():
+        assert not _entry(False)(*ts[:3]).requires_grad
+    with torch.inference_mode():
+        assert _entry(False)(*ts[:3]).is_inference()
+    assert not _entry(False)(*(t.detach() for t in ts[:3])).requires_grad

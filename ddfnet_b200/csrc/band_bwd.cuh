@@ -1,5 +1,5 @@
-// Band form of the two filter gradients, for planes of any height and width (see band_fwd.cuh for the
-// bands, the ring and the thread layout):
+// Band form of the two filter gradients, for planes of any height and any width up to 320 output columns (see
+// band_fwd.cuh for the bands, the ring and the thread layout):
 //
 //   gcf[b,c,t]   = sum_{y,x} go[b,c,y,x] * x[b,c,y*s+oi,x*s+oj] * (sf[b,t,y,x] | 1)
 //   gsf[b,t,y,x] = sum_c     go[b,c,y,x] * x[b,c,y*s+oi,x*s+oj] * (cf[b,c,t]   | 1)

@@ -1,5 +1,6 @@
-// Band kernel: DDF forward (and grad-x at stride 1) for planes of ANY height and width, k = 3 and 5,
-// dilation 1 and 2 (stride 1) or stride 2 (k = 3, dilation 1), float and the 2-byte types.  It takes
+// Band kernel: DDF forward (and grad-x at stride 1) for planes of any height and any width up to 320 output
+// columns (352 at k = 5: a band holds whole rows, a CTA a column per thread), k = 3 and 5, dilation 1 and 2
+// (stride 1) or stride 2 (k = 3, dilation 1), float and the 2-byte types.  It takes
 // what the plane kernels (row, ring, stream) decline: planes too large for one CTA's threads, widths
 // that no vector divides, H or W that the stride does not divide, channel counts without a factor.
 //
@@ -16,11 +17,12 @@
 // filter values stay in registers, paired (p, p + PH/2) for the two-wide FMA.  A column of the window is
 // loaded once and serves k taps of PH pixels.
 //
-// What bounds it: instruction issue and the latency of a pass at 20 warps per SM (57% of issue slots busy,
-// DRAM at 21%, shared loads at 31%), and on small problems the filters' way into registers: one pointer per
-// pixel instead of an address per value took (4,128,50x67) f16 from 17.7 to 11.3 us.  (2,256,200x300) f32:
-// 80 us, 3.1 TB/s; the generic kernel 655.  Eight pixels per thread instead of four (half the CTAs fit): 97;
-// scalar instead of two-wide FMAs: 93 (k = 5, (8,96,75x101): 50 against 58 before the pointers, 48 after).
+// What bounds it: instruction issue and the latency of a pass at 20 warps per SM ((2,256,200x300) f32: 57% of
+// issue slots busy, DRAM at 31% of its peak, shared loads at 29%), and on small problems the filters' way into
+// registers: one pointer per pixel instead of an address per value took (4,128,50x67) f16 from 17.7 to 11.3 us.
+// (2,256,200x300) f32: 80 us, 3.1 TB/s; the generic kernel 655.  Eight pixels per thread instead of four (half
+// the CTAs fit): 97; scalar instead of two-wide FMAs: 93 (k = 5, (8,96,75x101): 50 against 58 before the
+// pointers, 48 after).
 //
 // Zero padding.  Rows outside the plane are read from a zeroed spot of the slot (their offset is a
 // per-thread constant), columns outside are masked.  A zero times an infinite filter value would be

@@ -279,6 +279,26 @@ static bool stream_worthwhile(const Problem& p, int sm_count) {
     return planes >= sm_count && bytes >= (256ll << 10);
 }
 
+// AUTO prefers the band forward and grad-x to the generic kernels except, us of both in a graph:
+//  - planes of one row, where most taps are padding, which the generic kernels skip: (16,64,1x100) f16 forward
+//    5.8 against 3.5, grad-x 8.3 against 4.1, (4096,64,1x7) f32 k = 5 155 against 30; and of one column, unless
+//    there are very many: (64,64,7x1) f32 1.2 times, but (64,64,300x1) f32 k = 5 18 against 31 (at 2^19 outputs
+//    the two are level);
+//  - planes of fewer than nine pixels: (256,64,2x2) f16 5.1 against 3.9, (4096,2048,1x1) f32 k = 5 2916 against
+//    134; (256,16,3x3) f32 is 4.0 against 4.5 (k = 5, 3x3: 0.7 times for few samples, 1.6 at (8000,64));
+//  - more samples than four CTAs per SM take at once, each with little work: a change of sample costs 2 to 3 us
+//    (k = 5: 4 to 7).  (4096,1,5x5) f16 15 against 5.2, (600,4,5x5) f32 5.6 against 4.7; with 162 outputs a sample
+//    ((2000,2,9x9) f32 k = 5) 0.87 times.
+// Elsewhere it wins from the smallest size on: (1,16,7x7) f16 3.6 against 3.9, (1,256,14x14) f16 3.7 against
+// 4.4, (2,64,29x31) f32 4.1 against 5.3, (1,16,33x31) f16 k = 5 5.3 against 7.8, (2,256,200x300) f32 80 against
+// 655.  The filter gradients win everywhere ((1,16,7x7) f16 7.7 against 11.3, (1,2048,1x1) f16 18 against 193).
+static bool band_worthwhile(const Problem& p, int sm_count) {
+    const long long pixels = (long long)p.OH * p.OW;
+    if (p.OH == 1 || pixels < 9) return false;
+    if (p.OW == 1 && p.B * (long long)p.C * pixels < (1ll << 19)) return false;
+    return p.C * pixels >= 160 || p.B <= 4 * sm_count;
+}
+
 // Forward for a checked problem: the streaming kernel where it applies, else the generic one.
 static int forward_impl(const Problem& p, const void* x, const void* cf, const void* sf, void* out,
                         int variant, void* stream) {
@@ -305,12 +325,10 @@ static int forward_impl(const Problem& p, const void* x, const void* cf, const v
             if (rc != kNotHandled) return rc;
         }
         if (variant == DDF_B200_VARIANT_STREAM) return DDF_B200_E_UNSUPPORTED;
-        // AUTO's next choice wins over the generic kernel at every size measured, in a graph: (1,16,7x7)
-        // f16 3.6 us against 3.9, (1,256,14x14) f16 3.7 against 4.4, (2,64,29x31) f32 4.1 against 5.3,
-        // (1,16,33x31) f16 at k = 5 5.3 against 7.8, (2,256,200x300) f32 80 against 655; its gradients
-        // likewise ((1,16,7x7) f16: grad-x 4.2 against 5.3, filters 7.7 against 11.3).
-        rc = run_band(BandArgs{x, cf, sf, out, p, false, di->sm_count, di->fault, di->index}, st);
-        if (rc != kNotHandled) return rc;
+        if (band_worthwhile(p, di->sm_count)) {
+            rc = run_band(BandArgs{x, cf, sf, out, p, false, di->sm_count, di->fault, di->index}, st);
+            if (rc != kNotHandled) return rc;
+        }
     }
     return run_generic_forward(p, x, cf, sf, out, di->sm_count, st);
 }
@@ -510,7 +528,7 @@ int ddf_b200_backward(const void* go, const void* x, const void* cf, const void*
             }
             if (!done && variant == DDF_B200_VARIANT_STREAM) return DDF_B200_E_UNSUPPORTED;
         }
-        if (!done && allow_stream) {
+        if (!done && allow_stream && band_worthwhile(p, di->sm_count)) {
             rc = run_band(BandArgs{go, cf, sf, gx, p, true, di->sm_count, di->fault, di->index}, st);
             if (rc == 0) done = true;
             else if (rc != kNotHandled) return rc;

@@ -193,7 +193,7 @@ int ddf_b200_rate_probe(int mode, void* scratch, size_t scratch_bytes, int iters
 /* Which variant (GENERIC or STREAM) AUTO resolves to for this problem; pointers
  * are assumed 16-byte aligned.  `backward` = 0 for the forward, 1 for the backward.
  * Returns a DDF_B200_VARIANT_* value, or a negative status.  GENERIC covers the band
- * kernels too, which AUTO prefers to the generic ones where they are built. */
+ * kernels too, which AUTO prefers to the generic ones where they are built and faster. */
 int ddf_b200_plan(int B, int C, int H, int W, int k, int d, int s,
                   int combine, int dtype, int backward);
 

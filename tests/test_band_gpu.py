@@ -22,6 +22,10 @@ SHAPES = [
     (1, 3, 11, 640, 3, 1, 2), (1, 3, 10, 641, 3, 1, 2), (1, 3, 11, 642, 3, 1, 2),   # the widest at stride 2, and wider
     (1, 70, 101, 75, 3, 2, 1), (3, 67, 50, 67, 3, 1, 1), (2, 131, 101, 75, 3, 1, 2), (1, 24, 61, 99, 5, 1, 1),
     (1, 24, 63, 101, 5, 2, 1), (1, 40, 30, 167, 5, 2, 1), (40, 75, 17, 13, 3, 1, 1),
+    # both sides of where the forward and grad-x leave small planes to the generic kernels: pixels of a plane, one
+    # column and few or many planes, samples and work in each
+    (3, 50, 2, 4, 3, 1, 1), (3, 50, 3, 3, 3, 1, 1), (3, 20, 33, 1, 5, 1, 1), (40, 400, 33, 1, 5, 1, 1),
+    (600, 10, 5, 3, 3, 2, 1), (600, 11, 5, 3, 3, 2, 1), (592, 3, 7, 6, 5, 1, 1), (593, 3, 7, 6, 5, 1, 1),
 ]
 
 

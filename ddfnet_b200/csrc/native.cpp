@@ -20,7 +20,6 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/record_function.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
-#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -28,7 +27,6 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
-#include <torch/csrc/jit/frontend/tracer.h>
 
 #include <cstring>
 #include <string>
@@ -234,9 +232,11 @@ bool parse(PyObject* const* args, Py_ssize_t n, bool norm, Params& p, const Tens
 
 // Nothing watches or transforms the program (see the head of this file).
 bool ordinary(std::initializer_list<const Tensor*> tensors) {
-    if (torch::jit::tracer::isTracing() || c10::impl::TorchDispatchModeTLS::any_modes_set() ||
-        c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode))
-        return false;
+    using c10::DispatchKey;
+    // set while a thread traces, has a dispatch mode, is inside a functorch transform
+    constexpr c10::DispatchKeySet watching({DispatchKey::Tracer, DispatchKey::Python,
+                                            DispatchKey::FuncTorchDynamicLayerFrontMode});
+    if (c10::impl::tls_local_dispatch_key_set().included_.has_any(watching)) return false;
     for (const Tensor* t : tensors)  // wrappers hold no storage of their own
         if (!t->has_storage() || torch::autograd::isFwGradDefined(*t)) return false;
     return true;

@@ -141,7 +141,9 @@ struct RingGeo {
     // static alignment (bytes) of a thread's window base inside a stage
     static constexpr int ALIGN = cgcd(16, cgcd(PH * S * WIN * 2, PW * S * 2));
     static constexpr int CFS = (KK + 3) / 4 * 4;   // entries per plane of the converted channel filter
-    static constexpr int CFP = CFS * 4;            // bytes per plane of it (floats for mul, halves for add)
+    // bytes per plane of it: floats for mul, halves for add; k = 5 (mul alone): (c, c) pairs, a tap row in whole 16s
+    static constexpr int CFR = (K * 8 + 15) / 16 * 16;
+    static constexpr int CFP = K == 3 ? CFS * 4 : K * CFR;
     static constexpr int CW = CFS;      // words a thread holds of it: floats (mul) / packed halves (add)
     static constexpr int NLW = (HALO + 1) / 2;                               // window words left of the patch
     static constexpr int NRW = ((PW - 1) * S + HALO) / 2 - PW * S / 2 + 1 > 0 ? ((PW - 1) * S + HALO) / 2 - PW * S / 2 + 1 : 0;   // and right of it
@@ -235,6 +237,45 @@ struct RingPlane {
     }
 };
 
+// The same for k = 5, mul: the filter's tap rows come one after the other (its 25 values and the 50 words of the
+// spatial filter do not fit the registers together), and two pixels take the float filter value in one instruction.
+template <typename T, typename G, int K, int PW, int PH>
+__device__ __forceinline__ void ring_plane_rows(uint32_t tb, uint32_t zb, uint32_t rowsel,
+                                                const uint32_t (&lmask)[G::NLW > 0 ? G::NLW : 1],
+                                                const uint32_t (&rmask)[G::NRW > 0 ? G::NRW : 1],
+                                                const uint32_t (&sfw)[K * K][PW * PH / 2], uint32_t cfa, float (&res)[PW * PH]) {
+    constexpr int P = PW * PH;
+    uint32_t w[G::NR][G::NWIN];
+    RingPlane<T, G, K, 1, 1, PW, PH, DDF_B200_MUL>::template Rows<0>::load(tb, zb, rowsel, lmask, rmask, w);
+    unsigned long long acc2[P / 2];
+#pragma unroll
+    for (int q = 0; q < P / 2; ++q) acc2[q] = 0ull;
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+        unsigned long long cc[(K + 1) / 2 * 2];
+#pragma unroll
+        for (int t = 0; t < (K + 1) / 2; ++t)
+            asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(cc[2 * t]), "=l"(cc[2 * t + 1])
+                         : "r"(cfa + (uint32_t)(i * G::CFR + 16 * t)));
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+#pragma unroll
+            for (int q = 0; q < P / 2; ++q) {
+                float y[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int pp = 2 * q + h, n = pp / PW + i;
+                    const int idx = pp % PW + j - G::R - 2 * G::w0(0);   // element within the row window
+                    y[h] = Mix<T>::fmaw(idx & 1, h, w[n][idx / 2], sfw[i * K + j][q], 0.f);
+                }
+                acc2[q] = f2_fma(f2_pack(y[0], y[1]), cc[j], acc2[q]);
+            }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < P / 2; ++q) f2_unpack(acc2[q], res[2 * q], res[2 * q + 1]);
+}
+
 // Non-blocking probe (mbarrier.test_wait): the issuing thread must never be parked on a
 // barrier that other warps complete much later.
 __device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity) {
@@ -253,16 +294,18 @@ constexpr int kRingMaxSlots = 12;
 
 // 25 compute warps + the producer warp: 7 warps on one SM sub-partition at most, i.e. up to 72
 // registers per thread.
-constexpr int kRingMaxThreads = 832;
+// k = 5: 50 words of spatial filter a thread, 16 warps of up to 128 registers.
+template <int K> constexpr int kRingMaxThreads = K == 3 ? 832 : 512;
 
 template <typename T, int K, int D, int S, int PW, int PH, int WIN, int MODE, bool BWDX>
-__global__ void __launch_bounds__(kRingMaxThreads, 1)
+__global__ void __launch_bounds__(kRingMaxThreads<K>, 1)
 ring_kernel(const __grid_constant__ RingPlan pl) {
     using G = RingGeo<K, D, S, PW, PH, WIN>;
     constexpr int KK = G::KK;
     constexpr int P = G::P;
     static_assert(!BWDX || S == 1, "grad-x ring kernel is stride 1 only");
     static_assert(sizeof(T) == 2, "2-byte element types only");
+    static_assert(K == 3 || (K == 5 && D == 1 && S == 1 && MODE == DDF_B200_MUL), "k = 5: mul, dilation 1, stride 1");
 
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const uint32_t sbase = smem_u32(smem_raw);
@@ -439,7 +482,8 @@ ring_kernel(const __grid_constant__ RingPlan pl) {
                 const int tt = BWDX ? KK - 1 - t : t;          // grad-x reads the filter mirrored
                 const uint32_t raw = lds16(src + 2u * (uint32_t)((pq * TG + g_lo + gi) * KK + t));
                 const uint32_t dst = cfw + (uint32_t)((pq * 2 + gi) * G::CFP);
-                if constexpr (MODE == DDF_B200_MUL) sts32(dst + 4u * (uint32_t)tt, Mix<T>::f32_bits(raw));
+                if constexpr (K != 3) sts64(dst + (uint32_t)(tt / K * G::CFR + tt % K * 8), Mix<T>::f32_bits(raw), Mix<T>::f32_bits(raw));
+                else if constexpr (MODE == DDF_B200_MUL) sts32(dst + 4u * (uint32_t)tt, Mix<T>::f32_bits(raw));
                 else sts16(dst + 2u * (uint32_t)tt, raw);
             }
             __syncwarp();
@@ -502,17 +546,21 @@ ring_kernel(const __grid_constant__ RingPlan pl) {
             if (to_next_sample == 0) to_next_sample = sample_passes;
 #pragma unroll 1
             for (; run > 0; --run) {
-                // the plane's converted channel filter: KK floats (mul) or KK packed halves (add)
-                uint32_t c[G::CFS];
-                constexpr int CWORDS = MODE == DDF_B200_MUL ? KK : (KK + 1) / 2;
-                constexpr int NV = CWORDS / 4, REM = CWORDS % 4;
-#pragma unroll
-                for (int v = 0; v < NV; ++v) lds128(cfa + 16u * v, c[4 * v], c[4 * v + 1], c[4 * v + 2], c[4 * v + 3]);
-                if constexpr (REM == 1) c[4 * NV] = lds32(cfa + 16u * NV);
-                else if constexpr (REM == 2) lds64(cfa + 16u * NV, c[4 * NV], c[4 * NV + 1]);
-                else if constexpr (REM == 3) lds128(cfa + 16u * NV, c[4 * NV], c[4 * NV + 1], c[4 * NV + 2], c[4 * NV + 3]);
                 float res[P];
-                RingPlane<T, G, K, D, S, PW, PH, MODE>::run(tb, zb, rowsel, lmask, rmask, sfw, c, res);
+                if constexpr (K != 3) {
+                    ring_plane_rows<T, G, K, PW, PH>(tb, zb, rowsel, lmask, rmask, sfw, cfa, res);
+                } else {
+                    // the plane's converted channel filter: KK floats (mul) or KK packed halves (add)
+                    uint32_t c[G::CFS];
+                    constexpr int CWORDS = MODE == DDF_B200_MUL ? KK : (KK + 1) / 2;
+                    constexpr int NV = CWORDS / 4, REM = CWORDS % 4;
+#pragma unroll
+                    for (int v = 0; v < NV; ++v) lds128(cfa + 16u * v, c[4 * v], c[4 * v + 1], c[4 * v + 2], c[4 * v + 3]);
+                    if constexpr (REM == 1) c[4 * NV] = lds32(cfa + 16u * NV);
+                    else if constexpr (REM == 2) lds64(cfa + 16u * NV, c[4 * NV], c[4 * NV + 1]);
+                    else if constexpr (REM == 3) lds128(cfa + 16u * NV, c[4 * NV], c[4 * NV + 1], c[4 * NV + 2], c[4 * NV + 3]);
+                    RingPlane<T, G, K, D, S, PW, PH, MODE>::run(tb, zb, rowsel, lmask, rmask, sfw, c, res);
+                }
                 if (active) {
 #pragma unroll
                     for (int r = 0; r < PH; ++r) {
@@ -565,9 +613,9 @@ bool make_ring_plan(const RingArgs& a, RingPlan& pl, uint32_t& smem_bytes, int& 
     if (OW % PW != 0 || OH % PH != 0) return false;
     if (p.sf_norm) return false;
     const int TPP = (OH / PH) * (OW / PW);
-    if (TPP < 32 || TPP > kRingMaxThreads - 32) return false;
+    if (TPP < 32 || TPP > kRingMaxThreads<K> - 32) return false;
     const uint32_t plane_bytes = (uint32_t)(H * W * 2);
-    int TG = (kRingMaxThreads - 32) / TPP;
+    int TG = (kRingMaxThreads<K> - 32) / TPP;
     while (TG > 1 && (p.C % TG != 0 || ((unsigned long long)TG * plane_bytes) % 16 != 0)) --TG;
     if (p.C % TG != 0 || ((unsigned long long)TG * plane_bytes) % 16 != 0) return false;
     if (plane_bytes % G::ALIGN != 0) return false;
@@ -578,7 +626,7 @@ bool make_ring_plan(const RingArgs& a, RingPlan& pl, uint32_t& smem_bytes, int& 
     if (!al16(a.in) || !al16(a.cf) || !al16(a.sf) || !al16(a.out)) return false;
 
     const uint32_t pass_bytes = (uint32_t)TG * plane_bytes;
-    const uint32_t target = 36u << 10;
+    const uint32_t target = (K == 3 ? 36u : 18u) << 10;
     int PPS = (int)(target / pass_bytes);
     if (PPS < 1) PPS = 1;
     const long long share = (total_passes + a.sm_count - 1) / a.sm_count;

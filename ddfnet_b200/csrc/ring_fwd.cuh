@@ -33,6 +33,7 @@
 #pragma once
 
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
 #include "stream_fwd.cuh"
@@ -272,8 +273,29 @@ __device__ __forceinline__ void ring_plane_rows(uint32_t tb, uint32_t zb, uint32
             }
         }
     }
+    float sum = 0.f;
 #pragma unroll
-    for (int q = 0; q < P / 2; ++q) f2_unpack(acc2[q], res[2 * q], res[2 * q + 1]);
+    for (int q = 0; q < P / 2; ++q) {
+        f2_unpack(acc2[q], res[2 * q], res[2 * q + 1]);
+        sum += fabsf(res[2 * q]) + fabsf(res[2 * q + 1]);
+    }
+    // x * sf may have left float's range although x * (cf * sf) does not (not with float16's values): again, w first
+    if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+        if (!(sum < __int_as_float(0x7f800000))) {
+#pragma unroll
+            for (int pp = 0; pp < P; ++pp) res[pp] = 0.f;
+#pragma unroll
+            for (int t = 0; t < K * K; ++t) {
+                const int i = t / K, j = t % K;
+                const float c = __uint_as_float(lds32(cfa + (uint32_t)(i * G::CFR + 8 * j)));
+#pragma unroll
+                for (int pp = 0; pp < P; ++pp) {
+                    const int idx = pp % PW + j - G::R - 2 * G::w0(0);
+                    res[pp] = fmaf(Word<T>::get(w[pp / PW + i][idx / 2], idx & 1), c * Word<T>::get(sfw[t][pp / 2], pp & 1), res[pp]);
+                }
+            }
+        }
+    }
 }
 
 // Non-blocking probe (mbarrier.test_wait): the issuing thread must never be parked on a

@@ -26,3 +26,19 @@ def test_matches_oracle(shape, dt):
     (gx,) = torch.autograd.grad(out, xd, go.to(dev))
     check_close(gx, oracle_backward(go, x, cf, sf, 5, 1, 1, "mul")[0], DTYPES[dt], f"grad_x {shape} {dt}")
     assert _lib.load().ddf_b200_take_fault() == 0
+
+
+@pytest.mark.parametrize("shape", [(12, 64, 28, 28), (40, 48, 14, 14)])
+def test_inputs_near_the_types_limit(shape):
+    """x * sf leaves float's range, x * (cf * sf) does not: at most a few such values in a window, of one sign, so the
+    results are held in the 2-norm (bfloat16's rounding of each: 2^-9)."""
+    from ddfnet_b200 import ddf
+    B, C, H, W = shape
+    x, cf, sf, _ = make_inputs(B, C, H, W, 5, 1, torch.bfloat16, 7)
+    x.view(-1)[::29] = -3.3e38
+    cf, sf = (cf * 2.0 ** -8), (sf * 2.0 ** 4)
+    dev = torch.device("cuda:0")
+    out = ddf(x.to(dev), cf.to(dev), sf.to(dev), 5, 1, 1, "mul").cpu().double()
+    want = oracle_forward(x, cf, sf, 5, 1, 1, "mul")
+    assert torch.isfinite(want).all() and torch.isfinite(out).all()
+    assert (out - want).norm() <= 4e-3 * want.norm()

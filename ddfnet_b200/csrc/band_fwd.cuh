@@ -11,23 +11,31 @@
 // that a persistent grid cuts into equal shares: no last wave, and a producer lane keeps a ring of slots
 // full across the changes of band.  At such a change the compute warps reload their filters.
 //
-// A thread owns PH output pixels of one column, D rows apart (so neighbouring windows share rows at
+// A thread owns four output pixels of one column, D rows apart (so neighbouring windows share rows at
 // every dilation).  Lanes of a warp own neighbouring columns: every shared load is conflict-free and
-// every store coalesced at any width and alignment, which vectors along x would not be.  The k*k*PH
-// filter values stay in registers, paired (p, p + PH/2) for the two-wide FMA.  A column of the window is
-// loaded once and serves k taps of PH pixels.
+// every store coalesced at any width and alignment, which vectors along x would not be.  One thread per position
+// fetches its pixels' k*k filter values when a band begins and leaves them in shared memory, laid out for its
+// own later loads; k = 3 takes them into registers from there, k = 5 a column of taps at a time, for two channels.
 //
-// What bounds it: instruction issue and the latency of a pass at 20 warps per SM ((2,256,200x300) f32: 57% of
-// issue slots busy, DRAM at 31% of its peak, shared loads at 29%), and on small problems the filters' way into
-// registers: one pointer per pixel instead of an address per value took (4,128,50x67) f16 from 17.7 to 11.3 us.
-// (2,256,200x300) f32: 80 us, 3.1 TB/s; the generic kernel 655.  Eight pixels per thread instead of four (half
-// the CTAs fit): 97; scalar instead of two-wide FMAs: 93 (k = 5, (8,96,75x101): 50 against 58 before the
-// pointers, 48 after).
+// Arithmetic.  2-byte types, mul: x * sf exact by the mixed-precision FMA from the 2-byte operands, then a float FMA
+// with cf (two-wide FMAs there wait for the pipe: 42.3 against 39.7 us at (2,128,200x280) bf16).  Float, add, and
+// filters normalised here: w = cf * sf (or cf + sf) and x * w, two pixels (p, p + 2) an instruction.
+//
+// What bounds it: instruction issue (9 FMAs of 10 instructions at k = 5, 18 of 51 per output at k = 3 in mul).  Half
+// of what it issued before were products and selects that the compiler formed again in each pass (see pin); stores
+// under a predicate instead of a branch took another eighth.  us, forward / grad-x, before (filters in registers
+// from global memory, 80 to 168 registers) -> now: (2,256,200x300) f32 80.4 / 84.0 -> 76.4 / 78.7 and bf16
+// 84.9 / 89.3 -> 68.0 / 67.8, (4,128,50x67) f16 11.2 / 14.9 -> 10.1 / 11.5, (8,48,150x130) f16 add 25.9 / 30.4 ->
+// 24.8 / 25.6, k = 5 (8,96,75x101) f16 50.1 / 54.9 -> 35.3 / 37.9, f32 47.9 / 52.4 -> 43.1 / 41.7, and
+// (128,64,56x56) bf16 178 / 191 -> 139 / 139; (1,300,60x60) f32 8.3 / 11.4 -> 9.2 / 9.5.  Not kept: four channels a
+// unit (the same or slower), the filters of k = 3 out of shared memory in every pass.
 //
 // Zero padding.  Rows outside the plane are read from a zeroed spot of the slot (their offset is a
 // per-thread constant), columns outside are masked.  A zero times an infinite filter value would be
 // NaN where the definition skips the tap: while the filters hold anything not below kBandFilterMax
-// in magnitude (so that cf * sf is finite too) a CTA takes a plain loop that skips those taps.
+// in magnitude (so that cf * sf is finite too) a CTA takes a plain loop that skips those taps.  A thread takes it too
+// where x * sf may have left float's range although x * (cf * sf) does not (bfloat16 alone): where a result is not
+// finite.
 //
 // Every mbarrier wait is bounded by the plan's wait_cycles.  A thread whose wait ran out records a fault,
 // stays for the barriers of the others, and neither stores nor hands slots back: the producer's own wait
@@ -35,8 +43,10 @@
 #pragma once
 
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
+#include "ring_fwd.cuh"
 #include "stream_fwd.cuh"
 
 namespace ddf {
@@ -63,7 +73,8 @@ struct BandPlan {
     int bwdx, norm;
     float sf_scale;
     unsigned long long in_total;
-    uint32_t off_cf, off_slot0, slot_stride, zero_off;  // zero_off: from a slot's data start
+    uint32_t off_cf, off_sf, off_slot0, slot_stride;
+    uint32_t part_stride, zero_off;  // a slot's channel parts, and from a part's data to its zeros
     int* fault;
     long long wait_cycles;    // limit of every mbarrier wait, in SM clocks
     uint32_t tx_skew;         // self-test: bytes announced beyond what is copied, so that no stage completes
@@ -89,6 +100,8 @@ template <typename T> struct Masked;
 template <> struct Masked<float> {
     static __device__ __forceinline__ uint32_t mask(bool ok) { return ok ? 0xffffffffu : 0u; }
     static __device__ __forceinline__ float load(uint32_t a, uint32_t m) { return __uint_as_float(lds32(a) & m); }
+    template <int OFF> static __device__ __forceinline__ float at(uint32_t a) { return __uint_as_float(lds32i<OFF>(a)); }
+    template <int OFF> static __device__ __forceinline__ float at(uint32_t a, uint32_t m) { return __uint_as_float(lds32i<OFF>(a) & m); }
     static __device__ __forceinline__ float load(uint32_t a) { return ldsf(a); }
 };
 template <> struct Masked<__nv_bfloat16> {
@@ -97,16 +110,22 @@ template <> struct Masked<__nv_bfloat16> {
         return __uint_as_float(__byte_perm(lds16(a), 0u, m));
     }
     static __device__ __forceinline__ float load(uint32_t a) { return __uint_as_float(lds16(a) << 16); }
+    template <int OFF> static __device__ __forceinline__ float at(uint32_t a) { return __uint_as_float(lds16i<OFF>(a) << 16); }
+    template <int OFF> static __device__ __forceinline__ float at(uint32_t a, uint32_t m) {
+        return __uint_as_float(__byte_perm(lds16i<OFF>(a), 0u, m));
+    }
 };
 template <> struct Masked<__half> {
     static __device__ __forceinline__ uint32_t mask(bool ok) { return ok ? 0xffffffffu : 0u; }
     static __device__ __forceinline__ float load(uint32_t a, uint32_t m) { return Word<__half>::get(lds16(a) & m, 0); }
     static __device__ __forceinline__ float load(uint32_t a) { return Word<__half>::get(lds16(a), 0); }
+    template <int OFF> static __device__ __forceinline__ float at(uint32_t a) { return Word<__half>::get(lds16i<OFF>(a), 0); }
+    template <int OFF> static __device__ __forceinline__ float at(uint32_t a, uint32_t m) { return Word<__half>::get(lds16i<OFF>(a) & m, 0); }
 };
 
 // Bytes of a channel's filter in shared memory: (c, c) pairs column by column, each column padded to
-// whole 16 bytes.
-template <int K> constexpr int kBandCf = K * ((K + 1) / 2 * 16);
+// whole 16 bytes; SINGLE: plain floats.
+template <int K, bool SINGLE = false> constexpr int kBandCf = K * (SINGLE ? (K + 3) / 4 * 16 : (K + 1) / 2 * 16);
 
 __device__ __forceinline__ void lds128_pairs(uint32_t a, unsigned long long& x, unsigned long long& y) {
     asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "r"(a));
@@ -127,10 +146,23 @@ __device__ __forceinline__ bool band_sync_or(int n, int v) {
     return r != 0;
 }
 
-// k = 3: two CTAs per SM at 80 registers a thread; k = 5: the 100 filter values a thread holds leave one.
 template <int K> constexpr int kBandThreads = K == 3 ? 352 : 384;
-template <int K> constexpr int kBandCtas = K == 3 ? 2 : 1;
-template <int K> constexpr int kBandRegs = K == 3 ? 80 : 168;
+constexpr int kBandPixels = 4;  // rows a thread owns in its column
+// Registers of a thread: 24 warps of an SM, or 20 where 36 filter values (k = 3, float) or two channels' rows of a
+// 5 x 5 window are held.
+template <int K, bool MIX> constexpr int kBandRegs = K == 3 && MIX ? 80 : 96;
+
+// Stores v where pixel P is one of the first n; a predicate and no branch.
+template <int P>
+__device__ __forceinline__ void store_below(float* at, float v, int n) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.gt.s32 q, %2, %3;\n\t@q st.global.b32 [%0], %1;\n\t}" ::"l"(at), "f"(v), "r"(n), "n"(P) : "memory");
+}
+template <int P, typename T>
+__device__ __forceinline__ void store_below(T* at, float v, int n) {
+    const uint32_t h = Word<T>::put(v, 0.f);
+    asm volatile("{\n\t.reg .pred q;\n\t.reg .b16 l, u;\n\tmov.b32 {l, u}, %1;\n\tsetp.gt.s32 q, %2, %3;\n\t@q st.global.b16 [%0], l;\n\t}"
+                 ::"l"(at), "r"(h), "r"(n), "n"(P) : "memory");
+}
 
 // Output row of a thread's first pixel.  Groups count in blocks of D: group g of a band covers rows
 // (g / D) * PH * D + g % D, + D, + 2D ...
@@ -142,15 +174,83 @@ __device__ __forceinline__ int band_row(int group) { return D == 1 ? group * PH 
 template <int D, int PH>
 __host__ __device__ __forceinline__ int band_rows(int groups) { return groups % D == 0 ? groups * PH : D * (PH - 1) + 1; }
 
-template <typename T, int K, int D, int S, int PH, int MODE>
-__global__ void __launch_bounds__(kBandThreads<K>, kBandCtas<K>)
+// One column of taps of one channel: its window values, then the taps of the four pixels.  s: the column's filters,
+// pixel halves (p0, p1) (p2, p3) or float pairs (p0, p2) (p1, p3).
+template <int J, typename T, int K, int D, int S, bool MUL, bool MIX, int NR, typename SF, typename A>
+__device__ __forceinline__ void band_column(const uint32_t (&row)[NR], uint32_t cmask, uint32_t ca, const SF (*s)[2], A& acc) {
+    constexpr int R = (K - 1) / 2, CFC = kBandCf<K, MIX> / K, DX = D * (J - R) * (int)sizeof(T);
+    if constexpr (MIX) {
+        uint32_t c[(K + 3) / 4 * 4];
+        lds128i<J * CFC>(ca, c[0], c[1], c[2], c[3]);
+        if constexpr (K > 4) c[4] = lds32i<J * CFC + 16>(ca);
+        uint32_t v[NR];
+#pragma unroll
+        for (int r = 0; r < NR; ++r) v[r] = J == R ? lds16i<DX>(row[r]) : lds16i<DX>(row[r]) & cmask;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+#pragma unroll
+            for (int p = 0; p < kBandPixels; ++p)
+                acc[p] = fmaf(Mix<T>::fmaw(0, p & 1, v[S * p + k], s[k][p / 2], 0.f), __uint_as_float(c[k]), acc[p]);
+        }
+    } else {
+        unsigned long long cp[(K + 1) / 2 * 2];
+        lds128i_pairs<J * CFC>(ca, cp[0], cp[1]);
+        lds128i_pairs<J * CFC + 16>(ca, cp[2], cp[3]);
+        if constexpr (K > 4) lds128i_pairs<J * CFC + 32>(ca, cp[4], cp[5]);
+        float v[NR];
+#pragma unroll
+        for (int r = 0; r < NR; ++r) v[r] = J == R ? Masked<T>::template at<DX>(row[r]) : Masked<T>::template at<DX>(row[r], cmask);
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const unsigned long long w2 = MUL ? f2_mul(cp[k], s[k][q]) : f2_add(cp[k], s[k][q]);
+                acc[q] = f2_fma(w2, f2_pack(v[S * q + k], v[S * (q + 2) + k]), acc[q]);
+            }
+        }
+    }
+}
+// All columns of one channel, the filters in registers.
+template <int J, typename T, int K, int D, int S, bool MUL, bool MIX, int NR, typename SF, typename A>
+__device__ __forceinline__ void band_columns(const uint32_t (&row)[NR], const uint32_t (&cmask)[K], uint32_t ca, const SF (*s)[2], A& acc) {
+    if constexpr (J < K) {
+        band_column<J, T, K, D, S, MUL, MIX>(row, cmask[J], ca, s + J * K, acc);
+        band_columns<J + 1, T, K, D, S, MUL, MIX>(row, cmask, ca, s, acc);
+    }
+}
+// All columns of CH channels, the filters of a column at a time out of shared memory.
+template <int J, typename T, int K, int D, int S, bool MUL, bool MIX, int CH, int NR, typename A>
+__device__ __forceinline__ void band_columns_shared(const uint32_t (&row)[CH][NR], const uint32_t (&cmask)[K], uint32_t ca,
+                                                    uint32_t sf_s, uint32_t sf_tap, A (&acc)[CH]) {
+    if constexpr (J < K) {
+        std::conditional_t<MIX, uint32_t, unsigned long long> s[K][2];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            if constexpr (MIX) lds64(sf_s, s[k][0], s[k][1]);
+            else lds128_pairs(sf_s, s[k][0], s[k][1]);
+            sf_s += sf_tap;
+        }
+#pragma unroll
+        for (int ch = 0; ch < CH; ++ch)
+            band_column<J, T, K, D, S, MUL, MIX>(row[ch], cmask[J], ca + (uint32_t)(ch * kBandCf<K, MIX>), s, acc[ch]);
+        band_columns_shared<J + 1, T, K, D, S, MUL, MIX, CH>(row, cmask, ca, sf_s, sf_tap, acc);
+    }
+}
+
+// MIX: 2-byte filters as they are, x * sf exact by the mixed-precision FMA; else float filters (float tensors, and
+// filters normalised here).  CH: channels a thread has of a unit.
+template <typename T, int K, int D, int S, int MODE, bool MIX, int CH>
+__global__ void __maxnreg__((kBandRegs<K, MIX>))
 band_kernel(const __grid_constant__ BandPlan pl) {
     constexpr int KK = K * K, R = (K - 1) / 2, ES = (int)sizeof(T);
-    constexpr int NR = S * (PH - 1) + K;      // window rows of a thread, D input rows apart
-    constexpr int HP = PH / 2;
-    constexpr int CFC = (K + 1) / 2 * 16;     // bytes of one tap column's (c, c) pairs, whole 16s
-    constexpr int CFB = kBandCf<K>;
+    constexpr int PH = kBandPixels, NR = S * (PH - 1) + K;   // window rows of a thread, D input rows apart
+    constexpr bool MUL = MODE == DDF_B200_MUL;
+    constexpr int CFB = kBandCf<K, MIX>;
+    constexpr int CFC = CFB / K;              // bytes of one tap column
+    constexpr uint32_t SFB = PH * (MIX ? 2 : 4);   // bytes of a tap of a thread's pixels
+    constexpr bool REG = K == 3;              // the filters of a thread's pixels stay in registers
     static_assert(D == 1 || S == 1, "dilated windows are built at stride 1");
+    static_assert(!MIX || (ES == 2 && MUL), "mixed-precision products take 2-byte factors; w = cf + sf is float");
 
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const uint32_t sbase = smem_u32(smem_raw);
@@ -162,14 +262,14 @@ band_kernel(const __grid_constant__ BandPlan pl) {
 
     if (tid == 0) {
         for (int s = 0; s < NST; ++s) {
-            mbar_init(BAND_FULL(s), 1);
+            mbar_init(BAND_FULL(s), CH);
             mbar_init(BAND_EMPTY(s), (uint32_t)NW);
         }
         mbar_fence_init();
     }
-    for (int e = tid; e < NST * (int)(kBandZero / 4); e += blockDim.x) {
+    for (int e = tid; e < NST * CH * (int)(kBandZero / 4); e += blockDim.x) {
         const int s = e / (int)(kBandZero / 4);
-        sts32(BAND_DATA(s) + pl.zero_off + 4u * (uint32_t)(e - s * (int)(kBandZero / 4)), 0u);
+        sts32(BAND_DATA(s / CH) + (uint32_t)(s % CH) * pl.part_stride + pl.zero_off + 4u * (uint32_t)(e - s * (int)(kBandZero / 4)), 0u);
     }
     __syncthreads();
     asm volatile("griddepcontrol.launch_dependents;");
@@ -178,6 +278,7 @@ band_kernel(const __grid_constant__ BandPlan pl) {
     const int u_lo = (int)(((unsigned long long)pl.units * blockIdx.x) / gridDim.x);
     const int u_hi = (int)(((unsigned long long)pl.units * (blockIdx.x + 1)) / gridDim.x);
     const unsigned long long plane_bytes = (unsigned long long)pl.H * pl.W * ES;
+    const int GC = G * CH;   // channels of a unit: part ch holds planes [ch * G, ch * G + G) of it
     // a (sample, band)'s rows
     struct Rows { int b, y_lo, iy_lo, iy_hi; };
     auto rows_of = [&](int seg) {
@@ -201,8 +302,7 @@ band_kernel(const __grid_constant__ BandPlan pl) {
     };
 
     if (warp == NW) {
-        // ------------------------------------------------------------- producer
-        if (lane != 0) return;
+        // ------------------------------------------------------------- producer: a lane per part
         int seg = u_lo / pl.passes;
         int pass = u_lo - seg * pl.passes;
         Rows r = rows_of(seg);
@@ -210,22 +310,28 @@ band_kernel(const __grid_constant__ BandPlan pl) {
         int issued = 0;
         for (; issued < n; ++issued) {
             const int slot = issued % NST;
-            if (!band_slot_free(BAND_EMPTY(slot), issued, NST, pl.wait_cycles, pl.tx_skew)) break;
-            const int c = pass * G;
-            const int count = pl.C - c < G ? pl.C - c : G;
-            const unsigned long long g0 = run_start(r, c);
-            const Span sp = span_prepare(BAND_DATA(slot), pl.in, g0,
-                                         g0 + (unsigned long long)(count - 1) * plane_bytes +
-                                             (unsigned long long)(r.iy_hi - r.iy_lo) * pl.W * ES,
-                                         pl.in_total);
-            mbar_arrive_expect_tx(BAND_FULL(slot), sp.bytes + pl.tx_skew);
-            span_issue(sp, BAND_FULL(slot));
+            if (!__all_sync(0xffffffffu, band_slot_free(BAND_EMPTY(slot), issued, NST, pl.wait_cycles, pl.tx_skew))) break;
+            if (lane < CH) {
+                const int c = pass * GC + lane * G;
+                const int count = pl.C - c < G ? pl.C - c : G;
+                Span sp{0u, nullptr, 0u};
+                if (count > 0) {
+                    const unsigned long long g0 = run_start(r, c);
+                    sp = span_prepare(BAND_DATA(slot) + (uint32_t)lane * pl.part_stride, pl.in, g0,
+                                      g0 + (unsigned long long)(count - 1) * plane_bytes +
+                                          (unsigned long long)(r.iy_hi - r.iy_lo) * pl.W * ES,
+                                      pl.in_total);
+                }
+                mbar_arrive_expect_tx(BAND_FULL(slot), sp.bytes + (lane == 0 ? pl.tx_skew : 0u));
+                span_issue(sp, BAND_FULL(slot));
+            }
+            __syncwarp();
             if (++pass == pl.passes) {
                 pass = 0;
                 r = rows_of(++seg);
             }
         }
-        band_leave(BAND_FULL(0), issued, n, NST, pl.wait_cycles, pl.tx_skew, pl.fault);
+        if (lane == 0) band_leave(BAND_FULL(0), issued, n, NST, pl.wait_cycles, pl.tx_skew, pl.fault);
         return;
     }
 
@@ -241,28 +347,43 @@ band_kernel(const __grid_constant__ BandPlan pl) {
 #pragma unroll
     for (int j = 0; j < K; ++j) {
         const int ix = x * S + D * (j - R);
-        cmask[j] = Masked<T>::mask(ix >= 0 && ix < pl.W);
+        const bool ok = ix >= 0 && ix < pl.W;
+        cmask[j] = MIX ? (ok ? 0xffffu : 0u) : Masked<T>::mask(ok);
+        pin(cmask[j]);
     }
     const long long out_plane = (long long)pl.OH * pl.OW;
-    const int row_step = D * pl.OW;
-    const uint32_t g_step = (uint32_t)((unsigned long long)G * plane_bytes);
+    // steps from a channel part to the next, in bytes: kept, since products of 64 bits in every pass were a sixth of
+    // the instructions
+    unsigned long long out_step = (unsigned long long)G * out_plane * ES;
+    uint32_t in_step = (uint32_t)((unsigned long long)G * plane_bytes);   // (its remainder of 16 is all that matters)
+    uint32_t row_step = (uint32_t)(D * pl.OW * ES);
+    pin(out_step);
+    pin(in_step);
+    pin(row_step);
+    const uint32_t sf_s = sbase + pl.off_sf + (uint32_t)pos * SFB;   // taps column by column, a tap of all positions after the other
+    const uint32_t sf_tap = (uint32_t)npos * SFB;
 
     int slot = -1;
-    uint32_t ph = 1;
+    uint32_t ph = 1, data = BAND_DATA(0) - pl.slot_stride;
+    uint32_t cf_step = (uint32_t)(G * CH) * CFB;
+    pin(cf_step);
     int seg = u_lo / pl.passes;
     int pass = u_lo - seg * pl.passes;
     bool fresh = true;  // the next unit starts another (sample, band)
     Rows rw = rows_of(seg);
     int big_sf = 0;     // a spatial-filter value too large for products with padding zeros (or NaN)
     uint32_t rowoff[NR];
-    unsigned long long sf2[KK][HP];  // spatial filters of this thread's pixels, [column-major tap][pair]
+    // the filters of this thread's pixels, [column-major tap][pair]: halves (p0, p1) (p2, p3), or floats (p0, p2) (p1, p3)
+    std::conditional_t<MIX, uint32_t, unsigned long long> sfr[REG ? KK : 1][2];
     int y0 = 0, rows_left = 0;
     for (int u = u_lo; u < u_hi;) {
         int npass = pl.passes - pass;
         if (npass > u_hi - u) npass = u_hi - u;
         if (npass > pl.stage_passes) npass = pl.stage_passes;
-        const int c_lo = pass * G;
-        const int c_hi = c_lo + npass * G < pl.C ? c_lo + npass * G : pl.C;
+        const int c_lo = pass * GC;
+        const int c_hi = c_lo + npass * GC < pl.C ? c_lo + npass * GC : pl.C;
+        if (u != u_lo) band_sync(NW * 32);  // every warp is done with the filters staged before
+        const bool started = fresh;
         if (fresh) {
             fresh = false;
             y0 = rw.y_lo + band_row<D, PH>(grp);
@@ -274,166 +395,279 @@ band_kernel(const __grid_constant__ BandPlan pl) {
                 rowoff[r] = (active && iy >= 0 && iy < pl.H)
                                 ? (uint32_t)pip * (uint32_t)plane_bytes + (uint32_t)(((iy - rw.iy_lo) * pl.W + x * S) * ES)
                                 : pl.zero_off + 16u;
+                pin(rowoff[r]);
             }
-            // Loads from clamped addresses and values dropped after: a load behind a branch would wait for
-            // the one before.
-            const T* sfb = reinterpret_cast<const T*>(pl.sf) + (long long)rw.b * KK * out_plane;
-            float sum_abs = 0.f;
+            pin(rows_left);
+            // Spatial filters of the position's pixels, by one thread each.  Loads from clamped addresses and
+            // values dropped after: a load behind a branch would wait for the one before.
+            big_sf = 0;
+            if (owner && pip == 0) {
+                const T* sfb = reinterpret_cast<const T*>(pl.sf) + (long long)rw.b * KK * out_plane;
+                float sum_abs = 0.f;
+                if (!pl.bwdx) {
+                    const T* at[PH];
+                    bool ok[PH];
 #pragma unroll
-            for (int q = 0; q < HP; ++q) {
-                float v[2][KK];
+                    for (int p = 0; p < PH; ++p) {
+                        ok[p] = p < rows_left;
+                        at[p] = ok[p] ? sfb + (y0 + D * p) * pl.OW + x : sfb;
+                    }
+                    if constexpr (MIX) {
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int p = q + h * HP;
-                    if (!pl.bwdx) {
-                        const bool ok = p < rows_left;
-                        const T* at = ok ? sfb + (y0 + D * p) * pl.OW + x : sfb;
+                        for (int t = 0; t < KK; ++t) {
+                            uint32_t v[PH];
 #pragma unroll
-                        for (int t = 0; t < KK; ++t) v[h][t] = Elem<T>::load(at + t * out_plane);
-                        if (!ok) {
-#pragma unroll
-                            for (int t = 0; t < KK; ++t) v[h][t] = 0.f;
+                            for (int p = 0; p < PH; ++p) {
+                                v[p] = __ldg(reinterpret_cast<const uint16_t*>(at[p]));
+                                at[p] += out_plane;
+                                if (!ok[p]) v[p] = 0u;
+                            }
+                            const uint32_t lo = v[0] | (v[1] << 16), hi = v[2] | (v[3] << 16);
+                            sum_abs += fabsf(Word<T>::get(lo, 0)) + fabsf(Word<T>::get(lo, 1)) + fabsf(Word<T>::get(hi, 0)) +
+                                       fabsf(Word<T>::get(hi, 1));
+                            sts64(sf_s + (uint32_t)((t % K) * K + t / K) * sf_tap, lo, hi);
                         }
                     } else {
 #pragma unroll
-                        for (int i = 0; i < K; ++i) {
-                            const int yy = y0 + D * (p + i - R);
-                            const bool row = p < rows_left && yy >= 0 && yy < pl.OH;
-                            const T* at = row ? sfb + (KK - 1 - i * K) * out_plane + yy * pl.OW + x : sfb;
+                        for (int h = 0; h < PH; h += 2) {   // two pixels' taps at a time
+                            float v[2][KK];
 #pragma unroll
-                            for (int j = 0; j < K; ++j) {
-                                const bool ok = row && x + D * (j - R) >= 0 && x + D * (j - R) < pl.OW;
-                                const float w = Elem<T>::load(ok ? at + (D * (j - R) - j * out_plane) : sfb);
-                                v[h][i * K + j] = ok ? w : 0.f;
+                            for (int e = 0; e < 2; ++e) {
+#pragma unroll
+                                for (int t = 0; t < KK; ++t) v[e][t] = Elem<T>::load(at[h + e] + t * (long long)out_plane);
+                            }
+#pragma unroll
+                            for (int e = 0; e < 2; ++e) {
+                                if (pl.norm) {
+                                    float sum = 0.f;
+#pragma unroll
+                                    for (int t = 0; t < KK; ++t) sum += v[e][t];
+                                    const float mean = sum / (float)KK;
+                                    float var = 0.f;
+#pragma unroll
+                                    for (int t = 0; t < KK; ++t) {
+                                        v[e][t] -= mean;
+                                        var = fmaf(v[e][t], v[e][t], var);
+                                    }
+                                    const float inv = pl.sf_scale / (sqrtf(var / (float)(KK - 1)) + 1e-10f);
+#pragma unroll
+                                    for (int t = 0; t < KK; ++t) v[e][t] *= inv;
+                                }
+#pragma unroll
+                                for (int t = 0; t < KK; ++t) {
+                                    if (!ok[h + e]) v[e][t] = 0.f;
+                                    sum_abs += fabsf(v[e][t]);
+                                }
+                            }
+#pragma unroll
+                            for (int t = 0; t < KK; ++t) {
+                                const uint32_t to = sf_s + (uint32_t)((t % K) * K + t / K) * sf_tap + 2u * h;  // p0 p2 p1 p3
+                                sts32(to, __float_as_uint(v[0][t]));
+                                sts32(to + 8u, __float_as_uint(v[1][t]));
+                            }
+                        }
+                    }
+                } else {
+                    // grad-x pairs a window tap with the mirrored tap's filter at the neighbour it came from
+#pragma unroll
+                    for (int i = 0; i < K; ++i) {
+                        const T* at[PH];
+                        bool row[PH];
+#pragma unroll
+                        for (int p = 0; p < PH; ++p) {
+                            const int yy = y0 + D * (p + i - R);
+                            row[p] = p < rows_left && yy >= 0 && yy < pl.OH;
+                            at[p] = sfb + (KK - 1 - i * K) * (long long)out_plane + (row[p] ? yy * pl.OW + x : x);
+                        }
+#pragma unroll
+                        for (int j = 0; j < K; ++j) {
+                            const bool col = x + D * (j - R) >= 0 && x + D * (j - R) < pl.OW;
+                            const int step = col ? D * (j - R) : 0;
+                            uint32_t v[PH];
+#pragma unroll
+                            for (int p = 0; p < PH; ++p) {
+                                const T* from = at[p] + (step - j * (long long)out_plane);
+                                if constexpr (MIX) v[p] = __ldg(reinterpret_cast<const uint16_t*>(from));
+                                else v[p] = __float_as_uint(Elem<T>::load(from));
+                                if (!(row[p] && col)) v[p] = 0u;
+                            }
+                            const uint32_t to = sf_s + (uint32_t)(j * K + i) * sf_tap;
+                            if constexpr (MIX) {
+                                const uint32_t lo = v[0] | (v[1] << 16), hi = v[2] | (v[3] << 16);
+                                sum_abs += fabsf(Word<T>::get(lo, 0)) + fabsf(Word<T>::get(lo, 1)) + fabsf(Word<T>::get(hi, 0)) +
+                                           fabsf(Word<T>::get(hi, 1));
+                                sts64(to, lo, hi);
+                            } else {
+                                sts128(to, v[0], v[2], v[1], v[3]);
+#pragma unroll
+                                for (int p = 0; p < PH; ++p) sum_abs += fabsf(__uint_as_float(v[p]));
                             }
                         }
                     }
                 }
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    if (pl.norm) {
-                        float sum = 0.f;
-#pragma unroll
-                        for (int t = 0; t < KK; ++t) sum += v[h][t];
-                        const float mean = sum / (float)KK;
-                        float var = 0.f;
-#pragma unroll
-                        for (int t = 0; t < KK; ++t) {
-                            v[h][t] -= mean;
-                            var = fmaf(v[h][t], v[h][t], var);
-                        }
-                        const float inv = pl.sf_scale / (sqrtf(var / (float)(KK - 1)) + 1e-10f);
-#pragma unroll
-                        for (int t = 0; t < KK; ++t) v[h][t] *= inv;
-                    }
-#pragma unroll
-                    for (int t = 0; t < KK; ++t) sum_abs += fabsf(v[h][t]);
-                }
-#pragma unroll
-                for (int t = 0; t < KK; ++t) sf2[(t % K) * K + t / K][q] = f2_pack(v[0][t], v[1][t]);
+                big_sf = !(sum_abs < kBandFilterMax);
             }
-            big_sf = !(sum_abs < kBandFilterMax);
         }
-        // Channel filters of the next units as (c, c) pairs, one column of taps after the other; grad-x
-        // pairs window tap (i, j) with the mirrored filter tap.
+        // Channel filters of the next units, one column of taps after the other; grad-x pairs window tap (i, j)
+        // with the mirrored filter tap.
         int big = big_sf;
-        if (u != u_lo) band_sync(NW * 32);  // every warp is done with the filters staged before
         {
             const T* cfp = reinterpret_cast<const T*>(pl.cf) + ((long long)rw.b * pl.C + c_lo) * KK;
             const int n = (c_hi - c_lo) * KK;
             for (int e = tid; e < n; e += NW * 32) {
                 const int c = e / KK, t = e - c * KK;
+                const int unit = c / GC, part = (c - unit * GC) / G, plane = c - unit * GC - part * G;
                 const int w = pl.bwdx ? KK - 1 - t : t;
                 const float v = Elem<T>::load(cfp + e);
                 big |= !(fabsf(v) < kBandFilterMax);
                 const uint32_t bits = __float_as_uint(v);
-                sts64(sbase + pl.off_cf + (uint32_t)c * CFB + (uint32_t)((w % K) * CFC + 8 * (w / K)), bits, bits);
+                const uint32_t to = sbase + pl.off_cf + (uint32_t)((unit * G + plane) * CH + part) * CFB + (uint32_t)((w % K) * CFC);
+                if constexpr (MIX) sts32(to + (uint32_t)(4 * (w / K)), bits);
+                else sts64(to + (uint32_t)(8 * (w / K)), bits, bits);
             }
         }
         const bool plain = band_sync_or(NW * 32, big);
 
-        T* outp = reinterpret_cast<T*>(pl.out) + ((long long)rw.b * pl.C + c_lo + pip) * out_plane +
-                  (long long)y0 * pl.OW + x;
+        if constexpr (REG) {
+            if (started) {
+#pragma unroll
+                for (int t = 0; t < KK; ++t) {
+                    const uint32_t from = sf_s + (uint32_t)t * sf_tap;
+                    if constexpr (MIX) lds64v(from, sfr[t][0], sfr[t][1]);
+                    else {
+                        uint32_t w[4];
+                        lds128v(from, w[0], w[1], w[2], w[3]);
+                        sfr[t][0] = f2_pack(__uint_as_float(w[0]), __uint_as_float(w[1]));
+                        sfr[t][1] = f2_pack(__uint_as_float(w[2]), __uint_as_float(w[3]));
+                    }
+                }
+            }
+        }
+
+        char* outp = reinterpret_cast<char*>(pl.out) +
+                     (((long long)rw.b * pl.C + c_lo + pip) * out_plane + (long long)y0 * pl.OW + x) * ES;
         uint32_t g_lo = (uint32_t)run_start(rw, c_lo);
-        uint32_t cf_s = sbase + pl.off_cf + (uint32_t)pip * CFB;
-        int left = c_hi - c_lo - pip;  // > 0 while this thread's plane of the unit exists
+        uint32_t cf_s = sbase + pl.off_cf + (uint32_t)(pip * CH) * CFB;
+        int left = c_hi - c_lo - pip;  // channel ch of a unit exists for this thread: left > ch * G
         for (int i = 0; i < npass; ++i) {
-            if (++slot == NST) slot = 0;
+            data += pl.slot_stride;
+            if (++slot == NST) {
+                slot = 0;
+                data = BAND_DATA(0);
+            }
             if (slot == 0) ph ^= 1u;
             if (ph < kBandDead && !mbar_wait_for(BAND_FULL(slot), ph, pl.wait_cycles)) {
                 atomicCAS(pl.fault, 0, (int)kFaultConsumerFull);
                 ph |= kBandDead;
             }
-            const uint32_t base = BAND_DATA(slot) + (g_lo & 15u);
-            unsigned long long acc2[HP];
+            const uint32_t alive = ph < kBandDead;
+            auto base_of = [&](int ch) {
+                return data + (uint32_t)ch * pl.part_stride + ((g_lo + (uint32_t)ch * in_step) & 15u);
+            };
+            // the results of one channel, one after the other
+            auto finish = [&](int ch, const float (&res)[PH]) {
+                const int n = alive && left > ch * G ? rows_left : 0;
+                store_below<0>(reinterpret_cast<T*>(outp), res[0], n);
+                store_below<1>(reinterpret_cast<T*>(outp + row_step), res[1], n);
+                store_below<2>(reinterpret_cast<T*>(outp + 2ull * row_step), res[2], n);
+                store_below<3>(reinterpret_cast<T*>(outp + 3ull * row_step), res[3], n);
+                outp += out_step;
+            };
+            using Acc = std::conditional_t<MIX, float[PH], unsigned long long[2]>;
+            auto clear = [](Acc& acc) {
 #pragma unroll
-            for (int q = 0; q < HP; ++q) acc2[q] = 0ull;
-            if (!plain) {
-                uint32_t row[NR];
+                for (auto& a : acc) a = 0;
+            };
+            auto unpack = [](const Acc& acc, float (&res)[PH]) {
+                if constexpr (MIX) {
 #pragma unroll
-                for (int r = 0; r < NR; ++r) row[r] = base + rowoff[r];
-#pragma unroll
-                for (int j = 0; j < K; ++j) {
-                    unsigned long long cp[(K + 1) / 2 * 2];
-#pragma unroll
-                    for (int t = 0; t < (K + 1) / 2; ++t)
-                        lds128_pairs(cf_s + (uint32_t)(j * CFC + 16 * t), cp[2 * t], cp[2 * t + 1]);
-                    float v[NR];
-#pragma unroll
-                    for (int r = 0; r < NR; ++r)
-                        v[r] = j == R ? Masked<T>::load(row[r])
-                                      : Masked<T>::load(row[r] + (uint32_t)((D * (j - R)) * ES), cmask[j]);
-#pragma unroll
-                    for (int k = 0; k < K; ++k) {
-#pragma unroll
-                        for (int q = 0; q < HP; ++q) {
-                            const unsigned long long w2 = MODE == DDF_B200_MUL ? f2_mul(cp[k], sf2[j * K + k][q])
-                                                                               : f2_add(cp[k], sf2[j * K + k][q]);
-                            acc2[q] = f2_fma(w2, f2_pack(v[S * q + k], v[S * (q + HP) + k]), acc2[q]);
-                        }
-                    }
+                    for (int p = 0; p < PH; ++p) res[p] = acc[p];
+                } else {
+                    f2_unpack(acc[0], res[0], res[2]);
+                    f2_unpack(acc[1], res[1], res[3]);
                 }
-            } else {
-                // taps outside the plane are skipped, not multiplied by zero
-                auto tap = [&](int iy, int ix, float cv, float sv, float a) {
-                    if (iy < 0 || iy >= pl.H || ix < 0 || ix >= pl.W) return a;
-                    const uint32_t at = base + (uint32_t)pip * (uint32_t)plane_bytes +
-                                        (uint32_t)(((iy - rw.iy_lo) * pl.W + ix) * ES);
-                    return fmaf(combine_w<MODE, float>(cv, sv), Masked<T>::load(at), a);
-                };
-#pragma unroll
-                for (int q = 0; q < HP; ++q) {
-                    float a0 = 0.f, a1 = 0.f;
-#pragma unroll
-                    for (int t = 0; t < KK; ++t) {  // t = column-major tap
-                        float s0, s1;
-                        f2_unpack(sf2[t][q], s0, s1);
-                        const float cv = ldsf(cf_s + (uint32_t)((t / K) * CFC + 8 * (t % K)));
-                        const int ix = x * S + D * (t / K - R), iy = y0 * S + D * (t % K - R);
-                        if (q < rows_left) a0 = tap(iy + q * S * D, ix, cv, s0, a0);
-                        if (q + HP < rows_left) a1 = tap(iy + (q + HP) * S * D, ix, cv, s1, a1);
-                    }
-                    acc2[q] = f2_pack(a0, a1);
-                }
-            }
-            // the slot is handed back before the stores: nothing below reads it
-            __syncwarp();
-            if (lane == 0 && ph < kBandDead) mbar_arrive(BAND_EMPTY(slot));
-            if (left > 0 && ph < kBandDead) {
-                T* o = outp;
-                float res[PH];
-#pragma unroll
-                for (int q = 0; q < HP; ++q) f2_unpack(acc2[q], res[q], res[q + HP]);
+            };
+            // the slot is handed back before the last stores: nothing below reads it
+            auto hand_back = [&] {
+                __syncwarp();
+                if (lane == 0 && alive) mbar_arrive(BAND_EMPTY(slot));
+            };
+            // one channel, tap by tap: w = cf * sf before it meets x, taps outside the plane skipped, not multiplied by zero
+            auto exact = [&](int ch, float (&res)[PH]) {
+                const uint32_t base = base_of(ch);
 #pragma unroll
                 for (int p = 0; p < PH; ++p) {
-                    if (p < rows_left) Elem<T>::store(o, res[p]);
-                    o += row_step;
+                    float a = 0.f;
+#pragma unroll 1
+                    for (int t = 0; t < KK; ++t) {  // t = column-major tap
+                        const int col = t / K, k = t - col * K;
+                        const int ix = x * S + D * (col - R), iy = (y0 + p * D) * S + D * (k - R);
+                        if (p >= rows_left || iy < 0 || iy >= pl.H || ix < 0 || ix >= pl.W) continue;
+                        const uint32_t sa = sf_s + (uint32_t)t * sf_tap;
+                        float sv;
+                        if constexpr (MIX) sv = Word<T>::get(lds16(sa + 2u * p), 0);
+                        else sv = ldsf(sa + 4u * (uint32_t)((p & 1) * 2 + (p >> 1)));
+                        const float cv = ldsf(cf_s + (uint32_t)(ch * CFB + col * CFC + (MIX ? 4 : 8) * k));
+                        const uint32_t at = base + (uint32_t)pip * (uint32_t)plane_bytes +
+                                            (uint32_t)(((iy - rw.iy_lo) * pl.W + ix) * ES);
+                        a = fmaf(combine_w<MODE, float>(cv, sv), Masked<T>::load(at), a);
+                    }
+                    res[p] = a;
                 }
+            };
+            // (2-byte values of float16 have products of three inside float's range)
+            auto overflowed = [](const float (&res)[PH]) {
+                return MIX && std::is_same<T, __nv_bfloat16>::value &&
+                       !(fabsf(res[0]) + fabsf(res[1]) + fabsf(res[2]) + fabsf(res[3]) < __int_as_float(0x7f800000));
+            };
+            if (plain) {
+#pragma unroll 1
+                for (int ch = 0; ch < CH; ++ch) {
+                    float res[PH];
+                    exact(ch, res);
+                    if (ch == CH - 1) hand_back();
+                    finish(ch, res);
+                }
+            } else if constexpr (REG) {
+#pragma unroll
+                for (int ch = 0; ch < CH; ++ch) {
+                    const uint32_t base = base_of(ch);
+                    uint32_t row[NR];
+#pragma unroll
+                    for (int r = 0; r < NR; ++r) row[r] = base + rowoff[r];
+                    Acc acc;
+                    clear(acc);
+                    band_columns<0, T, K, D, S, MUL, MIX>(row, cmask, cf_s + (uint32_t)(ch * CFB), sfr, acc);
+                    float res[PH];
+                    unpack(acc, res);
+                    if (overflowed(res)) exact(ch, res);
+                    if (ch == CH - 1) hand_back();
+                    finish(ch, res);
+                }
+            } else {
+                uint32_t row[CH][NR];
+                Acc acc[CH];
+#pragma unroll
+                for (int ch = 0; ch < CH; ++ch) {
+                    const uint32_t base = base_of(ch);
+#pragma unroll
+                    for (int r = 0; r < NR; ++r) row[ch][r] = base + rowoff[r];
+                    clear(acc[ch]);
+                }
+                band_columns_shared<0, T, K, D, S, MUL, MIX, CH>(row, cmask, cf_s, sf_s, sf_tap, acc);
+                float res[CH][PH];
+#pragma unroll
+                for (int ch = 0; ch < CH; ++ch) {
+                    unpack(acc[ch], res[ch]);
+                    if (overflowed(res[ch])) exact(ch, res[ch]);
+                }
+                hand_back();
+#pragma unroll
+                for (int ch = 0; ch < CH; ++ch) finish(ch, res[ch]);
             }
-            outp += G * out_plane;
-            cf_s += (uint32_t)G * CFB;
-            g_lo += g_step;
-            left -= G;
+            cf_s += cf_step;
+            g_lo += CH * in_step;
+            left -= GC;
         }
         u += npass;
         pass += npass;
@@ -496,36 +730,23 @@ inline bool band_split(int B, int C, int OH, int OW, int D, int PH, int max_thre
     return (long long)B * s.bands * C <= (1ll << 40);
 }
 
-// Slot layout for runs of up to `run` bytes: [guard | data + 16 | zeros], ring depth within `budget`.
-inline int band_slots(uint32_t run, uint32_t off_slot0, uint32_t budget, uint32_t& zero_off, uint32_t& stride) {
-    zero_off = round_up(run + 16u + 32u, 16);
-    stride = round_up(kBandGuard + zero_off + kBandZero, 128);
-    for (int n = kBandSlots; n >= 2; --n)
-        if (off_slot0 + (uint32_t)n * stride <= budget) return n;
-    return 0;
-}
-
-template <typename T, int K, int D, int S, int PH, int MODE>
-int band_launch(const BandArgs& a, cudaStream_t stream) {
+// The launch of one instantiation; kNotHandled where it does not fit.
+template <typename T, int K, int D, int S, int MODE, bool MIX, int CH>
+int band_launch_split(const BandArgs& a, const BandSplit& sp, cudaStream_t stream) {
     const Problem& p = a.p;
-    constexpr int ES = (int)sizeof(T), R = (K - 1) / 2;
-    if ((reinterpret_cast<uintptr_t>(a.in) & 15u) != 0) return kNotHandled;
-    if (a.bwdx && p.sf_norm) return kNotHandled;
+    constexpr int ES = (int)sizeof(T), R = (K - 1) / 2, PH = kBandPixels;
     BandPlan pl;
     pl.in = a.in; pl.cf = a.cf; pl.sf = a.sf; pl.out = a.out;
     pl.C = p.C;
     pl.OH = p.OH; pl.OW = p.OW;
     pl.H = a.bwdx ? p.OH : p.H;
     pl.W = a.bwdx ? p.OW : p.W;
-    BandSplit sp;
-    if (!band_split(p.B, p.C, p.OH, p.OW, D, PH, kBandThreads<K>, false, sp)) return kNotHandled;
     pl.bands = sp.bands; pl.groups = sp.groups; pl.planes = sp.planes; pl.n_warps = sp.warps;
-    pl.passes = (p.C + sp.planes - 1) / sp.planes;
+    const int per_unit = sp.planes * CH;
+    pl.passes = (p.C + per_unit - 1) / per_unit;
     const long long units = (long long)p.B * sp.bands * pl.passes;
     if (units > (1ll << 30)) return kNotHandled;
     pl.units = (int)units;
-    pl.stage_passes = kBandStage / sp.planes > 1 ? kBandStage / sp.planes : 1;
-    if (pl.stage_passes > pl.passes) pl.stage_passes = pl.passes;
     pl.bwdx = a.bwdx; pl.norm = p.sf_norm; pl.sf_scale = (float)p.sf_scale;
     pl.in_total = (unsigned long long)p.B * p.C * pl.H * pl.W * ES;
     pl.fault = a.fault; pl.wait_cycles = a.wait_cycles; pl.tx_skew = a.tx_skew;
@@ -534,21 +755,32 @@ int band_launch(const BandArgs& a, cudaStream_t stream) {
     const long long run = (sp.planes - 1) * plane_bytes + (rows < pl.H ? rows : pl.H) * (long long)pl.W * ES;
     if (run > (100 << 10)) return kNotHandled;
     pl.off_cf = round_up(16u * kBandSlots, 128);
-    pl.off_slot0 = round_up(pl.off_cf + (uint32_t)(pl.stage_passes * sp.planes) * kBandCf<K>, 128);
-    // as many CTAs per SM as the registers allow, each with at least three slots
+    pl.zero_off = round_up((uint32_t)run + 16u + 32u, 16);
+    pl.part_stride = round_up(kBandGuard + pl.zero_off + kBandZero, 128);
+    pl.slot_stride = CH * pl.part_stride;
+    // as many CTAs per SM as the registers allow, each with at least two slots; fewer channels' filters staged
+    // together where only that makes them fit
     const int threads = (sp.warps + 1) * 32;
-    int ctas = 65536 / (kBandRegs<K> * threads);
-    if (ctas > 4) ctas = 4;
-    for (;; --ctas) {
-        if (ctas < 1) return kNotHandled;
-        const uint32_t budget = ctas == 1 ? kSmemBudget : (227u << 10) / (uint32_t)ctas - 1024u;
-        pl.n_slots = band_slots((uint32_t)run, pl.off_slot0, budget, pl.zero_off, pl.slot_stride);
-        if (pl.n_slots >= 3 || (ctas == 1 && pl.n_slots == 2)) break;
+    int ctas = 0;
+    for (int stage = kBandStage; stage >= 16 && ctas < 1; stage /= 4) {
+        pl.stage_passes = stage / per_unit > 1 ? stage / per_unit : 1;
+        if (pl.stage_passes > pl.passes) pl.stage_passes = pl.passes;
+        pl.off_sf = round_up(pl.off_cf + (uint32_t)(pl.stage_passes * per_unit) * kBandCf<K, MIX>, 128);
+        pl.off_slot0 = round_up(pl.off_sf + (uint32_t)(K * K * sp.groups * p.OW * PH * (MIX ? 2 : 4)), 128);
+        const int fit = 4 * (65536 / 4 / 32 / kBandRegs<K, MIX>) / (sp.warps + 1);  // whole warps in each quarter of an SM
+        for (ctas = fit < 1 ? 1 : fit < 4 ? fit : 4; ctas >= 1; --ctas) {
+            const uint32_t budget = ctas == 1 ? kSmemBudget : (227u << 10) / (uint32_t)ctas - 1024u;
+            if (pl.off_slot0 >= budget) continue;
+            pl.n_slots = (int)((budget - pl.off_slot0) / pl.slot_stride);
+            if (pl.n_slots > kBandSlots) pl.n_slots = kBandSlots;
+            if (pl.n_slots >= 2) break;
+        }
     }
+    if (ctas < 1) return kNotHandled;
     const long long most = (long long)ctas * a.sm_count;
     const long long grid = units < most ? units : most;
     const uint32_t smem = pl.off_slot0 + (uint32_t)pl.n_slots * pl.slot_stride;
-    auto kern = band_kernel<T, K, D, S, PH, MODE>;
+    auto kern = band_kernel<T, K, D, S, MODE, MIX, CH>;
     static std::atomic<unsigned long long> opted_in{0};
     const unsigned long long bit = 1ull << (a.device & 63);
     if (!(opted_in.load(std::memory_order_acquire) & bit)) {
@@ -557,6 +789,24 @@ int band_launch(const BandArgs& a, cudaStream_t stream) {
         opted_in.fetch_or(bit, std::memory_order_release);
     }
     return (int)launch_overlapped(kern, dim3((unsigned)grid), dim3((unsigned)threads), smem, stream, true, pl);
+}
+
+template <typename T, int K, int D, int S, int MODE, bool MIX>
+int band_launch(const BandArgs& a, cudaStream_t stream) {
+    const Problem& p = a.p;
+    if ((reinterpret_cast<uintptr_t>(a.in) & 15u) != 0) return kNotHandled;
+    if (a.bwdx && p.sf_norm) return kNotHandled;
+    BandSplit sp;
+    if (!band_split(p.B, p.C, p.OH, p.OW, D, kBandPixels, kBandThreads<K>, false, sp)) return kNotHandled;
+    // Two channels a thread and unit share the waits and, at k = 5, the filters' way out of shared memory; one where
+    // the units of two would not go evenly into the CTAs ((1,300,60x60) f32: two or three each, 9.3 us against 8.3).
+    auto units = [&](int planes, int ch) { return (long long)p.B * sp.bands * ((p.C + planes * ch - 1) / (planes * ch)); };
+    // fewer planes together while there are SMs without a unit
+    while (K == 3 && sp.planes > 1 && units(sp.planes, 1) < a.sm_count) sp.planes = (sp.planes + 1) / 2;
+    sp.warps = (sp.planes * sp.groups * p.OW + 31) / 32;
+    if constexpr (K == 3)
+        if (units(sp.planes, 2) < 6ll * a.sm_count) return band_launch_split<T, K, D, S, MODE, MIX, 1>(a, sp, stream);
+    return band_launch_split<T, K, D, S, MODE, MIX, 2>(a, sp, stream);
 }
 
 // Defined once per element type in band_inst_<type>.cu.

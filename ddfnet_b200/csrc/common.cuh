@@ -137,8 +137,8 @@ __device__ __forceinline__ uint32_t lds32v(uint32_t a) {
     return v;
 }
 __device__ __forceinline__ uint32_t lds16v(uint32_t a) {
-    uint16_t v;
-    asm volatile("ld.volatile.shared.u16 %0, [%1];" : "=h"(v) : "r"(a) : "memory");
+    uint32_t v;
+    asm volatile("ld.volatile.shared.u16 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
     return v;
 }
 __device__ __forceinline__ void lds64v(uint32_t a, uint32_t& x, uint32_t& y) {
@@ -150,9 +150,10 @@ __device__ __forceinline__ void lds128v(uint32_t a, uint32_t& x, uint32_t& y, ui
                  : "r"(a)
                  : "memory");
 }
+// (straight into a 32-bit register, zero-extended: a 16-bit result would cost an instruction to widen)
 __device__ __forceinline__ uint32_t lds16(uint32_t a) {
-    uint16_t v;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
+    uint32_t v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(a));
     return v;
 }
 __device__ __forceinline__ void lds64(uint32_t a, uint32_t& x, uint32_t& y) {
@@ -163,6 +164,23 @@ __device__ __forceinline__ void lds128(uint32_t a, uint32_t& x, uint32_t& y, uin
     asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(x), "=r"(y), "=r"(z), "=r"(w)
                  : "r"(a));
+}
+// With a constant offset in the instruction (added to the address, it costs an instruction of its own).
+template <int OFF> __device__ __forceinline__ uint32_t lds16i(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u16 %0, [%1+%2];" : "=r"(v) : "r"(a), "n"(OFF));
+    return v;
+}
+template <int OFF> __device__ __forceinline__ uint32_t lds32i(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.b32 %0, [%1+%2];" : "=r"(v) : "r"(a), "n"(OFF));
+    return v;
+}
+template <int OFF> __device__ __forceinline__ void lds128i_pairs(uint32_t a, unsigned long long& x, unsigned long long& y) {
+    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2+%3];" : "=l"(x), "=l"(y) : "r"(a), "n"(OFF));
+}
+template <int OFF> __device__ __forceinline__ void lds128i(uint32_t a, uint32_t& x, uint32_t& y, uint32_t& z, uint32_t& w) {
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4+%5];" : "=r"(x), "=r"(y), "=r"(z), "=r"(w) : "r"(a), "n"(OFF));
 }
 __device__ __forceinline__ float ldsf(uint32_t a) { return __uint_as_float(lds32(a)); }
 __device__ __forceinline__ unsigned long long lds64_pair(uint32_t a) {
@@ -205,6 +223,13 @@ __device__ __forceinline__ Span span_prepare(uint32_t dst, const void* base, uns
 __device__ __forceinline__ void span_issue(const Span& s, uint32_t bar) {
     if (s.bytes) bulk_g2s(s.dst, s.src, s.bytes, bar);
 }
+
+// Fixes a value in its register: without it the compiler may compute a thread's constants (offsets, masks, selected
+// values) again in every turn of a loop, which costs the issue slots that the registers would have saved.
+__device__ __forceinline__ void pin(uint32_t& v) { asm volatile("" : "+r"(v)); }
+__device__ __forceinline__ void pin(int& v) { asm volatile("" : "+r"(v)); }
+__device__ __forceinline__ void pin(float& v) { asm volatile("" : "+f"(v)); }
+__device__ __forceinline__ void pin(unsigned long long& v) { asm volatile("" : "+l"(v)); }
 
 // ------------------------------------------------------------------ packed f32x2
 __device__ __forceinline__ unsigned long long f2_pack(float a, float b) {

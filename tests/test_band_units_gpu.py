@@ -1,0 +1,45 @@
+"""The band kernel's forward and grad-x where a thread has two channels of a unit (many units per CTA), one (few), or
+two with the filters read from shared memory (k = 5): channel counts that leave the last unit without its second
+channel, the split that spreads few planes over more CTAs, and inputs near bfloat16's limit."""
+import pytest
+import torch
+
+from tests.util import DTYPES, check_close, make_inputs, oracle_backward, oracle_forward
+
+pytestmark = pytest.mark.gpu
+
+# (B, C, H, W, k, d, s)
+SHAPES = [(8, 131, 50, 67, 3, 1, 1), (7, 259, 40, 70, 3, 2, 1), (17, 75, 100, 75, 3, 1, 2),    # two
+          (1, 43, 50, 67, 3, 1, 1), (1, 37, 14, 13, 3, 1, 1), (3, 11, 7, 9, 3, 2, 1),            # one
+          (2, 37, 50, 67, 5, 1, 1), (1, 5, 14, 13, 5, 2, 1)]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("dt", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("mode", ["mul", "add"])
+def test_matches_oracle(shape, dt, mode):
+    from ddfnet_b200 import _lib, ddf
+    B, C, H, W, k, d, s = shape
+    x, cf, sf, go = make_inputs(B, C, H, W, k, s, DTYPES[dt], 80 + sum(shape))
+    dev = torch.device("cuda:0")
+    xd = x.to(dev).requires_grad_()
+    out = ddf(xd, cf.to(dev), sf.to(dev), k, d, s, mode)
+    check_close(out, oracle_forward(x, cf, sf, k, d, s, mode), DTYPES[dt], f"forward {shape} {dt} {mode}")
+    (gx,) = torch.autograd.grad(out, xd, go.to(dev))
+    check_close(gx, oracle_backward(go, x, cf, sf, k, d, s, mode)[0], DTYPES[dt], f"grad_x {shape} {dt} {mode}")
+    assert _lib.load().ddf_b200_take_fault() == 0
+
+
+@pytest.mark.parametrize("shape", [SHAPES[0], SHAPES[3], SHAPES[6]])
+def test_inputs_near_the_types_limit(shape):
+    """x * sf leaves float's range, x * (cf * sf) does not; see the same test of the plane-ring kernel."""
+    from ddfnet_b200 import ddf
+    B, C, H, W, k, d, s = shape
+    x, cf, sf, _ = make_inputs(B, C, H, W, k, s, torch.bfloat16, 8)
+    x.view(-1)[::29] = -3.3e38
+    cf, sf = (cf * 2.0 ** -8), (sf * 2.0 ** 4)
+    dev = torch.device("cuda:0")
+    out = ddf(x.to(dev), cf.to(dev), sf.to(dev), k, d, s, "mul").cpu().double()
+    want = oracle_forward(x, cf, sf, k, d, s, "mul")
+    assert torch.isfinite(want).all() and torch.isfinite(out).all()
+    assert (out - want).norm() <= 4e-3 * want.norm()

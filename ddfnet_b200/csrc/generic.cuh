@@ -74,10 +74,6 @@ generic_forward(const T* __restrict__ x, const T* __restrict__ cf, const T* __re
     }
 }
 
-template <typename T> __device__ __forceinline__ typename Elem<T>::acc_t to_acc(T v) { return (typename Elem<T>::acc_t)v; }
-template <> __device__ __forceinline__ float to_acc<__half>(__half v) { return __half2float(v); }
-template <> __device__ __forceinline__ float to_acc<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
-
 // grad-x for k = 3, dilation 1, stride 2: the case of the down-sampling layers.  A thread owns one
 // OUTPUT pixel q = (qy, qx) of a sample and walks a chunk of channels; per channel it writes the
 // 2 x 2 input pixels (2qy.., 2qx..).  With stride
@@ -95,27 +91,17 @@ template <> __device__ __forceinline__ float to_acc<__nv_bfloat16>(__nv_bfloat16
 // Same arithmetic as generic_grad_x, without its per-tap divisions and parity tests:
 // (16,128,101x75) f32 20 us against 392.
 // ODD: H or W is odd, or gx is not aligned to two elements; otherwise a row's two results leave as one store.
-// (64,128,56x56) bf16: 22.9 us (24.7 before the loads below were batched); two stores per row 28, and 32 with the tests
-// for odd edges beside them.  Bound by the latency of its loads.
+// (64,128,56x56) bf16: 24 us; two stores per row 28, and 32 with the tests for odd edges beside them.
 template <typename T, int MODE, int CH, bool ODD>
 __global__ void __launch_bounds__(256)
 grad_x_k3s2(const T* __restrict__ go, const T* __restrict__ cf, const T* __restrict__ sf,
             T* __restrict__ gx, Problem p) {
     using A = typename Elem<T>::acc_t;
-    // four channels' loads in flight, and the channel filters out of shared memory: with a channel at a time, its
-    // nine filter values loaded by every thread, the kernel waited for loads (8.9 of 11 stalled warps)
-    constexpr int U = 4, WS = 12;
-    __shared__ __align__(16) A w_s[CH * WS];
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     const int opl = p.OH * p.OW;
-    const long long b = blockIdx.z;
-    const int c_lo = blockIdx.y * CH;
-    const int c_hi = c_lo + CH < p.C ? c_lo + CH : p.C;
-    for (int e = threadIdx.x; e < (c_hi - c_lo) * 9; e += blockDim.x)
-        w_s[e / 9 * WS + e % 9] = (A)Elem<T>::load(cf + (b * p.C + c_lo) * 9 + e);
-    __syncthreads();
     if (q >= opl) return;
     const int qy = q / p.OW, qx = q - qy * p.OW;
+    const long long b = blockIdx.z;
     const bool has_x = qx + 1 < p.OW, has_y = qy + 1 < p.OH;
     const bool odd_x = ODD && !has_x && (p.W & 1), odd_y = ODD && !has_y && (p.H & 1);
     const T* sfb = sf + b * 9 * (long long)opl + q;
@@ -124,61 +110,53 @@ grad_x_k3s2(const T* __restrict__ go, const T* __restrict__ cf, const T* __restr
     const A s3 = sfv(3, 1, has_x), s6 = sfv(6, 1, has_x);
     const A s1 = sfv(1, p.OW, has_y), s2 = sfv(2, p.OW, has_y);
     const A s0 = sfv(0, p.OW + 1, has_x && has_y);
+    const int c_lo = blockIdx.y * CH;
+    const int c_hi = c_lo + CH < p.C ? c_lo + CH : p.C;
     const long long ipl = (long long)p.H * p.W;
-    const int off_x = has_x ? 1 : 0, off_y = has_y ? p.OW : 0;   // a neighbour outside the plane: loaded from here, not used
-    const T* gop = go + (b * p.C + c_lo) * opl + q;
-    T* o = gx + (b * p.C + c_lo) * ipl + (long long)(2 * qy) * p.W + 2 * qx;
-    for (int c = c_lo; c < c_hi; c += U) {
-        T g[U][4];
+    for (int c = c_lo; c < c_hi; ++c) {
+        const long long plane = b * p.C + c;
+        const T* gop = go + plane * opl + q;
+        const T* cfp = cf + plane * 9;
+        A w[9];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const T* at = gop + (c + u < c_hi ? (long long)u * opl : 0);
-            g[u][0] = __ldg(at);
-            g[u][1] = __ldg(at + off_x);
-            g[u][2] = __ldg(at + off_y);
-            g[u][3] = __ldg(at + off_y + off_x);
+        for (int t = 0; t < 9; ++t) w[t] = Elem<T>::load(cfp + t);
+        const A g00 = Elem<T>::load(gop);
+        const A g01 = has_x ? (A)Elem<T>::load(gop + 1) : (A)0;
+        const A g10 = has_y ? (A)Elem<T>::load(gop + p.OW) : (A)0;
+        const A g11 = (has_x && has_y) ? (A)Elem<T>::load(gop + p.OW + 1) : (A)0;
+        const A r00 = g00 * combine_w<MODE, A>(w[4], s4);
+        A r01 = g00 * combine_w<MODE, A>(w[5], s5), r10 = g00 * combine_w<MODE, A>(w[7], s7);
+        A r11 = g00 * combine_w<MODE, A>(w[8], s8);
+        if (has_x) {
+            r01 += g01 * combine_w<MODE, A>(w[3], s3);
+            r11 += g01 * combine_w<MODE, A>(w[6], s6);
         }
-        gop += (long long)U * opl;
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (c + u >= c_hi) break;
-            const A* w = w_s + (c + u - c_lo) * WS;
-            const A g00 = to_acc<T>(g[u][0]), g01 = to_acc<T>(g[u][1]);
-            const A g10 = to_acc<T>(g[u][2]), g11 = to_acc<T>(g[u][3]);
-            const A r00 = g00 * combine_w<MODE, A>(w[4], s4);
-            A r01 = g00 * combine_w<MODE, A>(w[5], s5), r10 = g00 * combine_w<MODE, A>(w[7], s7);
-            A r11 = g00 * combine_w<MODE, A>(w[8], s8);
-            if (has_x) {
-                r01 += g01 * combine_w<MODE, A>(w[3], s3);
-                r11 += g01 * combine_w<MODE, A>(w[6], s6);
-            }
-            if (has_y) {
-                r10 += g10 * combine_w<MODE, A>(w[1], s1);
-                r11 += g10 * combine_w<MODE, A>(w[2], s2);
-            }
-            if (has_x && has_y) r11 += g11 * combine_w<MODE, A>(w[0], s0);
-            if constexpr (!ODD && sizeof(T) == 2) {
-                *reinterpret_cast<uint32_t*>(o) = Word<T>::put(r00, r01);
-                *reinterpret_cast<uint32_t*>(o + p.W) = Word<T>::put(r10, r11);
-            } else if constexpr (!ODD && sizeof(T) == 4) {
-                *reinterpret_cast<float2*>(o) = make_float2(r00, r01);
-                *reinterpret_cast<float2*>(o + p.W) = make_float2(r10, r11);
-            } else {
-                Elem<T>::store(o, r00);
-                Elem<T>::store(o + 1, r01);
-                Elem<T>::store(o + p.W, r10);
-                Elem<T>::store(o + p.W + 1, r11);
-            }
-            if (odd_x) {
-                Elem<T>::store(o + 2, (A)0);
-                Elem<T>::store(o + p.W + 2, (A)0);
-            }
-            if (odd_y) {
-                Elem<T>::store(o + 2 * p.W, (A)0);
-                Elem<T>::store(o + 2 * p.W + 1, (A)0);
-                if (odd_x) Elem<T>::store(o + 2 * p.W + 2, (A)0);
-            }
-            o += ipl;
+        if (has_y) {
+            r10 += g10 * combine_w<MODE, A>(w[1], s1);
+            r11 += g10 * combine_w<MODE, A>(w[2], s2);
+        }
+        if (has_x && has_y) r11 += g11 * combine_w<MODE, A>(w[0], s0);
+        T* o = gx + plane * ipl + (long long)(2 * qy) * p.W + 2 * qx;
+        if constexpr (!ODD && sizeof(T) == 2) {
+            *reinterpret_cast<uint32_t*>(o) = Word<T>::put(r00, r01);
+            *reinterpret_cast<uint32_t*>(o + p.W) = Word<T>::put(r10, r11);
+        } else if constexpr (!ODD && sizeof(T) == 4) {
+            *reinterpret_cast<float2*>(o) = make_float2(r00, r01);
+            *reinterpret_cast<float2*>(o + p.W) = make_float2(r10, r11);
+        } else {
+            Elem<T>::store(o, r00);
+            Elem<T>::store(o + 1, r01);
+            Elem<T>::store(o + p.W, r10);
+            Elem<T>::store(o + p.W + 1, r11);
+        }
+        if (odd_x) {
+            Elem<T>::store(o + 2, (A)0);
+            Elem<T>::store(o + p.W + 2, (A)0);
+        }
+        if (odd_y) {
+            Elem<T>::store(o + 2 * p.W, (A)0);
+            Elem<T>::store(o + 2 * p.W + 1, (A)0);
+            if (odd_x) Elem<T>::store(o + 2 * p.W + 2, (A)0);
         }
     }
 }

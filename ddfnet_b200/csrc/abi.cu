@@ -475,9 +475,14 @@ size_t ddf_b200_backward_workspace(int B, int C, int H, int W, int k, int d, int
     if (device_info(di) == 0) sm = di->sm_count;
     // one call takes one of the two forms; AUTO may take either
     size_t need = bwd_stream_supported(p) ? bwd_stream_workspace(p, sm) : 0, band = 0, least = 0;
-    if (variant == DDF_B200_VARIANT_AUTO && !(need > 0 && stream_worthwhile(p, sm)) &&
-        band_filters_workspace(p, sm, &band, &least) && band > need)
-        need = band;
+    const bool stream = need > 0 && stream_worthwhile(p, sm);
+    if (variant == DDF_B200_VARIANT_AUTO && (!stream || band_cols_preferred(p, sm)) &&
+        band_filters_workspace(p, sm, &band, &least)) {
+        // beside the plane-streaming form, whose scratch grows with the batch, the slices that the array of
+        // ddf_b200_backward_noalloc holds are enough: thousands of CTAs each
+        if (stream && band > kColsScratch) band = least > kColsScratch ? least : kColsScratch;
+        if (band > need) need = band;
+    }
     return need;
 }
 
@@ -498,11 +503,16 @@ int ddf_b200_backward(const void* go, const void* x, const void* cf, const void*
 
     // Decide the filter-gradient path first, so that a missing workspace is reported before
     // anything has been launched.  Only the spatial-filter gradient uses the workspace.
-    const bool filters_stream = (gcf || gsf) && allow_stream && want && bwd_stream_supported(p);
+    bool filters_stream = (gcf || gsf) && allow_stream && want && bwd_stream_supported(p);
     if (filters_stream && gsf) {
         const size_t need = bwd_stream_workspace(p, di->sm_count);
         if (need > 0 && (!workspace || workspace_bytes < need)) return DDF_B200_E_WORKSPACE;
     }
+    size_t band = 0, least = 0;
+    const bool band_ok = (gcf || gsf) && allow_stream && variant == DDF_B200_VARIANT_AUTO &&
+                         band_filters_workspace(p, di->sm_count, &band, &least) &&
+                         (least == 0 || (workspace && workspace_bytes >= least && (reinterpret_cast<uintptr_t>(workspace) & 7u) == 0));
+    if (band_ok && band_cols_preferred(p, di->sm_count)) filters_stream = false;
 
     // grad wrt x: the streaming forward kernel run over go with mirrored taps.
     if (gx) {
@@ -555,9 +565,7 @@ int ddf_b200_backward(const void* go, const void* x, const void* cf, const void*
         }
         if (!done && variant == DDF_B200_VARIANT_STREAM) return DDF_B200_E_UNSUPPORTED;
         // the band form; a caller without scratch for it gets the generic kernels, which need none
-        size_t band = 0, least = 0;
-        if (!done && allow_stream && band_filters_workspace(p, di->sm_count, &band, &least) &&
-            (least == 0 || (workspace && workspace_bytes >= least && (reinterpret_cast<uintptr_t>(workspace) & 7u) == 0))) {
+        if (!done && band_ok) {
             int launches = 0;
             rc = band_filters(p, go, x, cf, sf, gcf, gsf, workspace, workspace_bytes, di->sm_count, di->fault, di->index,
                               st, &launches);

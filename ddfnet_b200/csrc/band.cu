@@ -1,13 +1,27 @@
 // Band filter gradients: host-side entry (see band.cuh).
 #include "band.cuh"
 
-#include "band_bwd.cuh"
+#include "band_bwd_cols.cuh"
 
 namespace ddf {
 
+// The plane-streaming form takes a row in pieces of four pixels where four divide it, else of two or one, and its
+// instructions per channel are then spread over as few pixels.  us, plane-streaming -> a thread per tap column:
+// (64,512,14x14) f16 59.6 -> 41.8, bf16 k = 5 167 -> 124; (64,512,7x7) f16 35.3 -> 28.8, bf16 k = 5 123 -> 64.  With
+// four: (64,256,28x28) bf16 49.7 -> 80.6, k = 5 186 -> 188; (128,64,56x56) bf16 117 -> 120.  Where five eighths of the
+// lanes have no pixel it takes many planes to be worth it ((16,256,9x11) bf16 11.1 -> 12.5, (8,512,7x7) 11.0 both), and
+// two-pixel pieces with dilation 2 are level ((16,256,22x26) bf16 22.2 -> 22.9).
+bool band_cols_preferred(const Problem& p, int sm_count) {
+    BandColsSplit s;
+    if (p.OW % 4 == 0 || (p.k == 3 && p.d != 1) || !band_cols_split(p, sm_count, s)) return false;
+    const long long lanes = (long long)s.bands * s.col_warps * 32 * kColsPixels;
+    return 5 * lanes <= 8ll * p.OH * p.OW || (long long)p.B * p.C >= 8192;
+}
+
 bool band_filters_workspace(const Problem& p, int sm_count, size_t* bytes, size_t* least) {
-    BandBwdSplit s;
-    if (!band_filters_split(p, sm_count, s)) return false;
+    BandColsSplit s;
+    const bool cols = p.dtype != DDF_B200_F32 && p.s == 1;
+    if (!(cols ? band_cols_split(p, sm_count, s) : band_filters_split(p, sm_count, s))) return false;
     *least = band_part_sf(p, s) + band_part_cf(p, s);
     size_t samples = *least > 0 ? kBandBwdScratch / *least : 1;
     if (samples < 1) samples = 1;

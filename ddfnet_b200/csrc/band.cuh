@@ -9,6 +9,10 @@ namespace ddf {
 // false when the band form is not built for p.
 bool band_filters_workspace(const Problem& p, int sm_count, size_t* bytes, size_t* least);
 
+// Whether AUTO takes the form of a thread per tap column (band_bwd_cols.cuh) where the plane-streaming form is built too.
+bool band_cols_preferred(const Problem& p, int sm_count);
+constexpr size_t kColsScratch = 16u << 20;
+
 // kNotHandled: not built, or a tensor is not aligned for bulk copies.  `workspace` holds at
 // least what band_filters_workspace says, aligned to 8 bytes; the results do not depend on how much.
 int band_filters(const Problem& p, const void* go, const void* x, const void* cf, const void* sf, void* gcf, void* gsf,

@@ -1,5 +1,6 @@
 // Band form of the two filter gradients, for planes of any height and any width up to 320 output columns (see
-// band_fwd.cuh for the bands, the ring and the thread layout):
+// band_fwd.cuh for the bands, the ring and the thread layout; the 2-byte types take it at stride 2, at stride 1 see
+// band_bwd_cols.cuh):
 //
 //   gcf[b,c,t]   = sum_{y,x} go[b,c,y,x] * x[b,c,y*s+oi,x*s+oj] * (sf[b,t,y,x] | 1)
 //   gsf[b,t,y,x] = sum_c     go[b,c,y,x] * x[b,c,y*s+oi,x*s+oj] * (cf[b,c,t]   | 1)
@@ -12,11 +13,11 @@
 //
 // The sums over channels are compensated for float tensors, as in the generic kernels this one stands in
 // for, and their partials are doubles: relative error of gsf against 64 bits at (4,128,50x67) 4.4e-8, as the
-// generic kernel's; Kahan sums and float partials gave 5.4e-8 (and 256 us instead of 300 at (2,256,200x300);
+// generic kernel's; Kahan sums and float partials gave 5.4e-8 (and 256 us instead of 300 at (2,256,200x300), now 280;
 // the generic kernels 3230).  For the 2-byte types the final rounding is 2^13 (f16) or 2^16 (bf16) times a
 // float's, and the sums are plain, over 64 channels at most before a compensated sum takes them: the error of
-// gsf against 64 bits is the generic kernel's to six digits (2.1e-4 f16, 1.66e-3 bf16; 77 drawn problems), and
-// (2,256,200x300) bf16 takes 180 us, bound by issue as the forward is, where Kahan's sum takes 265.
+// gsf against 64 bits is the generic kernel's to six digits (2.1e-4 f16, 1.66e-3 bf16; 77 drawn problems); Kahan's sum
+// took (2,256,200x300) bf16 from 180 to 265 us.
 // gcf: the pixels of a warp are added as a tree, in plain float, the warps and bands compensated.  Error for
 // float against 64 bits 0.94 to 1.005 times the generic kernel's (which adds a thread's pixels compensated and
 // the threads plainly), for the 2-byte types the same to six digits.
@@ -178,11 +179,14 @@ band_filters_kernel(const __grid_constant__ BandBwdPlan pl) {
         rowbits |= ok ? 1u << r : 0u;
         rowoff[r] = ok ? (uint32_t)pip * (uint32_t)xplane + (uint32_t)(((iy - iy_lo) * pl.W + x * S) * ES)
                        : pl.zero_off + 16u;
+        pin(rowoff[r]);
     }
 #pragma unroll
-    for (int p = 0; p < PH; ++p)
+    for (int p = 0; p < PH; ++p) {
         gooff[p] = p < rows_left ? (uint32_t)pip * (uint32_t)gplane + (uint32_t)(((y0 + D * p - y_lo) * pl.OW + x) * ES)
                                  : pl.zero_off + 16u - pl.go_off;
+        pin(gooff[p]);
+    }
     uint32_t cmask[K];
 #pragma unroll
     for (int j = 0; j < K; ++j) {
@@ -190,6 +194,7 @@ band_filters_kernel(const __grid_constant__ BandBwdPlan pl) {
         const bool ok = ix >= 0 && ix < pl.W;
         colbits |= ok ? 1u << j : 0u;
         cmask[j] = Masked<T>::mask(ok);
+        pin(cmask[j]);
     }
     // products with padding zeros, or of pixels outside the plane, in this thread / warp
     const bool edge = colbits != (1u << K) - 1u || rowbits != (1u << NR) - 1u || rows_left < PH;
@@ -223,7 +228,10 @@ band_filters_kernel(const __grid_constant__ BandBwdPlan pl) {
                 v[p] = p < rows_left ? w : 0.f;
             }
 #pragma unroll
-            for (int q = 0; q < HP; ++q) sf2[(t % K) * K + t / K][q] = f2_pack(v[q], v[q + HP]);
+            for (int q = 0; q < HP; ++q) {
+                sf2[(t % K) * K + t / K][q] = f2_pack(v[q], v[q + HP]);
+                pin(sf2[(t % K) * K + t / K][q]);
+            }
         }
     }
     band_sync(NW * 32);
@@ -527,6 +535,27 @@ struct BandBwdArgs {
     uint32_t tx_skew = 0;
 };
 
+// The second launch of a slice of samples: the partials added up.
+template <typename T>
+int band_reduce_launch(const BandBwdArgs& a, const BandBwdSplit& sp, const BandBwdPlan& pl, int b0, int nb, cudaStream_t stream,
+                       int* launches) {
+    if (!pl.part_sf && !pl.part_cf) return 0;
+    const long long kk = a.p.k * a.p.k, sf_size = kk * a.p.OH * a.p.OW, cf_size = a.p.C * kk;
+    auto blocks = [&](long long n) {
+        const long long most = 4ll * a.sm_count;
+        return (int)((n + 255) / 256 < most ? (n + 255) / 256 : most);
+    };
+    const int nb_sf = pl.part_sf ? blocks(sf_size * nb) : 0, nb_cf = pl.part_cf ? blocks(cf_size * nb) : 0;
+    T* gsf = pl.part_sf ? reinterpret_cast<T*>(a.gsf) + b0 * sf_size : nullptr;
+    T* gcf = pl.part_cf ? reinterpret_cast<T*>(a.gcf) + b0 * cf_size : nullptr;
+    const cudaError_t e = launch_overlapped(band_reduce_kernel<T>, dim3((unsigned)(nb_sf + nb_cf)), dim3(256), 0, stream, true,
+                                            (const BandPart<T>*)pl.part_sf, gsf, sp.chunks, sf_size, (const float*)pl.part_cf,
+                                            gcf, sp.bands, cf_size, nb, nb_sf);
+    if (e != cudaSuccess) return (int)e;
+    ++*launches;
+    return 0;
+}
+
 template <typename T, int K, int D, int S, int MODE>
 int band_filters_launch(const BandBwdArgs& a, cudaStream_t stream, int* launches) {
     constexpr int PH = kBandBwdPixels<K>, ES = (int)sizeof(T);
@@ -582,7 +611,6 @@ int band_filters_launch(const BandBwdArgs& a, cudaStream_t stream, int* launches
         if (e != cudaSuccess) return (int)e;
         opted_in.fetch_or(bit, std::memory_order_release);
     }
-    const long long sf_size = (long long)K * K * p.OH * p.OW, cf_size = (long long)p.C * K * K;
     for (int b0 = 0; b0 < p.B; b0 += samples) {
         const int nb = p.B - b0 < samples ? p.B - b0 : samples;
         pl.b0 = b0;
@@ -590,19 +618,8 @@ int band_filters_launch(const BandBwdArgs& a, cudaStream_t stream, int* launches
                                           dim3((unsigned)(sp.warps + 1) * 32), smem, stream, true, pl);
         if (e != cudaSuccess) return (int)e;
         ++*launches;
-        if (!pl.part_sf && !pl.part_cf) continue;
-        auto blocks = [&](long long n) {
-            const long long most = 4ll * a.sm_count;
-            return (int)((n + 255) / 256 < most ? (n + 255) / 256 : most);
-        };
-        const int nb_sf = pl.part_sf ? blocks(sf_size * nb) : 0, nb_cf = pl.part_cf ? blocks(cf_size * nb) : 0;
-        T* gsf = pl.part_sf ? reinterpret_cast<T*>(a.gsf) + b0 * sf_size : nullptr;
-        T* gcf = pl.part_cf ? reinterpret_cast<T*>(a.gcf) + b0 * cf_size : nullptr;
-        e = launch_overlapped(band_reduce_kernel<T>, dim3((unsigned)(nb_sf + nb_cf)), dim3(256), 0, stream, true,
-                              (const BandPart<T>*)pl.part_sf, gsf, sp.chunks, sf_size, (const float*)pl.part_cf, gcf, sp.bands,
-                              cf_size, nb, nb_sf);
-        if (e != cudaSuccess) return (int)e;
-        ++*launches;
+        const int rc = band_reduce_launch<T>(a, sp, pl, b0, nb, stream, launches);
+        if (rc) return rc;
     }
     return 0;
 }

@@ -146,11 +146,13 @@ int ddf_b200_backward_noalloc(const void* go, const void* x, const void* cf, con
             if (rc) return rc;
         }
         int launches = 0;
-        rc = bwd_stream_filters(p, go, x, cf, sf, gcf, gsf, scratch, sm_count, fault, index,
-                                reinterpret_cast<cudaStream_t>(stream), &launches);
+        rc = band_cols_preferred(p, sm_count)
+                 ? kNotHandled
+                 : bwd_stream_filters(p, go, x, cf, sf, gcf, gsf, scratch, sm_count, fault, index,
+                                      reinterpret_cast<cudaStream_t>(stream), &launches);
         if (rc != kNotHandled) return rc;
     }
-    // Outside the streaming kernel's range: the band kernel where the array holds its scratch for one sample,
+    // Outside the streaming kernel's range, or where the band form is the faster one: the band kernel where the array holds its scratch for one sample,
     // else the generic kernels, which use no scratch at all.
     size_t band = 0, least = 0;
     if (band_filters_workspace(p, sm_count, &band, &least) && least <= kStaticScratchBytes) {

@@ -202,6 +202,9 @@ int ddf_b200_plan(int B, int C, int H, int W, int k, int d, int s,
  * ddf_b200_plan says GENERIC it is at most 256 MiB, unless a single sample needs more,
  * and less scratch (or none) is no error: the filter gradients then take fewer samples
  * at a time, with the same results, or, without room for one, the generic kernels.
+ * Where it says STREAM, less than the plane-streaming form's own need is an error when gsf
+ * is asked for; 2-byte planes whose width four does not divide take another form and ask
+ * for up to 16 MiB if that is more.
  * The reference makes its caller allocate three zero-filled scratch tensors
  * (ddf/ddf.py:106-108, resized in ddf/src/cuda/ddf_mul_cuda.cpp:85-87); here the
  * caller provides one untyped block, 256-byte aligned, which need not be zeroed.

@@ -2,18 +2,24 @@
 // the pooled sums the channel branch needs, so that a channels_last network runs its DDF
 // layers without any layout copy.
 //
-// Mapping.  A thread owns 8 adjacent channels (one 16-byte vector) of one output pixel column.  Its channel-filter values -- K*K taps x 8 channels, fixed for a sample -- sit in
+// Mapping.  A thread owns 8 adjacent channels (one 16-byte vector) of one output pixel column.  Its channel-filter
+// values -- K*K taps x 8 channels, fixed for a sample -- sit in
 // registers as packed 2-byte pairs laid out like the input words (channels 2q, 2q+1 in word
 // q), so the mixed-precision FMA forms x * cf for both halves of a word without any
 // unpacking:  y = x * cf (exact in float),  acc = fma(y, sf, acc)  with the pixel's
-// spatial-filter value in float.  The spatial filter is the same for all channels of a
-// pixel: every thread takes its pixels' K*K values (adding the convolution bias and applying
-// the spatial FilterNorm in float when asked to) once per pixel and reuses them for its 8
-// channels.  The threads of a pixel read C contiguous channels -- full 128-byte lines --
-// and the 3 x 3 window of a thread overlaps its neighbours', which the L1 cache
-// absorbs: there is no shared-memory staging and no barrier in this kernel.  Pixels outside
-// the image are not loaded (zeros take their place).  An optional per-channel affine map
+// spatial-filter value in float.  An optional per-channel affine map
 // and ReLU (an eval-mode BatchNorm + activation) ride on the store.
+//
+// Movement.  A CTA's threads cover all channels of a few columns; a tile is these columns of a few output rows.
+// The CTAs are persistent and walk neighbouring tiles, the next tile's input rows (one contiguous run each, with the
+// halo columns) arriving by bulk copies in the other of two buffers meanwhile.  Three columns' threads read each
+// vector, and a row serves three output rows; loaded from global memory by each of them, one row ahead, the kernel had
+// some 8 KB of distinct data in flight per SM and ran at a sixth of the memory's rate.  Pixels outside
+// the image are not read (zeros take their place).  The spatial filter is the same for all channels of a pixel: bias
+// and FilterNorm are applied once per pixel, by one thread, and the result is left in shared memory.
+// The sixteen layers of a ResNet-50 at 256 images of 224 x 224, float16: 822 -> 670 us.  Bound now by the 14 warps that an SM
+// holds at 128 registers (44 % of the issue slots), which meet at a barrier once per tile, and the FMA pipe (49 % of
+// the instructions are the FMAs).
 #include <atomic>
 
 #include "common.cuh"
@@ -37,9 +43,12 @@ struct NhwcPlan {
     int relu;
     float sf_scale;
     int vecs;               // C / 8
-    int slots;              // strips a CTA works on = blockDim / vecs
-    int strip_rows;         // output rows per strip
-    int sf_vector;          // the K*K values of a pixel are contiguous and 16-byte aligned
+    int cols, rows;         // output columns and rows of a tile
+    int tiles_x, tiles_y;   // tiles of an image
+    int tiles;              // of all images
+    int sf_bulk;            // a pixel's K*K values are contiguous, 16-byte aligned, and so are a row's pixels: bulk copies
+    uint32_t off_sf, sf_stride, off_affine, off_buf, buf_stride, off_raw, row_bytes;  // off_raw: inside a buffer
+    int* fault;
 };
 
 __device__ __forceinline__ uint4 ldg128(const void* p) {
@@ -55,220 +64,318 @@ template <> __device__ __forceinline__ float elem_to_float<__half>(uint32_t h) {
 }
 template <typename T> __device__ __forceinline__ uint32_t pack2(float a, float b) { return Word<T>::put(a, b); }
 
+template <typename T> __device__ __forceinline__ uint32_t relu2(uint32_t v);   // of two packed values; NaN becomes 0, as fmaxf makes it
+template <> __device__ __forceinline__ uint32_t relu2<__half>(uint32_t v) {
+    uint32_t r;
+    asm("max.f16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(0u));
+    return r;
+}
+template <> __device__ __forceinline__ uint32_t relu2<__nv_bfloat16>(uint32_t v) {
+    uint32_t r;
+    asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(0u));
+    return r;
+}
+
 constexpr int kNhwcThreads = 256;
+constexpr int kNhwcRows = 8;   // output rows of a tile at most
 
-// A thread walks a strip of output rows: PX adjacent columns wide, up to `strip_rows` high.
-// Going down one output row it loads only the input rows it has not seen (one at stride 1,
-// two at stride 2) and keeps the others in registers; the loop is unrolled by three so that
-// the row rotation is register renaming, not moves.
+// Bytes of a pixel's filter in shared memory: mul (s, s) float pairs, add packed 2-byte values; whole 16s.
+template <int MODE> constexpr uint32_t kNhwcPixel = MODE == DDF_B200_MUL ? 80 : 32;
+
 // NORM: `sf` holds the raw output of the spatial branch's convolution; bias and FilterNorm here.
-template <typename T, int S, int PX, int MODE, bool NORM>
-__global__ void __launch_bounds__(kNhwcThreads, 2) nhwc_forward_kernel(const NhwcPlan pl) {
+template <typename T, int S, int MODE, bool NORM>
+__global__ void __launch_bounds__(kNhwcThreads, 2) nhwc_forward_kernel(const __grid_constant__ NhwcPlan pl) {
     constexpr int K = 3, KK = 9;
-    constexpr int NCOL = (PX - 1) * S + 3;
+    constexpr bool MUL = MODE == DDF_B200_MUL;
+    constexpr uint32_t PXB = kNhwcPixel<MODE>;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const uint32_t sbase = smem_u32(smem_raw);
     const int tid = threadIdx.x;
-    const int vec = tid % pl.vecs, slot = tid / pl.vecs;
-    const int b = blockIdx.y;
+    const int vec = tid % pl.vecs, col = tid / pl.vecs;
     const int C = pl.C, W = pl.W, H = pl.H, OW = pl.OW, OH = pl.OH;
-    const int ppr = OW / PX;                                  // column groups per row
-    const int strip = blockIdx.x * pl.slots + slot;
-    const int seg = strip / ppr, cg = strip - seg * ppr;
-    const int oy0 = seg * pl.strip_rows;
-    if (oy0 >= OH) return;
-    const int oy1 = (oy0 + pl.strip_rows) < OH ? (oy0 + pl.strip_rows) : OH;
-    const int ox0 = cg * PX;
-    const T* xb = reinterpret_cast<const T*>(pl.x) + (size_t)b * H * W * C + vec * 8;
-    T* op = reinterpret_cast<T*>(pl.out) + ((size_t)b * OH * OW + (size_t)oy0 * OW + ox0) * C + vec * 8;
-    const T* sp = reinterpret_cast<const T*>(pl.sf) + (long long)b * pl.sf_batch_stride +
-                  ((long long)oy0 * OW + ox0) * pl.sf_pixel_stride;
+    const uint32_t affine = sbase + pl.off_affine;
+#define NH_FULL(i) (sbase + 8u * (uint32_t)(i))
+#define NH_BUF(i) (sbase + pl.off_buf + (uint32_t)(i) * pl.buf_stride)
 
-    // channel filter of this thread's 8 channels: 72 contiguous values -> cfw[t][q] = channels (2q, 2q+1) of tap t
-    uint32_t cfw[KK][4];
-    {
-        const uint4* cp = reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(pl.cf) + ((size_t)b * C + vec * 8) * KK);
-        uint32_t raw[36];
-#pragma unroll
-        for (int v = 0; v < 9; ++v) {
-            const uint4 u = ldg128(cp + v);
-            raw[4 * v] = u.x; raw[4 * v + 1] = u.y; raw[4 * v + 2] = u.z; raw[4 * v + 3] = u.w;
+    if (tid == 0) {
+        mbar_init(NH_FULL(0), 1);
+        mbar_init(NH_FULL(1), 1);
+        mbar_fence_init();
+    }
+    if (tid < KK) sts32(sbase + 16u + 4u * tid, pl.sf_bias != nullptr ? __float_as_uint(__ldg(pl.sf_bias + tid)) : 0u);
+    if (pl.oscale != nullptr)
+        for (int c = tid; c < C; c += kNhwcThreads) {
+            sts32(affine + 4u * c, __float_as_uint(__ldg(pl.oscale + c)));
+            sts32(affine + 4u * (C + c), __float_as_uint(__ldg(pl.oshift + c)));
         }
-#pragma unroll
-        for (int t = 0; t < KK; ++t) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int ha = (2 * q) * KK + t, hb = (2 * q + 1) * KK + t;   // element indices
-                const uint32_t lo = (ha & 1) ? (raw[ha / 2] >> 16) : (raw[ha / 2] & 0xffffu);
-                const uint32_t hi = (hb & 1) ? (raw[hb / 2] & 0xffff0000u) : (raw[hb / 2] << 16);
-                cfw[t][q] = lo | hi;
+    __syncthreads();
+
+    const int t_lo = (int)(((long long)pl.tiles * blockIdx.x) / gridDim.x);
+    const int t_hi = (int)(((long long)pl.tiles * (blockIdx.x + 1)) / gridDim.x);
+    // tiles run along a row of tiles, down an image, image by image; found by division once
+    struct Tile { int b, ox0, oy0, nx, ny; };
+    auto clip = [&](Tile& r) {
+        r.nx = OW - r.ox0 < pl.cols ? OW - r.ox0 : pl.cols;
+        r.ny = OH - r.oy0 < pl.rows ? OH - r.oy0 : pl.rows;
+    };
+    auto next_of = [&](Tile r) {
+        r.ox0 += pl.cols;
+        if (r.ox0 >= OW) {
+            r.ox0 = 0;
+            r.oy0 += pl.rows;
+            if (r.oy0 >= OH) {
+                r.oy0 = 0;
+                ++r.b;
             }
         }
+        clip(r);
+        return r;
+    };
+    Tile r;
+    {
+        const int per = pl.tiles_x * pl.tiles_y, in = t_lo % per, ty = in / pl.tiles_x;
+        r.b = t_lo / per;
+        r.ox0 = (in - ty * pl.tiles_x) * pl.cols;
+        r.oy0 = ty * pl.rows;
+        clip(r);
     }
-    // which window columns lie inside the image (the same for every row of the strip)
-    bool colok[NCOL];
-#pragma unroll
-    for (int cidx = 0; cidx < NCOL; ++cidx) {
-        const int ix = ox0 * S + cidx - 1;
-        colok[cidx] = ix >= 0 && ix < W;
-    }
-    const T* xcol = xb + (ptrdiff_t)(ox0 * S - 1) * C;   // window column 0 of input row 0
-    auto load_row = [&](int iy, uint32_t (&v)[NCOL][4]) {
-        const bool rowok = iy >= 0 && iy < H;
-        const T* rp = xcol + (size_t)(rowok ? iy : 0) * W * C;
-#pragma unroll
-        for (int cidx = 0; cidx < NCOL; ++cidx) {
-            uint4 u = make_uint4(0u, 0u, 0u, 0u);
-            if (rowok && colok[cidx]) u = ldg128(rp + (size_t)cidx * C);
-            v[cidx][0] = u.x; v[cidx][1] = u.y; v[cidx][2] = u.z; v[cidx][3] = u.w;
+    // the first warp: the tile's input rows and its raw filters into a buffer, a row per lane.  Window column 0 of the
+    // tile lies at a row's start, window row 0 at the buffer's.
+    auto request = [&](const Tile& r, int buf) {
+        const int ix0 = r.ox0 * S - 1, iy0 = r.oy0 * S - 1;
+        const int cx0 = ix0 > 0 ? ix0 : 0, cx1 = (ix0 + (r.nx - 1) * S + K) < W ? (ix0 + (r.nx - 1) * S + K) : W;
+        const int cy0 = iy0 > 0 ? iy0 : 0, cy1 = (iy0 + (r.ny - 1) * S + K) < H ? (iy0 + (r.ny - 1) * S + K) : H;
+        const int n = cy1 - cy0;
+        const uint32_t bytes = (uint32_t)(cx1 - cx0) * (uint32_t)C * 2u;
+        const uint32_t sfb = pl.sf_bulk ? (uint32_t)(r.nx * (int)pl.sf_pixel_stride) * 2u : 0u;
+        // behind the tensor's last pixel there may be nothing to read: 8 of its values by the copy, the ninth apart
+        const bool last = pl.sf_bulk && r.b == pl.B - 1 && r.oy0 + r.ny == OH && r.ox0 + r.nx == OW;
+        const uint32_t less = last ? (uint32_t)pl.sf_pixel_stride * 2u - 16u : 0u;
+        if (tid == 0) mbar_arrive_expect_tx(NH_FULL(buf), (uint32_t)n * bytes + (uint32_t)r.ny * sfb - less);
+        __syncwarp();
+        if (tid < n) {
+            bulk_g2s(NH_BUF(buf) + (uint32_t)(cy0 - iy0 + tid) * pl.row_bytes + (uint32_t)((cx0 - ix0) * C * 2),
+                     reinterpret_cast<const T*>(pl.x) + (((size_t)r.b * H + cy0 + tid) * W + cx0) * C, bytes, NH_FULL(buf));
+        } else if (pl.sf_bulk && tid < n + r.ny) {
+            const int y = tid - n;
+            bulk_g2s(NH_BUF(buf) + pl.off_raw + (uint32_t)(y * pl.cols * (int)pl.sf_pixel_stride) * 2u,
+                     reinterpret_cast<const T*>(pl.sf) + r.b * pl.sf_batch_stride +
+                         ((long long)(r.oy0 + y) * OW + r.ox0) * pl.sf_pixel_stride,
+                     y == r.ny - 1 ? sfb - less : sfb, NH_FULL(buf));
         }
     };
+    static_assert((kNhwcRows - 1) * S + K + kNhwcRows <= 32, "a lane per row of a tile and of its filters");
+    if (tid < 32) {
+        if (t_lo < t_hi) request(r, 0);
+        if (t_lo + 1 < t_hi) request(next_of(r), 1);
+    }
 
-    // raw spatial-filter values of PX pixels as packed pairs (taps 2u, 2u+1)
-    auto load_sf = [&](const T* spp0, uint32_t (&raw)[PX][5]) {
+    // a thread's constants of the row loop, kept (see pin)
+    uint32_t row_bytes = pl.row_bytes, pixel_bytes = (uint32_t)C * 2u, aff_s = affine + 32u * (uint32_t)vec;
+    unsigned long long out_step = (unsigned long long)OW * C * 2u;
+    pin(row_bytes);
+    pin(pixel_bytes);
+    pin(aff_s);
+    pin(out_step);
+    uint32_t cfw[KK][4];
+    int cf_of = -1;   // the sample whose channel filters are in registers
+    for (int t = t_lo; t < t_hi; ++t) {
+        const int buf = (t - t_lo) & 1;
+        const bool active = col < r.nx;
+        if (r.b != cf_of) {
+            // channel filter of this thread's 8 channels: 72 contiguous values -> cfw[t][q] = channels (2q, 2q+1) of tap t
+            cf_of = r.b;
+            const uint4* cp = reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(pl.cf) + ((size_t)r.b * C + vec * 8) * KK);
+            uint32_t raw[36];
 #pragma unroll
-        for (int px = 0; px < PX; ++px) {
-            const T* spp = spp0 + (long long)px * pl.sf_pixel_stride;
-            if (pl.sf_vector) {   // K*K contiguous values, 16-byte aligned
-                const uint4 u = ldg128(spp);
-                raw[px][0] = u.x; raw[px][1] = u.y; raw[px][2] = u.z; raw[px][3] = u.w;
-                raw[px][4] = __ldg(reinterpret_cast<const uint16_t*>(spp + 8));
-            } else {
+            for (int v = 0; v < 9; ++v) {
+                const uint4 u = ldg128(cp + v);
+                raw[4 * v] = u.x; raw[4 * v + 1] = u.y; raw[4 * v + 2] = u.z; raw[4 * v + 3] = u.w;
+            }
 #pragma unroll
-                for (int u = 0; u < 5; ++u) {
-                    const uint32_t lo = __ldg(reinterpret_cast<const uint16_t*>(spp + (2 * u) * pl.sf_tap_stride));
-                    const uint32_t hi = 2 * u + 1 < KK ? __ldg(reinterpret_cast<const uint16_t*>(spp + (2 * u + 1) * pl.sf_tap_stride)) : 0u;
-                    raw[px][u] = lo | (hi << 16);
+            for (int k = 0; k < KK; ++k) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int ha = (2 * q) * KK + k, hb = (2 * q + 1) * KK + k;   // element indices
+                    const uint32_t lo = (ha & 1) ? (raw[ha / 2] >> 16) : (raw[ha / 2] & 0xffffu);
+                    const uint32_t hi = (hb & 1) ? (raw[hb / 2] & 0xffff0000u) : (raw[hb / 2] << 16);
+                    cfw[k][q] = lo | hi;
                 }
             }
         }
-    };
-    uint32_t sraw[PX][5];
-    load_sf(sp, sraw);
-    // the spatial branch's bias (added before the FilterNorm), in registers for the whole strip
-    float bias[NORM ? KK : 1];
-    if constexpr (NORM) {
-#pragma unroll
-        for (int t = 0; t < KK; ++t) bias[t] = pl.sf_bias != nullptr ? __ldg(pl.sf_bias + t) : 0.f;
-    }
-
-    uint32_t w0[NCOL][4], w1[NCOL][4], w2[NCOL][4];   // input rows oy*S - 1, oy*S, oy*S + 1
-    load_row(oy0 * S - 1, w0);
-    if constexpr (S == 1) load_row(oy0, w1);
-
-#pragma unroll 3
-    for (int oy = oy0; oy < oy1; ++oy) {
-        if constexpr (S == 2) load_row(oy * 2, w1);
-        load_row(oy * S + 1, w2);
-        // ---- the pixels' spatial-filter values in float (bias, FilterNorm); the raw values were
-        // requested one row ahead, and the next row's are requested now
-        float sfv[PX][KK];
-#pragma unroll
-        for (int px = 0; px < PX; ++px) {
-#pragma unroll
-            for (int t = 0; t < KK; ++t)
-                sfv[px][t] = elem_to_float<T>((t & 1) ? (sraw[px][t / 2] >> 16) : (sraw[px][t / 2] & 0xffffu));
+        if (!mbar_wait(NH_FULL(buf), (uint32_t)(((t - t_lo) >> 1) & 1))) {
+            atomicCAS(pl.fault, 0, (int)kFaultConsumerFull);
+            // the copies requested so far land before the block's memory goes
+            mbar_wait(NH_FULL(buf ^ 1), (uint32_t)(((t + 1 - t_lo) >> 1) & 1));
+            return;
         }
-        sp += (long long)OW * pl.sf_pixel_stride;
-        if (oy + 1 < oy1) load_sf(sp, sraw);
+        // Window columns and rows outside the image: zeros, where the copies left something else.
+        {
+            const int ix0 = r.ox0 * S - 1, iy0 = r.oy0 * S - 1, cols = (r.nx - 1) * S + K, rows = (r.ny - 1) * S + K;
+            auto zero_column = [&](int c) {
+                for (int e = tid; e < rows * pl.vecs; e += kNhwcThreads)
+                    sts128(NH_BUF(buf) + (uint32_t)(e / pl.vecs) * pl.row_bytes + (uint32_t)((c * pl.vecs + e % pl.vecs) * 16), 0u, 0u, 0u, 0u);
+            };
+            auto zero_row = [&](int y) {
+                for (int e = tid; e < cols * pl.vecs; e += kNhwcThreads)
+                    sts128(NH_BUF(buf) + (uint32_t)y * pl.row_bytes + (uint32_t)(e * 16), 0u, 0u, 0u, 0u);
+            };
+            if (ix0 < 0) zero_column(0);
+            if (ix0 + cols > W) zero_column(cols - 1);
+            if (iy0 < 0) zero_row(0);
+            if (iy0 + rows > H) zero_row(rows - 1);
+            if (ix0 < 0 || iy0 < 0 || ix0 + cols > W || iy0 + rows > H)
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // before the copies that come here next
+        }
+        // the filters of the tile's pixels, a pixel per thread and turn
+        const uint32_t filters = sbase + pl.off_sf + (uint32_t)buf * pl.sf_stride;
+        for (int i = tid; i < r.nx * r.ny; i += kNhwcThreads) {
+            const int py = i / r.nx, px = i - py * r.nx;
+            float sv[KK];
+            if (pl.sf_bulk) {
+                const uint32_t from = NH_BUF(buf) + pl.off_raw + (uint32_t)((py * pl.cols + px) * (int)pl.sf_pixel_stride) * 2u;
+                uint32_t raw[5];
+                lds128(from, raw[0], raw[1], raw[2], raw[3]);
+                if (r.b == pl.B - 1 && r.oy0 + py == OH - 1 && r.ox0 + px == OW - 1)
+                    raw[4] = __ldg(reinterpret_cast<const uint16_t*>(pl.sf) + r.b * pl.sf_batch_stride +
+                                   ((long long)OH * OW - 1) * pl.sf_pixel_stride + 8);
+                else raw[4] = lds16(from + 16u);
 #pragma unroll
-        for (int px = 0; px < PX; ++px) {
+                for (int k = 0; k < KK; ++k) sv[k] = elem_to_float<T>((k & 1) ? (raw[k / 2] >> 16) : (raw[k / 2] & 0xffffu));
+            } else {
+                const T* spp = reinterpret_cast<const T*>(pl.sf) + r.b * pl.sf_batch_stride +
+                               ((long long)(r.oy0 + py) * OW + r.ox0 + px) * pl.sf_pixel_stride;
+#pragma unroll
+                for (int k = 0; k < KK; ++k)
+                    sv[k] = elem_to_float<T>(__ldg(reinterpret_cast<const uint16_t*>(spp + k * pl.sf_tap_stride)));
+            }
             if constexpr (NORM) {
                 float sum = 0.f;
 #pragma unroll
-                for (int t = 0; t < KK; ++t) {
-                    sfv[px][t] += bias[t];
-                    sum += sfv[px][t];
+                for (int k = 0; k < KK; ++k) {
+                    sv[k] += ldsf(sbase + 16u + 4u * k);   // (zeros without one)
+                    sum += sv[k];
                 }
                 const float mean = sum * (1.f / KK);
                 float var = 0.f;
 #pragma unroll
-                for (int t = 0; t < KK; ++t) {
-                    sfv[px][t] -= mean;
-                    var = fmaf(sfv[px][t], sfv[px][t], var);
+                for (int k = 0; k < KK; ++k) {
+                    sv[k] -= mean;
+                    var = fmaf(sv[k], sv[k], var);
                 }
                 const float inv = norm_gain(var * (1.f / (KK - 1)), pl.sf_scale);
 #pragma unroll
-                for (int t = 0; t < KK; ++t) sfv[px][t] *= inv;
+                for (int k = 0; k < KK; ++k) sv[k] *= inv;
+            }
+            // a column's pixels in a row, and 16 bytes, so that neighbouring columns lie in different banks
+            const uint32_t at = filters + (uint32_t)px * ((uint32_t)pl.rows * PXB + 16u) + (uint32_t)py * PXB;
+            if constexpr (MUL) {
+#pragma unroll
+                for (int k = 0; k < KK; ++k) sts64(at + 8u * k, __float_as_uint(sv[k]), __float_as_uint(sv[k]));
+            } else {
+                sts128(at, pack2<T>(sv[0], sv[1]), pack2<T>(sv[2], sv[3]), pack2<T>(sv[4], sv[5]), pack2<T>(sv[6], sv[7]));
+                sts32(at + 16u, pack2<T>(sv[8], 0.f));
             }
         }
-        uint32_t sfh[PX][(KK + 1) / 2];   // add mode: the same values as packed 2-byte pairs (taps 2u, 2u+1)
-        if constexpr (MODE == DDF_B200_ADD) {
-#pragma unroll
-            for (int px = 0; px < PX; ++px)
-#pragma unroll
-                for (int u = 0; u < (KK + 1) / 2; ++u)
-                    sfh[px][u] = pack2<T>(sfv[px][2 * u], 2 * u + 1 < KK ? sfv[px][2 * u + 1] : 0.f);
-        }
+        __syncthreads();
+        // every thread is done with the tile before: its buffer takes the next one
+        const Tile next = next_of(r);
+        if (tid < 32 && t > t_lo && t + 1 < t_hi) request(next, buf ^ 1);
 
-        float acc[PX][8];
+        if (active) {
+            const int ox = r.ox0 + col;
+            uint32_t row_s = NH_BUF(buf) + (uint32_t)((col * S * C + vec * 8) * 2);   // the next window row to read
+            auto load_row = [&](uint32_t (&v)[K][4]) {
 #pragma unroll
-        for (int px = 0; px < PX; ++px)
+                for (int j = 0; j < K; ++j) lds128(row_s + (uint32_t)j * pixel_bytes, v[j][0], v[j][1], v[j][2], v[j][3]);
+                row_s += row_bytes;
+            };
+            uint32_t w[3][K][4];   // input rows, round robin
+            load_row(w[0]);
+            if constexpr (S == 1) load_row(w[1]);
+            uint32_t sf_s = filters + (uint32_t)col * ((uint32_t)pl.rows * PXB + 16u);
+            char* op = reinterpret_cast<char*>(pl.out) + ((((size_t)r.b * OH + r.oy0) * OW + ox) * C + vec * 8) * 2;
+            for (int y = 0; y < r.ny;) {
 #pragma unroll
-            for (int c = 0; c < 8; ++c) acc[px][c] = 0.f;
+                for (int u = 0; u < 3; ++u) {
+                    uint32_t (&r0)[K][4] = w[(S * u) % 3];
+                    uint32_t (&r1)[K][4] = w[(S * u + 1) % 3];
+                    uint32_t (&r2)[K][4] = w[(S * u + 2) % 3];
+                    if constexpr (S == 2) load_row(r1);
+                    load_row(r2);
+                    unsigned long long acc2[4] = {0ull, 0ull, 0ull, 0ull};
+                    float acc[8];
+                    unsigned long long sd[MUL ? 10 : 1];
+                    uint32_t sw[MUL ? 1 : 5];
+                    if constexpr (MUL) {
 #pragma unroll
-        for (int i = 0; i < K; ++i) {
+                        for (int k = 0; k < 10; k += 2)
+                            asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(sd[k]), "=l"(sd[k + 1]) : "r"(sf_s + 8u * k));
+                    } else {
+                        lds128(sf_s, sw[0], sw[1], sw[2], sw[3]);
+                        sw[4] = lds32(sf_s + 16u);
 #pragma unroll
-            for (int j = 0; j < K; ++j) {
-                const int t = i * K + j;
+                        for (int c = 0; c < 8; ++c) acc[c] = 0.f;
+                    }
 #pragma unroll
-                for (int px = 0; px < PX; ++px) {
-                    const int cidx = px * S + j;
+                    for (int i = 0; i < K; ++i) {
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const uint32_t xw = i == 0 ? w0[cidx][q] : (i == 1 ? w1[cidx][q] : w2[cidx][q]);
-                        if constexpr (MODE == DDF_B200_MUL) {
-                            // the two channels of a word: exact products, then one packed f32x2 FMA
-                            // against the tap's spatial-filter value (half the issue slots of two FFMAs)
-                            const float y0 = Mix<T>::fmaw(0, 0, xw, cfw[t][q], 0.f);
-                            const float y1 = Mix<T>::fmaw(1, 1, xw, cfw[t][q], 0.f);
-                            const unsigned long long r = f2_fma(f2_pack(y0, y1), f2_pack(sfv[px][t], sfv[px][t]),
-                                                                f2_pack(acc[px][2 * q], acc[px][2 * q + 1]));
-                            f2_unpack(r, acc[px][2 * q], acc[px][2 * q + 1]);
-                        } else {
+                        for (int j = 0; j < K; ++j) {
+                            const int k = i * K + j;
 #pragma unroll
-                            for (int h = 0; h < 2; ++h) {
-                                float a = acc[px][2 * q + h];
-                                a = Mix<T>::fmaw(h, h, xw, cfw[t][q], a);
-                                a = Mix<T>::fmaw(h, t & 1, xw, sfh[px][t / 2], a);
-                                acc[px][2 * q + h] = a;
+                            for (int q = 0; q < 4; ++q) {
+                                const uint32_t xw = i == 0 ? r0[j][q] : (i == 1 ? r1[j][q] : r2[j][q]);
+                                if constexpr (MUL) {
+                                    // the two channels of a word: exact products, then one packed f32x2 FMA
+                                    // against the tap's spatial-filter value (half the issue slots of two FFMAs)
+                                    const float y0 = Mix<T>::fmaw(0, 0, xw, cfw[k][q], 0.f);
+                                    const float y1 = Mix<T>::fmaw(1, 1, xw, cfw[k][q], 0.f);
+                                    acc2[q] = f2_fma(f2_pack(y0, y1), sd[k], acc2[q]);
+                                } else {
+#pragma unroll
+                                    for (int h = 0; h < 2; ++h) {
+                                        float a = acc[2 * q + h];
+                                        a = Mix<T>::fmaw(h, h, xw, cfw[k][q], a);
+                                        a = Mix<T>::fmaw(h, k & 1, xw, sw[k / 2], a);
+                                        acc[2 * q + h] = a;
+                                    }
+                                }
                             }
                         }
                     }
+                    if constexpr (!MUL) {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) acc2[q] = f2_pack(acc[2 * q], acc[2 * q + 1]);
+                    }
+                    if (pl.oscale != nullptr) {
+                        unsigned long long sc[4], sh[4];
+#pragma unroll
+                        for (int q = 0; q < 4; q += 2) {
+                            asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(sc[q]), "=l"(sc[q + 1]) : "r"(aff_s + 8u * q));
+                            asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(sh[q]), "=l"(sh[q + 1]) : "r"(aff_s + 2u * pixel_bytes + 8u * q));
+                        }
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) acc2[q] = f2_fma(acc2[q], sc[q], sh[q]);
+                    }
+                    uint32_t o[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        float lo, hi;
+                        f2_unpack(acc2[q], lo, hi);
+                        o[q] = pack2<T>(lo, hi);
+                        if (pl.relu) o[q] = relu2<T>(o[q]);
+                    }
+                    *reinterpret_cast<uint4*>(op) = make_uint4(o[0], o[1], o[2], o[3]);
+                    op += out_step;
+                    sf_s += PXB;
+                    if (++y >= r.ny) break;
                 }
             }
         }
-#pragma unroll
-        for (int px = 0; px < PX; ++px) {
-            float r[8];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) r[c] = acc[px][c];
-            if (pl.oscale != nullptr) {
-                const float4* sc = reinterpret_cast<const float4*>(pl.oscale + vec * 8);
-                const float4* sh = reinterpret_cast<const float4*>(pl.oshift + vec * 8);
-                const float4 a0 = __ldg(sc), a1 = __ldg(sc + 1), b0 = __ldg(sh), b1 = __ldg(sh + 1);
-                r[0] = fmaf(r[0], a0.x, b0.x); r[1] = fmaf(r[1], a0.y, b0.y); r[2] = fmaf(r[2], a0.z, b0.z); r[3] = fmaf(r[3], a0.w, b0.w);
-                r[4] = fmaf(r[4], a1.x, b1.x); r[5] = fmaf(r[5], a1.y, b1.y); r[6] = fmaf(r[6], a1.z, b1.z); r[7] = fmaf(r[7], a1.w, b1.w);
-            }
-            if (pl.relu) {
-#pragma unroll
-                for (int c = 0; c < 8; ++c) r[c] = fmaxf(r[c], 0.f);
-            }
-            const uint4 o = make_uint4(pack2<T>(r[0], r[1]), pack2<T>(r[2], r[3]), pack2<T>(r[4], r[5]), pack2<T>(r[6], r[7]));
-            *reinterpret_cast<uint4*>(op + (size_t)px * C) = o;
-        }
-        op += (size_t)OW * C;
-        // rotate the rows: what was below becomes what is above
-        if constexpr (S == 1) {
-#pragma unroll
-            for (int cidx = 0; cidx < NCOL; ++cidx)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) { w0[cidx][q] = w1[cidx][q]; w1[cidx][q] = w2[cidx][q]; }
-        } else {
-#pragma unroll
-            for (int cidx = 0; cidx < NCOL; ++cidx)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) w0[cidx][q] = w2[cidx][q];
-        }
+        r = next;
     }
+#undef NH_FULL
+#undef NH_BUF
 }
 
 // Partial sums of x over tiles of 196 pixels: partials[b][tile][c] (float), for the channel branch's
@@ -303,26 +410,30 @@ __global__ void __launch_bounds__(256) nhwc_pool_kernel(const T* __restrict__ x,
     }
 }
 
-template <typename T, int S, int PX>
-static int nhwc_launch(const NhwcPlan& pl, int combine, int norm, dim3 grid, cudaStream_t st) {
-    if (combine == DDF_B200_MUL) {
-        if (norm) nhwc_forward_kernel<T, S, PX, DDF_B200_MUL, true><<<grid, kNhwcThreads, 0, st>>>(pl);
-        else nhwc_forward_kernel<T, S, PX, DDF_B200_MUL, false><<<grid, kNhwcThreads, 0, st>>>(pl);
-    } else {
-        if (norm) nhwc_forward_kernel<T, S, PX, DDF_B200_ADD, true><<<grid, kNhwcThreads, 0, st>>>(pl);
-        else nhwc_forward_kernel<T, S, PX, DDF_B200_ADD, false><<<grid, kNhwcThreads, 0, st>>>(pl);
+// Most dynamic shared memory of the forward kernel: two CTAs per SM.
+constexpr uint32_t kNhwcSmem = 112 * 1024;
+
+template <typename T, int S, int MODE>
+static int nhwc_launch(const NhwcPlan& pl, int norm, uint32_t smem, int device, dim3 grid, cudaStream_t st) {
+    auto kern = norm ? nhwc_forward_kernel<T, S, MODE, true> : nhwc_forward_kernel<T, S, MODE, false>;
+    static std::atomic<unsigned long long> opted_in[2];
+    const unsigned long long bit = 1ull << (device & 63);
+    if (!(opted_in[norm ? 1 : 0].load(std::memory_order_acquire) & bit)) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNhwcSmem);
+        if (e != cudaSuccess) return (int)e;
+        opted_in[norm ? 1 : 0].fetch_or(bit, std::memory_order_release);
     }
+    kern<<<grid, kNhwcThreads, smem, st>>>(pl);
     return (int)cudaGetLastError();
 }
 
-// One pixel column per thread: two columns would halve the window loads per output but need
-// 48 registers for the window alone, which does not fit beside the resident channel filter.
-constexpr int kNhwcPX = 1;
-
 template <typename T>
-static int nhwc_dispatch(const NhwcPlan& pl, int s, int combine, int norm, dim3 grid, cudaStream_t st) {
-    if (s == 1) return nhwc_launch<T, 1, kNhwcPX>(pl, combine, norm, grid, st);
-    return nhwc_launch<T, 2, kNhwcPX>(pl, combine, norm, grid, st);
+static int nhwc_dispatch(const NhwcPlan& pl, int s, int combine, int norm, uint32_t smem, int device, dim3 grid, cudaStream_t st) {
+    if (combine == DDF_B200_MUL)
+        return s == 1 ? nhwc_launch<T, 1, DDF_B200_MUL>(pl, norm, smem, device, grid, st)
+                      : nhwc_launch<T, 2, DDF_B200_MUL>(pl, norm, smem, device, grid, st);
+    return s == 1 ? nhwc_launch<T, 1, DDF_B200_ADD>(pl, norm, smem, device, grid, st)
+                  : nhwc_launch<T, 2, DDF_B200_ADD>(pl, norm, smem, device, grid, st);
 }
 
 }  // namespace ddf
@@ -384,21 +495,42 @@ int ddf_b200_forward_nhwc(const void* x, const void* cf, const void* sf, const f
     pl.sf_batch_stride = sf_batch_stride; pl.sf_pixel_stride = sf_pixel_stride; pl.sf_tap_stride = sf_tap_stride;
     pl.relu = relu; pl.sf_scale = (float)sf_scale;
     pl.vecs = C / 8;
-    pl.slots = kNhwcThreads / pl.vecs;
-    // Strips of output rows, PX columns wide: long enough that the two extra input rows a
-    // strip reads are a small share, short enough that there are a few CTAs per SM.
-    const int ppr = pl.OW / kNhwcPX;
-    int rows = pl.OH < 8 ? pl.OH : 8;
-    auto n_ctas = [&](int r) { return (long long)B * (((long long)ppr * ((pl.OH + r - 1) / r) + pl.slots - 1) / pl.slots); };
-    while (rows > 2 && n_ctas(rows) < 4ll * sm_count) rows = (rows + 1) / 2;
-    pl.strip_rows = rows;
-    const long long strips = (long long)ppr * ((pl.OH + rows - 1) / rows);
-    dim3 grid((unsigned)((strips + pl.slots - 1) / pl.slots), (unsigned)B);
-    // vector loads of the spatial filter: taps contiguous, pixels 16-byte aligned
-    pl.sf_vector = (sf_tap_stride == 1 && sf_pixel_stride % 8 == 0 && sf_batch_stride % 8 == 0 && al16(sf)) ? 1 : 0;
+    pl.fault = fault;
+    // Tiles: equal column counts, as many as the threads cover; rows as two buffers of two CTAs leave room for (the
+    // two halo rows are then a quarter of the copies at most), fewer where the chip would not be full.
+    const int most = kNhwcThreads / pl.vecs;
+    pl.tiles_x = (pl.OW + most - 1) / most;
+    pl.cols = (pl.OW + pl.tiles_x - 1) / pl.tiles_x;
+    pl.tiles_x = (pl.OW + pl.cols - 1) / pl.cols;
+    const uint32_t pixel = combine == DDF_B200_MUL ? kNhwcPixel<DDF_B200_MUL> : kNhwcPixel<DDF_B200_ADD>;
+    // bulk copies of the raw filters: taps contiguous, whole 16 bytes a pixel, pixels of a row one after the other
+    pl.sf_bulk = (sf_tap_stride == 1 && sf_pixel_stride % 8 == 0 && sf_pixel_stride >= 16 && sf_pixel_stride <= 64 &&
+                  sf_batch_stride % 8 == 0 && al16(sf)) ? 1 : 0;
+    pl.row_bytes = (uint32_t)(((pl.cols - 1) * s + 3) * C * 2);
+    auto layout = [&](int r) {
+        pl.off_sf = 64;
+        pl.sf_stride = (uint32_t)pl.cols * ((uint32_t)r * pixel + 16u);
+        pl.off_affine = pl.off_sf + 2u * pl.sf_stride;
+        pl.off_buf = (pl.off_affine + 8u * (uint32_t)C + 127u) & ~127u;
+        pl.off_raw = (uint32_t)((r - 1) * s + 3) * pl.row_bytes;
+        pl.buf_stride = (pl.off_raw + (pl.sf_bulk ? (uint32_t)(r * pl.cols * (int)sf_pixel_stride) * 2u : 0u) + 127u) & ~127u;
+        return pl.off_buf + 2u * pl.buf_stride;
+    };
+    int rows = pl.OH < kNhwcRows ? pl.OH : kNhwcRows;
+    while (rows > 1 && layout(rows) > kNhwcSmem) --rows;
+    auto tiles = [&](int r) { return (long long)B * pl.tiles_x * ((pl.OH + r - 1) / r); };
+    while (rows > 2 && tiles(rows) < 2ll * sm_count) rows = (rows + 1) / 2;
+    rows = (pl.OH + (pl.OH + rows - 1) / rows - 1) / ((pl.OH + rows - 1) / rows);   // equal heights
+    pl.rows = rows;
+    pl.tiles_y = (pl.OH + rows - 1) / rows;
+    if (tiles(rows) > (1ll << 30)) return DDF_B200_E_UNSUPPORTED;
+    pl.tiles = (int)tiles(rows);
+    const uint32_t smem = layout(rows);
+    if (smem > kNhwcSmem) return DDF_B200_E_UNSUPPORTED;
+    dim3 grid((unsigned)(pl.tiles < 2 * sm_count ? pl.tiles : 2 * sm_count));
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    rc = dtype == DDF_B200_F16 ? nhwc_dispatch<__half>(pl, s, combine, norm, grid, st)
-                               : nhwc_dispatch<__nv_bfloat16>(pl, s, combine, norm, grid, st);
+    rc = dtype == DDF_B200_F16 ? nhwc_dispatch<__half>(pl, s, combine, norm, smem, index, grid, st)
+                               : nhwc_dispatch<__nv_bfloat16>(pl, s, combine, norm, smem, index, grid, st);
     if (rc == 0) g_launches.fetch_add(1, std::memory_order_relaxed);
     return rc;
 }

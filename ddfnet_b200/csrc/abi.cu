@@ -508,11 +508,15 @@ int ddf_b200_backward(const void* go, const void* x, const void* cf, const void*
         const size_t need = bwd_stream_workspace(p, di->sm_count);
         if (need > 0 && (!workspace || workspace_bytes < need)) return DDF_B200_E_WORKSPACE;
     }
-    size_t band = 0, least = 0;
-    const bool band_ok = (gcf || gsf) && allow_stream && variant == DDF_B200_VARIANT_AUTO &&
-                         band_filters_workspace(p, di->sm_count, &band, &least) &&
-                         (least == 0 || (workspace && workspace_bytes >= least && (reinterpret_cast<uintptr_t>(workspace) & 7u) == 0));
-    if (band_ok && band_cols_preferred(p, di->sm_count)) filters_stream = false;
+    // the band form; a caller without scratch for it gets the generic kernels, which need none
+    auto band_has_scratch = [&] {
+        size_t band = 0, least = 0;
+        return band_filters_workspace(p, di->sm_count, &band, &least) &&
+               (least == 0 || (workspace && workspace_bytes >= least && (reinterpret_cast<uintptr_t>(workspace) & 7u) == 0));
+    };
+    const bool cols = filters_stream && variant == DDF_B200_VARIANT_AUTO && band_cols_preferred(p, di->sm_count) &&
+                      band_has_scratch();
+    if (cols) filters_stream = false;
 
     // grad wrt x: the streaming forward kernel run over go with mirrored taps.
     if (gx) {
@@ -564,8 +568,7 @@ int ddf_b200_backward(const void* go, const void* x, const void* cf, const void*
             }
         }
         if (!done && variant == DDF_B200_VARIANT_STREAM) return DDF_B200_E_UNSUPPORTED;
-        // the band form; a caller without scratch for it gets the generic kernels, which need none
-        if (!done && band_ok) {
+        if (!done && allow_stream && (cols || band_has_scratch())) {
             int launches = 0;
             rc = band_filters(p, go, x, cf, sf, gcf, gsf, workspace, workspace_bytes, di->sm_count, di->fault, di->index,
                               st, &launches);

@@ -449,25 +449,28 @@ inline bool band_cols_split(const Problem& p, int sm_count, BandColsSplit& s) {
     // Channels per CTA: the count with the least (waves of CTAs) x (channels a warp walks + the start's worth), and a
     // channel's worth for each set of partials ((8,48,150x130) f16: a start's worth of 12 channels 56.6 us, of 32 43.8).
     const int per_unit = s.planes * kColsCh;
-    long long best_chunk = -1;
     BandColsLayout l;
-    for (int n = 1; n <= kBandBwdParts || best_chunk < 0; ++n) {
-        int chunk = (p.C + n - 1) / n;
-        chunk = (chunk + per_unit - 1) / per_unit * per_unit;
-        if (chunk > kColsChunk && chunk > per_unit) continue;
-        BandColsSplit t = s;
-        t.chunk = chunk;
-        if (!band_cols_layout(p, t, l)) return false;
-        const int chunks = (p.C + chunk - 1) / chunk;
-        const long long slots = (long long)sm_count * l.ctas;
-        const long long waves = ((long long)p.B * s.bands * chunks + slots - 1) / slots;
-        const long long cost = waves * (chunk / s.planes + 32) + chunks;
-        if (best_chunk < 0 || cost < best_chunk) {
-            best_chunk = cost;
-            s.chunk = chunk;
-            s.chunks = chunks;
+    // (a launch's host time is part of a small problem's: the layout of the largest chunk stands for all, and 32-bit
+    // arithmetic does)
+    s.chunk = (p.C < kColsChunk ? p.C + per_unit - 1 : kColsChunk) / per_unit * per_unit;
+    if (s.chunk < per_unit) s.chunk = per_unit;
+    if (!band_cols_layout(p, s, l)) return false;
+    const long long items = (long long)p.B * s.bands;
+    if (items * p.C > (1ll << 30)) return false;
+    const unsigned slots = (unsigned)(sm_count * l.ctas), C = (unsigned)p.C, unit = (unsigned)per_unit;
+    unsigned long long best_cost_chunk = ~0ull;
+    for (unsigned chunk = unit;; chunk += unit) {
+        const unsigned chunks = (C + chunk - 1) / chunk;
+        const bool last = chunk + unit > (unsigned)kColsChunk || chunks == 1;
+        if (chunks > (unsigned)kBandBwdParts && !last) continue;
+        const unsigned waves = ((unsigned)items * chunks + slots - 1) / slots;
+        const unsigned long long cost = (unsigned long long)waves * (chunk / (unsigned)s.planes + 32u) + chunks;
+        if (cost < best_cost_chunk) {
+            best_cost_chunk = cost;
+            s.chunk = (int)chunk;
+            s.chunks = (int)chunks;
         }
-        if (chunk == per_unit) break;
+        if (last) break;
     }
     return (long long)p.B * s.bands * s.chunks <= (1ll << 30);
 }

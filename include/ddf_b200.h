@@ -162,7 +162,7 @@ int ddf_b200_sfnorm_backward(const void* raw, const void* grad_normed, void* gra
  * with norm != 0 the normalised filter is rounded to the element type before use, as the
  * reference's module sequence does when it stores it.
  *
- * ddf_b200_pool_nhwc leaves the float partial sums of x over tiles of 196 pixels,
+ * ddf_b200_pool_nhwc leaves the float partial sums of x over tiles of up to 196 pixels,
  * partials (B, ddf_b200_pool_nhwc_tiles(H,W), C): the global average pool at the head of the
  * channel branch (ddf/ddf.py:186), in the form ddf_b200_channel_filter takes.
  */

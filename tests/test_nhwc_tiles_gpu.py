@@ -28,3 +28,19 @@ def test_matches_oracle(shape, dt, mode):
     sf16[:, :9] = sf
     sf16 = sf16.to(dev).contiguous(memory_format=torch.channels_last)
     check_close(ddf_nhwc(xd, cfd, sf16, 3, 1, s, mode), want, DTYPES[dt], f"channels_last {shape} {dt} {mode}")
+
+
+@pytest.mark.parametrize("hw", [(1, 1), (1, 3), (5, 1), (7, 7), (27, 29), (28, 28), (57, 55)])
+@pytest.mark.parametrize("C", [8, 256, 2048])
+def test_pooled_partials(hw, C):
+    """Tiles of a quarter of the image below 784 pixels, of 196 from there on."""
+    from ddfnet_b200.nhwc import pool_partials
+    x = torch.randn(3, C, *hw, generator=torch.Generator().manual_seed(4)).to(torch.float16)
+    p = pool_partials(x.to("cuda:0").contiguous(memory_format=torch.channels_last))
+    n = hw[0] * hw[1]
+    tile = (n + 3) // 4 if n < 784 else 196
+    assert p.shape == (3, (n + tile - 1) // tile, C)
+    pixels = x.double().flatten(2).split(tile, 2)
+    want = torch.stack([t.sum(2) for t in pixels], 1)
+    # a chain of at most 196 float sums of values below 6: 196 * 2^-24 * 196 * 6 would be the worst case
+    assert torch.allclose(p.cpu().double(), want, rtol=0, atol=1.5e-2 * tile / 196 + 1e-6)

@@ -640,7 +640,7 @@ band_kernel(const __grid_constant__ BandPlan pl) {
                     band_columns<0, T, K, D, S, MUL, MIX>(row, cmask, cf_s + (uint32_t)(ch * CFB), sfr, acc);
                     float res[PH];
                     unpack(acc, res);
-                    if (overflowed(res)) exact(ch, res);
+                    if (left > ch * G && overflowed(res)) exact(ch, res);  // (a missing channel holds anything)
                     if (ch == CH - 1) hand_back();
                     finish(ch, res);
                 }
@@ -659,7 +659,7 @@ band_kernel(const __grid_constant__ BandPlan pl) {
 #pragma unroll
                 for (int ch = 0; ch < CH; ++ch) {
                     unpack(acc[ch], res[ch]);
-                    if (overflowed(res[ch])) exact(ch, res[ch]);
+                    if (left > ch * G && overflowed(res[ch])) exact(ch, res[ch]);
                 }
                 hand_back();
 #pragma unroll

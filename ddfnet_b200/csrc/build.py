@@ -31,7 +31,7 @@ def _nvcc() -> str:
 
 def _deps() -> list[str]:
     return sorted(os.path.join(HERE, f) for f in os.listdir(HERE)
-                  if f.endswith((".cu", ".cuh", ".inc"))) + [
+                  if f.endswith((".cu", ".cuh", ".inc", ".h"))) + [
         os.path.join(os.path.dirname(PKG), "include", "ddf_b200.h")]
 
 

@@ -23,33 +23,13 @@
 #include <atomic>
 
 #include "common.cuh"
+#include "nhwc_plan.h"
 #include "ring_fwd.cuh"
 
 namespace ddf {
 
 extern std::atomic<unsigned long long> g_launches;
 int device_facts(int* sm_count, int** fault, int* index);
-
-struct NhwcPlan {
-    const void* x;          // (B, H, W, C)
-    const void* cf;         // (B, C, K, K)
-    const void* sf;         // K*K values per output pixel, addressed by the two strides below
-    const float* sf_bias;   // K*K values added to the raw filter, or null
-    void* out;              // (B, OH, OW, C)
-    const float* oscale;    // per-channel output scale / shift, or null
-    const float* oshift;
-    int B, C, H, W, OH, OW;
-    long long sf_batch_stride, sf_pixel_stride, sf_tap_stride;   // in elements
-    int relu;
-    float sf_scale;
-    int vecs;               // C / 8
-    int cols, rows;         // output columns and rows of a tile
-    int tiles_x, tiles_y;   // tiles of an image
-    int tiles;              // of all images
-    int sf_bulk;            // a pixel's K*K values are contiguous, 16-byte aligned, and so are a row's pixels: bulk copies
-    uint32_t off_sf, sf_stride, off_affine, off_buf, buf_stride, off_raw, row_bytes;  // off_raw: inside a buffer
-    int* fault;
-};
 
 __device__ __forceinline__ uint4 ldg128(const void* p) {
     uint4 v;
@@ -147,21 +127,19 @@ __global__ void __launch_bounds__(kNhwcThreads, 2) nhwc_forward_kernel(const __g
         const int cy0 = iy0 > 0 ? iy0 : 0, cy1 = (iy0 + (r.ny - 1) * S + K) < H ? (iy0 + (r.ny - 1) * S + K) : H;
         const int n = cy1 - cy0;
         const uint32_t bytes = (uint32_t)(cx1 - cx0) * (uint32_t)C * 2u;
+        // the filters of the tile's rows: as many bytes each, but for the last one of an image
         const uint32_t sfb = pl.sf_bulk ? (uint32_t)(r.nx * (int)pl.sf_pixel_stride) * 2u : 0u;
-        // behind the tensor's last pixel there may be nothing to read: 8 of its values by the copy, the ninth apart
-        const bool last = pl.sf_bulk && r.b == pl.B - 1 && r.oy0 + r.ny == OH && r.ox0 + r.nx == OW;
-        const uint32_t less = last ? (uint32_t)pl.sf_pixel_stride * 2u - 16u : 0u;
-        if (tid == 0) mbar_arrive_expect_tx(NH_FULL(buf), (uint32_t)n * bytes + (uint32_t)r.ny * sfb - less);
+        const uint32_t sfb_last = pl.sf_bulk ? nhwc_filter_run(pl, r.b, r.oy0 + r.ny - 1, r.ox0, r.nx).bytes : 0u;
+        if (tid == 0) mbar_arrive_expect_tx(NH_FULL(buf), (uint32_t)n * bytes + (uint32_t)(r.ny - 1) * sfb + sfb_last);
         __syncwarp();
         if (tid < n) {
             bulk_g2s(NH_BUF(buf) + (uint32_t)(cy0 - iy0 + tid) * pl.row_bytes + (uint32_t)((cx0 - ix0) * C * 2),
                      reinterpret_cast<const T*>(pl.x) + (((size_t)r.b * H + cy0 + tid) * W + cx0) * C, bytes, NH_FULL(buf));
         } else if (pl.sf_bulk && tid < n + r.ny) {
             const int y = tid - n;
+            const NhwcRun run = nhwc_filter_run(pl, r.b, r.oy0 + y, r.ox0, r.nx);
             bulk_g2s(NH_BUF(buf) + pl.off_raw + (uint32_t)(y * pl.cols * (int)pl.sf_pixel_stride) * 2u,
-                     reinterpret_cast<const T*>(pl.sf) + r.b * pl.sf_batch_stride +
-                         ((long long)(r.oy0 + y) * OW + r.ox0) * pl.sf_pixel_stride,
-                     y == r.ny - 1 ? sfb - less : sfb, NH_FULL(buf));
+                     reinterpret_cast<const T*>(pl.sf) + run.from, run.bytes, NH_FULL(buf));
         }
     };
     static_assert((kNhwcRows - 1) * S + K + kNhwcRows <= 32, "a lane per row of a tile and of its filters");
@@ -236,7 +214,7 @@ __global__ void __launch_bounds__(kNhwcThreads, 2) nhwc_forward_kernel(const __g
                 const uint32_t from = NH_BUF(buf) + pl.off_raw + (uint32_t)((py * pl.cols + px) * (int)pl.sf_pixel_stride) * 2u;
                 uint32_t raw[5];
                 lds128(from, raw[0], raw[1], raw[2], raw[3]);
-                if (r.b == pl.B - 1 && r.oy0 + py == OH - 1 && r.ox0 + px == OW - 1)
+                if (nhwc_last_pixel(pl, r.oy0 + py, r.ox0 + px))
                     raw[4] = __ldg(reinterpret_cast<const uint16_t*>(pl.sf) + r.b * pl.sf_batch_stride +
                                    ((long long)OH * OW - 1) * pl.sf_pixel_stride + 8);
                 else raw[4] = lds16(from + 16u);

@@ -44,3 +44,25 @@ def test_pooled_partials(hw, C):
     want = torch.stack([t.sum(2) for t in pixels], 1)
     # a chain of at most 196 float sums of values below 6: 196 * 2^-24 * 196 * 6 would be the worst case
     assert torch.allclose(p.cpu().double(), want, rtol=0, atol=1.5e-2 * tile / 196 + 1e-6)
+
+
+@pytest.mark.parametrize("mode", ["mul", "add"])
+def test_one_filter_map_for_all_samples(mode):
+    """sf_batch_stride 0: what lies behind the map's last value belongs to no sample and must not matter."""
+    from ddfnet_b200 import _lib
+    B, C, H, W, g = 3, 64, 9, 20, 24
+    x, cf, sf = make_inputs(1, C, H, W, 3, 1, torch.float16, seed=77, with_go=False)
+    x, cf = (torch.cat([t * (i + 1) for i in range(B)]) for t in (x, cf))
+    dev = torch.device("cuda:0")
+    xd = x.to(dev).contiguous(memory_format=torch.channels_last)
+    maps = torch.full((H, W, g), float("nan"), dtype=torch.float16)
+    maps[..., :9] = sf[0].permute(1, 2, 0)
+    buf = torch.full((H * W * g + 512,), float("nan"), dtype=torch.float16)
+    buf[: (H * W - 1) * g + 9] = maps.flatten()[: (H * W - 1) * g + 9]
+    buf, cfd = buf.to(dev), cf.to(dev)
+    out = torch.empty_like(xd)
+    rc = _lib.load().ddf_b200_forward_nhwc(xd.data_ptr(), cfd.data_ptr(), buf.data_ptr(), None, out.data_ptr(), None, None, 0, B,
+                                           C, H, W, 3, 1, 1, {"mul": 0, "add": 1}[mode], 1, 0, g, 1, 0, 1.0,
+                                           torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    check_close(out, oracle_forward(x, cf, sf.expand(B, -1, -1, -1), 3, 1, 1, mode), torch.float16, f"shared filter {mode}")

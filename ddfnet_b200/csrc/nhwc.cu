@@ -56,9 +56,6 @@ template <> __device__ __forceinline__ uint32_t relu2<__nv_bfloat16>(uint32_t v)
     return r;
 }
 
-constexpr int kNhwcThreads = 256;
-constexpr int kNhwcRows = 8;   // output rows of a tile at most
-
 // Bytes of a pixel's filter in shared memory: mul (s, s) float pairs, add packed 2-byte values; whole 16s.
 template <int MODE> constexpr uint32_t kNhwcPixel = MODE == DDF_B200_MUL ? 80 : 32;
 
@@ -392,9 +389,6 @@ __global__ void __launch_bounds__(256) nhwc_pool_kernel(const T* __restrict__ x,
     }
 }
 
-// Most dynamic shared memory of the forward kernel: two CTAs per SM.
-constexpr uint32_t kNhwcSmem = 112 * 1024;
-
 template <typename T, int S, int MODE>
 static int nhwc_launch(const NhwcPlan& pl, int norm, uint32_t smem, int device, dim3 grid, cudaStream_t st) {
     auto kern = norm ? nhwc_forward_kernel<T, S, MODE, true> : nhwc_forward_kernel<T, S, MODE, false>;
@@ -478,37 +472,11 @@ int ddf_b200_forward_nhwc(const void* x, const void* cf, const void* sf, const f
     pl.relu = relu; pl.sf_scale = (float)sf_scale;
     pl.vecs = C / 8;
     pl.fault = fault;
-    // Tiles: equal column counts, as many as the threads cover; rows as two buffers of two CTAs leave room for (the
-    // two halo rows are then a quarter of the copies at most), fewer where the chip would not be full.
-    const int most = kNhwcThreads / pl.vecs;
-    pl.tiles_x = (pl.OW + most - 1) / most;
-    pl.cols = (pl.OW + pl.tiles_x - 1) / pl.tiles_x;
-    pl.tiles_x = (pl.OW + pl.cols - 1) / pl.cols;
-    const uint32_t pixel = combine == DDF_B200_MUL ? kNhwcPixel<DDF_B200_MUL> : kNhwcPixel<DDF_B200_ADD>;
     // bulk copies of the raw filters: taps contiguous, whole 16 bytes a pixel, pixels of a row one after the other
     pl.sf_bulk = (sf_tap_stride == 1 && sf_pixel_stride % 8 == 0 && sf_pixel_stride >= 16 && sf_pixel_stride <= 64 &&
                   sf_batch_stride % 8 == 0 && al16(sf)) ? 1 : 0;
-    pl.row_bytes = (uint32_t)(((pl.cols - 1) * s + 3) * C * 2);
-    auto layout = [&](int r) {
-        pl.off_sf = 64;
-        pl.sf_stride = (uint32_t)pl.cols * ((uint32_t)r * pixel + 16u);
-        pl.off_affine = pl.off_sf + 2u * pl.sf_stride;
-        pl.off_buf = (pl.off_affine + 8u * (uint32_t)C + 127u) & ~127u;
-        pl.off_raw = (uint32_t)((r - 1) * s + 3) * pl.row_bytes;
-        pl.buf_stride = (pl.off_raw + (pl.sf_bulk ? (uint32_t)(r * pl.cols * (int)sf_pixel_stride) * 2u : 0u) + 127u) & ~127u;
-        return pl.off_buf + 2u * pl.buf_stride;
-    };
-    int rows = pl.OH < kNhwcRows ? pl.OH : kNhwcRows;
-    while (rows > 1 && layout(rows) > kNhwcSmem) --rows;
-    auto tiles = [&](int r) { return (long long)B * pl.tiles_x * ((pl.OH + r - 1) / r); };
-    while (rows > 2 && tiles(rows) < 2ll * sm_count) rows = (rows + 1) / 2;
-    rows = (pl.OH + (pl.OH + rows - 1) / rows - 1) / ((pl.OH + rows - 1) / rows);   // equal heights
-    pl.rows = rows;
-    pl.tiles_y = (pl.OH + rows - 1) / rows;
-    if (tiles(rows) > (1ll << 30)) return DDF_B200_E_UNSUPPORTED;
-    pl.tiles = (int)tiles(rows);
-    const uint32_t smem = layout(rows);
-    if (smem > kNhwcSmem) return DDF_B200_E_UNSUPPORTED;
+    const uint32_t smem = nhwc_tiles(pl, s, combine == DDF_B200_MUL ? kNhwcPixel<DDF_B200_MUL> : kNhwcPixel<DDF_B200_ADD>, sm_count);
+    if (smem == 0) return DDF_B200_E_UNSUPPORTED;
     dim3 grid((unsigned)(pl.tiles < 2 * sm_count ? pl.tiles : 2 * sm_count));
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     rc = dtype == DDF_B200_F16 ? nhwc_dispatch<__half>(pl, s, combine, norm, smem, index, grid, st)

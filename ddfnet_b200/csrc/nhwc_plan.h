@@ -12,6 +12,10 @@
 
 namespace ddf {
 
+constexpr int kNhwcThreads = 256;
+constexpr int kNhwcRows = 8;                 // output rows of a tile at most
+constexpr uint32_t kNhwcSmem = 112 * 1024;   // shared memory of a CTA at most: two per SM
+
 struct NhwcPlan {
     const void* x;          // (B, H, W, C)
     const void* cf;         // (B, C, K, K)
@@ -45,6 +49,41 @@ NHWC_HD NhwcRun nhwc_filter_run(const NhwcPlan& pl, int b, int oy, int ox0, int 
     const uint32_t pixel = (uint32_t)pl.sf_pixel_stride * 2u;
     return {b * pl.sf_batch_stride + ((long long)oy * pl.OW + ox0) * pl.sf_pixel_stride,
             (uint32_t)nx * pixel - (nhwc_last_pixel(pl, oy, ox0 + nx - 1) ? pixel - 16u : 0u)};
+}
+
+// Tiles and shared-memory layout of a problem; `pixel`: bytes of a pixel's filter in shared memory.  Returns the bytes of
+// shared memory, 0 where there would be too many tiles.
+// Equal column counts, as many as the threads cover; rows as two buffers of two CTAs leave room for (the two halo rows are
+// then a quarter of the copies at most), fewer where the chip would not be full.  More tiles across where one row of that
+// many columns does not fit: C = 8 alone, whose 256 columns with 16-map filters at stride 2 take 115 072 bytes.
+inline uint32_t nhwc_tiles(NhwcPlan& pl, int s, uint32_t pixel, int sm_count) {
+    const int most = kNhwcThreads / pl.vecs;
+    auto layout = [&](int r) {
+        pl.row_bytes = (uint32_t)(((pl.cols - 1) * s + 3) * pl.C * 2);
+        pl.off_sf = 64;
+        pl.sf_stride = (uint32_t)pl.cols * ((uint32_t)r * pixel + 16u);
+        pl.off_affine = pl.off_sf + 2u * pl.sf_stride;
+        pl.off_buf = (pl.off_affine + 8u * (uint32_t)pl.C + 127u) & ~127u;
+        pl.off_raw = (uint32_t)((r - 1) * s + 3) * pl.row_bytes;
+        pl.buf_stride = (pl.off_raw + (pl.sf_bulk ? (uint32_t)(r * pl.cols * (int)pl.sf_pixel_stride) * 2u : 0u) + 127u) & ~127u;
+        return pl.off_buf + 2u * pl.buf_stride;
+    };
+    for (int across = (pl.OW + most - 1) / most;; ++across) {
+        pl.cols = (pl.OW + across - 1) / across;
+        if (pl.cols == 1 || layout(1) <= kNhwcSmem) break;
+    }
+    pl.tiles_x = (pl.OW + pl.cols - 1) / pl.cols;
+    int rows = pl.OH < kNhwcRows ? pl.OH : kNhwcRows;
+    while (rows > 1 && layout(rows) > kNhwcSmem) --rows;
+    auto tiles = [&](int r) { return (long long)pl.B * pl.tiles_x * ((pl.OH + r - 1) / r); };
+    while (rows > 2 && tiles(rows) < 2ll * sm_count) rows = (rows + 1) / 2;
+    rows = (pl.OH + (pl.OH + rows - 1) / rows - 1) / ((pl.OH + rows - 1) / rows);   // equal heights
+    pl.rows = rows;
+    pl.tiles_y = (pl.OH + rows - 1) / rows;
+    if (tiles(rows) > (1ll << 30)) return 0;
+    pl.tiles = (int)tiles(rows);
+    const uint32_t smem = layout(rows);
+    return smem <= kNhwcSmem ? smem : 0;
 }
 
 }  // namespace ddf

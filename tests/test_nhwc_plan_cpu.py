@@ -1,5 +1,5 @@
 """Host arithmetic of the channels_last forward (nhwc_plan.h), compiled with the host compiler: where the bulk copies of
-the raw filters end."""
+the raw filters end, and which problems have tiles."""
 import os
 import subprocess
 
@@ -31,13 +31,68 @@ int main(int, char** v) {
 """
 
 
+TILES = r"""
+#include <initializer_list>
+#include <cstdio>
+#include <cstdlib>
+#include "nhwc_plan.h"
+using namespace ddf;
+// argv: C stride -> the problems of every width up to 600 without tiles, or whose layout is unsound
+int main(int, char** v) {
+    int bad = 0, n = 0;
+    for (int s = atoi(v[2]), ow = 1; ow <= 600; ++ow)
+        for (int oh : {1, 2, 5, 8, 56})
+            for (int pixel : {32, 80})
+                for (int bulk = 0; bulk <= 64; bulk += bulk ? 8 : 16) {
+                    NhwcPlan pl = {};
+                    pl.B = 3; pl.C = atoi(v[1]); pl.vecs = pl.C / 8;
+                    pl.OH = oh; pl.OW = ow; pl.H = oh * s; pl.W = ow * s;
+                    pl.sf_bulk = bulk > 0; pl.sf_pixel_stride = bulk;
+                    const uint32_t smem = nhwc_tiles(pl, s, (uint32_t)pixel, 148);
+                    const int cols = (pl.cols - 1) * s + 3, rows = (pl.rows - 1) * s + 3;   // of a tile's window
+                    ++n;
+                    bad += !(smem > 0 && smem <= kNhwcSmem && pl.cols >= 1 && pl.cols * pl.vecs <= kNhwcThreads &&
+                             pl.rows >= 1 && pl.rows <= kNhwcRows && pl.tiles == 3 * pl.tiles_x * pl.tiles_y &&
+                             pl.cols * pl.tiles_x >= ow && pl.cols * (pl.tiles_x - 1) < ow &&
+                             pl.rows * pl.tiles_y >= oh && pl.rows * (pl.tiles_y - 1) < oh &&
+                             pl.row_bytes >= (uint32_t)(cols * pl.C * 2) && pl.off_raw >= (uint32_t)rows * pl.row_bytes &&
+                             pl.sf_stride >= (uint32_t)(pl.cols * (pl.rows * pixel + 16)) && pl.off_affine >= 64 + 2 * pl.sf_stride &&
+                             pl.off_buf >= pl.off_affine + 8u * pl.C &&
+                             pl.buf_stride >= pl.off_raw + (uint32_t)(pl.rows * pl.cols * bulk) * 2u &&
+                             smem >= pl.off_buf + 2u * pl.buf_stride && pl.off_buf % 128 == 0 && pl.buf_stride % 128 == 0);
+                }
+    printf("%d %d\n", bad, n);
+}
+"""
+
+
 @pytest.fixture(scope="module")
-def program(tmp_path_factory):
-    d = tmp_path_factory.mktemp("nhwc_plan")
-    (d / "main.cpp").write_text(PROGRAM)
-    subprocess.run(["g++", "-std=c++17", "-Wall", "-Werror", f"-I{CSRC}", str(d / "main.cpp"), "-o", str(d / "main")], check=True)
-    return lambda *args: [int(n) for n in subprocess.run([str(d / "main"), *map(str, args)], check=True, capture_output=True,
-                                                         text=True).stdout.split()]
+def compiled(tmp_path_factory):
+    def build(text):
+        d = tmp_path_factory.mktemp("nhwc_plan")
+        (d / "main.cpp").write_text(text)
+        subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Wno-sign-compare", "-Werror", f"-I{CSRC}", str(d / "main.cpp"), "-o", str(d / "main")],
+                       check=True)
+        return lambda *args: [int(n) for n in subprocess.run([str(d / "main"), *map(str, args)], check=True, capture_output=True,
+                                                             text=True).stdout.split()]
+    return build
+
+
+@pytest.fixture(scope="module")
+def program(compiled):
+    return compiled(PROGRAM)
+
+
+@pytest.fixture(scope="module")
+def tiles(compiled):
+    return compiled(TILES)
+
+
+@pytest.mark.parametrize("stride", [1, 2])
+@pytest.mark.parametrize("C", [8 << i for i in range(9)])
+def test_every_width_has_tiles_that_fit(tiles, C, stride):
+    bad, n = tiles(C, stride)
+    assert bad == 0 and n == 600 * 5 * 2 * 8
 
 
 @pytest.mark.parametrize("oh,ow,cols", [(1, 1, 1), (5, 7, 7), (3, 9, 4), (4, 8, 3)])

@@ -66,3 +66,18 @@ def test_one_filter_map_for_all_samples(mode):
                                            torch.cuda.current_stream().cuda_stream)
     assert rc == 0
     check_close(out, oracle_forward(x, cf, sf.expand(B, -1, -1, -1), 3, 1, 1, mode), torch.float16, f"shared filter {mode}")
+
+
+# B, H, W, stride, maps of the spatial filter: widths at which a row of 256 columns does not fit a CTA's shared memory
+@pytest.mark.parametrize("shape", [(1, 6, 512, 2, 16), (3, 9, 1022, 2, 16), (2, 5, 480, 2, 32), (1, 3, 256, 1, 48), (1, 4, 333, 1, 64)])
+@pytest.mark.parametrize("mode", ["mul", "add"])
+def test_wide_rows_of_eight_channels(shape, mode):
+    from ddfnet_b200.nhwc import ddf_nhwc
+    B, H, W, s, g = shape
+    x, cf, sf = make_inputs(B, 8, H, W, 3, s, torch.float16, seed=sum(shape), with_go=False)
+    dev = torch.device("cuda:0")
+    maps = torch.full((B, g, H // s, W // s), float("nan"), dtype=torch.float16)
+    maps[:, :9] = sf
+    out = ddf_nhwc(x.to(dev).contiguous(memory_format=torch.channels_last), cf.to(dev),
+                   maps.to(dev).contiguous(memory_format=torch.channels_last), 3, 1, s, mode)
+    check_close(out, oracle_forward(x, cf, sf, 3, 1, s, mode), torch.float16, f"{shape} {mode}")

@@ -26,7 +26,7 @@ SYMBOLS = (
     "ddf_b200_forward_sfnorm", "ddf_b200_nhwc_to_nchw", "ddf_b200_nchw_to_nhwc", "ddf_b200_nhwc_to_nchw_affine",
     "ddf_b200_channel_filter", "ddf_b200_channel_filter_slice",
     "ddf_b200_frontend_tiles", "ddf_b200_pack_frontend", "ddf_b200_forward_waitlimit", "ddf_b200_band_waitlimit",
-    "ddf_b200_forward_nhwc", "ddf_b200_pool_nhwc_tiles", "ddf_b200_pool_nhwc",
+    "ddf_b200_forward_nhwc", "ddf_b200_nhwc_waitlimit", "ddf_b200_pool_nhwc_tiles", "ddf_b200_pool_nhwc",
     "ddf_b200_sfnorm", "ddf_b200_sfnorm_backward", "ddf_b200_maxpool_nhwc",
     "ddf_b200_noop", "ddf_b200_rate_probe_bytes", "ddf_b200_rate_probe",
 )
@@ -62,6 +62,8 @@ def load() -> ctypes.CDLL:
         L.ddf_b200_band_waitlimit.argtypes = [vp] * 8 + [sz] + [i] * 9 + [ll, i, vp]
         L.ddf_b200_forward_nhwc.restype = i
         L.ddf_b200_forward_nhwc.argtypes = [vp] * 7 + [i] * 10 + [ll, ll, ll, i, ctypes.c_double, vp]
+        L.ddf_b200_nhwc_waitlimit.restype = i
+        L.ddf_b200_nhwc_waitlimit.argtypes = [vp] * 4 + [i] * 9 + [ll, ll, ll, ll, i, vp]
         L.ddf_b200_pool_nhwc_tiles.restype = i
         L.ddf_b200_pool_nhwc_tiles.argtypes = [i, i]
         L.ddf_b200_pool_nhwc.restype = i

@@ -118,7 +118,8 @@ __global__ void __launch_bounds__(kNhwcThreads, 2) nhwc_forward_kernel(const __g
     }
     // the first warp: the tile's input rows and its raw filters into a buffer, a row per lane.  Window column 0 of the
     // tile lies at a row's start, window row 0 at the buffer's.
-    auto request = [&](const Tile& r, int buf) {
+    auto request = [&](const Tile& r, int t) {
+        const int buf = (t - t_lo) & 1;
         const int ix0 = r.ox0 * S - 1, iy0 = r.oy0 * S - 1;
         const int cx0 = ix0 > 0 ? ix0 : 0, cx1 = (ix0 + (r.nx - 1) * S + K) < W ? (ix0 + (r.nx - 1) * S + K) : W;
         const int cy0 = iy0 > 0 ? iy0 : 0, cy1 = (iy0 + (r.ny - 1) * S + K) < H ? (iy0 + (r.ny - 1) * S + K) : H;
@@ -127,7 +128,9 @@ __global__ void __launch_bounds__(kNhwcThreads, 2) nhwc_forward_kernel(const __g
         // the filters of the tile's rows: as many bytes each, but for the last one of an image
         const uint32_t sfb = pl.sf_bulk ? (uint32_t)(r.nx * (int)pl.sf_pixel_stride) * 2u : 0u;
         const uint32_t sfb_last = pl.sf_bulk ? nhwc_filter_run(pl, r.b, r.oy0 + r.ny - 1, r.ox0, r.nx).bytes : 0u;
-        if (tid == 0) mbar_arrive_expect_tx(NH_FULL(buf), (uint32_t)n * bytes + (uint32_t)(r.ny - 1) * sfb + sfb_last);
+        if (tid == 0)
+            mbar_arrive_expect_tx(NH_FULL(buf), (uint32_t)n * bytes + (uint32_t)(r.ny - 1) * sfb + sfb_last +
+                                                    (t - t_lo + 1 == pl.starve ? 16u : 0u));
         __syncwarp();
         if (tid < n) {
             bulk_g2s(NH_BUF(buf) + (uint32_t)(cy0 - iy0 + tid) * pl.row_bytes + (uint32_t)((cx0 - ix0) * C * 2),
@@ -141,8 +144,8 @@ __global__ void __launch_bounds__(kNhwcThreads, 2) nhwc_forward_kernel(const __g
     };
     static_assert((kNhwcRows - 1) * S + K + kNhwcRows <= 32, "a lane per row of a tile and of its filters");
     if (tid < 32) {
-        if (t_lo < t_hi) request(r, 0);
-        if (t_lo + 1 < t_hi) request(next_of(r), 1);
+        if (t_lo < t_hi) request(r, t_lo);
+        if (t_lo + 1 < t_hi) request(next_of(r), t_lo + 1);
     }
 
     // a thread's constants of the row loop, kept (see pin)
@@ -178,12 +181,8 @@ __global__ void __launch_bounds__(kNhwcThreads, 2) nhwc_forward_kernel(const __g
                 }
             }
         }
-        if (!mbar_wait(NH_FULL(buf), (uint32_t)(((t - t_lo) >> 1) & 1))) {
-            atomicCAS(pl.fault, 0, (int)kFaultConsumerFull);
-            // the copies requested so far land before the block's memory goes
-            mbar_wait(NH_FULL(buf ^ 1), (uint32_t)(((t + 1 - t_lo) >> 1) & 1));
-            return;
-        }
+        const bool late = !mbar_wait_for(NH_FULL(buf), (uint32_t)(((t - t_lo) >> 1) & 1), pl.wait_cycles);
+        if (late) atomicCAS(pl.fault, 0, (int)kFaultConsumerFull);
         // Window columns and rows outside the image: zeros, where the copies left something else.
         {
             const int ix0 = r.ox0 * S - 1, iy0 = r.oy0 * S - 1, cols = (r.nx - 1) * S + K, rows = (r.ny - 1) * S + K;
@@ -252,10 +251,20 @@ __global__ void __launch_bounds__(kNhwcThreads, 2) nhwc_forward_kernel(const __g
                 sts32(at + 16u, pack2<T>(sv[8], 0.f));
             }
         }
-        __syncthreads();
+        if (__syncthreads_or(late)) {
+            // All threads leave together and store no more.  The copies under way -- this tile's, and behind the first
+            // one the next tile's too -- land before the block's memory goes.
+            if (tid == 0) {
+                bool landed = mbar_wait_for(NH_FULL(buf), (uint32_t)(((t - t_lo) >> 1) & 1), pl.wait_cycles);
+                if (t == t_lo && t + 1 < t_hi) landed &= mbar_wait_for(NH_FULL(buf ^ 1), 0u, pl.wait_cycles);
+                if (!landed && pl.starve == 0) atomicExch(pl.fault, (int)kFaultDrain);
+            }
+            __syncthreads();
+            return;
+        }
         // every thread is done with the tile before: its buffer takes the next one
         const Tile next = next_of(r);
-        if (tid < 32 && t > t_lo && t + 1 < t_hi) request(next, buf ^ 1);
+        if (tid < 32 && t > t_lo && t + 1 < t_hi) request(next, t + 1);
 
         if (active) {
             const int ox = r.ox0 + col;
@@ -442,11 +451,11 @@ int ddf_b200_pool_nhwc(const void* x, float* partials, int B, int C, int H, int 
     return (int)cudaGetLastError();
 }
 
-int ddf_b200_forward_nhwc(const void* x, const void* cf, const void* sf, const float* sf_bias, void* out,
-                          const float* out_scale, const float* out_shift, int relu, int B, int C, int H, int W,
-                          int k, int d, int s, int combine, int dtype, long long sf_batch_stride,
-                          long long sf_pixel_stride, long long sf_tap_stride, int norm, double sf_scale,
-                          void* stream) {
+static int nhwc_forward(const void* x, const void* cf, const void* sf, const float* sf_bias, void* out,
+                        const float* out_scale, const float* out_shift, int relu, int B, int C, int H, int W,
+                        int k, int d, int s, int combine, int dtype, long long sf_batch_stride,
+                        long long sf_pixel_stride, long long sf_tap_stride, int norm, double sf_scale,
+                        long long wait_cycles, int starve, void* stream) {
     if (!x || !cf || !sf || !out) return DDF_B200_E_NULL;
     if ((out_scale == nullptr) != (out_shift == nullptr)) return DDF_B200_E_NULL;
     if (B < 1 || C < 1 || H < 1 || W < 1 || s < 1 || H / s < 1 || W / s < 1) return DDF_B200_E_SHAPE;
@@ -471,7 +480,7 @@ int ddf_b200_forward_nhwc(const void* x, const void* cf, const void* sf, const f
     pl.sf_batch_stride = sf_batch_stride; pl.sf_pixel_stride = sf_pixel_stride; pl.sf_tap_stride = sf_tap_stride;
     pl.relu = relu; pl.sf_scale = (float)sf_scale;
     pl.vecs = C / 8;
-    pl.fault = fault;
+    pl.fault = fault; pl.wait_cycles = wait_cycles; pl.starve = starve;
     // bulk copies of the raw filters: taps contiguous, whole 16 bytes a pixel, pixels of a row one after the other
     pl.sf_bulk = (sf_tap_stride == 1 && sf_pixel_stride % 8 == 0 && sf_pixel_stride >= 16 && sf_pixel_stride <= 64 &&
                   sf_batch_stride % 8 == 0 && al16(sf)) ? 1 : 0;
@@ -483,6 +492,23 @@ int ddf_b200_forward_nhwc(const void* x, const void* cf, const void* sf, const f
                                : nhwc_dispatch<__nv_bfloat16>(pl, s, combine, norm, smem, index, grid, st);
     if (rc == 0) g_launches.fetch_add(1, std::memory_order_relaxed);
     return rc;
+}
+
+int ddf_b200_forward_nhwc(const void* x, const void* cf, const void* sf, const float* sf_bias, void* out,
+                          const float* out_scale, const float* out_shift, int relu, int B, int C, int H, int W,
+                          int k, int d, int s, int combine, int dtype, long long sf_batch_stride,
+                          long long sf_pixel_stride, long long sf_tap_stride, int norm, double sf_scale,
+                          void* stream) {
+    return nhwc_forward(x, cf, sf, sf_bias, out, out_scale, out_shift, relu, B, C, H, W, k, d, s, combine, dtype,
+                        sf_batch_stride, sf_pixel_stride, sf_tap_stride, norm, sf_scale, kWaitCycles, 0, stream);
+}
+
+int ddf_b200_nhwc_waitlimit(const void* x, const void* cf, const void* sf, void* out, int B, int C, int H, int W, int k,
+                            int d, int s, int combine, int dtype, long long sf_batch_stride, long long sf_pixel_stride,
+                            long long sf_tap_stride, long long wait_cycles, int starve, void* stream) {
+    if (wait_cycles < 1 || starve < 0) return DDF_B200_E_SHAPE;
+    return nhwc_forward(x, cf, sf, nullptr, out, nullptr, nullptr, 0, B, C, H, W, k, d, s, combine, dtype, sf_batch_stride,
+                        sf_pixel_stride, sf_tap_stride, 0, 1.0, wait_cycles, starve, stream);
 }
 
 }  // extern "C"

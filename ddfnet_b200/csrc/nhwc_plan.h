@@ -35,6 +35,8 @@ struct NhwcPlan {
     int sf_bulk;            // a pixel's K*K values are contiguous, 16-byte aligned, and so are a row's pixels: bulk copies
     uint32_t off_sf, sf_stride, off_affine, off_buf, buf_stride, off_raw, row_bytes;  // off_raw: inside a buffer
     int* fault;
+    long long wait_cycles;  // limit of every mbarrier wait, in SM clocks
+    int starve;             // self-test: this tile of every CTA (1: the first) is announced 16 bytes too large and never completes
 };
 
 // A row of a tile's raw filters, as one bulk copy (sf_bulk): `nx` pixels from column ox0 of row oy of sample b.  Behind

@@ -171,6 +171,12 @@ int ddf_b200_forward_nhwc(const void* x, const void* cf, const void* sf, const f
                           int B, int C, int H, int W, int k, int d, int s, int combine, int dtype,
                           long long sf_batch_stride, long long sf_pixel_stride,
                           long long sf_tap_stride, int norm, double sf_scale, void* stream);
+/* Self-test of its bounded waits, as ddf_b200_band_waitlimit: with `starve` = n > 0 the n-th tile of every
+ * CTA never completes.  The CTAs record fault 1 and leave, the tiles before it written, all others not. */
+int ddf_b200_nhwc_waitlimit(const void* x, const void* cf, const void* sf, void* out, int B, int C, int H, int W,
+                            int k, int d, int s, int combine, int dtype, long long sf_batch_stride,
+                            long long sf_pixel_stride, long long sf_tap_stride, long long wait_cycles, int starve,
+                            void* stream);
 int ddf_b200_pool_nhwc_tiles(int H, int W);
 int ddf_b200_pool_nhwc(const void* x, float* partials, int B, int C, int H, int W, int dtype,
                        void* stream);

@@ -81,3 +81,37 @@ def test_wide_rows_of_eight_channels(shape, mode):
     out = ddf_nhwc(x.to(dev).contiguous(memory_format=torch.channels_last), cf.to(dev),
                    maps.to(dev).contiguous(memory_format=torch.channels_last), 3, 1, s, mode)
     check_close(out, oracle_forward(x, cf, sf, 3, 1, s, mode), torch.float16, f"{shape} {mode}")
+
+
+@pytest.mark.parametrize("starve", [1, 2, 3])
+def test_a_wait_that_runs_out(starve):
+    """The CTAs leave together: tiles before the one that never completes are whole, no other element is written, and
+    the context stays usable."""
+    from ddfnet_b200 import _lib
+    L = _lib.load()
+    B, C, H, W, g = 64, 256, 56, 56, 16   # 56 rows in tiles of at most 8 by 8: more than three a CTA
+    x, cf, sf = make_inputs(2, C, H, W, 3, 1, torch.float16, seed=78, with_go=False)
+    dev = torch.device("cuda:0")
+    xd = x.to(dev).repeat(B // 2, 1, 1, 1).contiguous(memory_format=torch.channels_last)
+    cfd = cf.to(dev).repeat(B // 2, 1, 1, 1)
+    maps = torch.zeros(B, H, W, g, dtype=torch.float16, device=dev)
+    maps[..., :9] = sf.to(dev).permute(0, 2, 3, 1).repeat(B // 2, 1, 1, 1)
+    out = torch.full_like(xd, float("nan"))
+
+    def call(limit, starve):
+        return L.ddf_b200_nhwc_waitlimit(xd.data_ptr(), cfd.data_ptr(), maps.data_ptr(), out.data_ptr(), B, C, H, W, 3, 1, 1,
+                                         _lib.MUL, 1, H * W * g, g, 1, limit, starve, torch.cuda.current_stream().cuda_stream)
+
+    assert L.ddf_b200_take_fault() == 0
+    assert call(2_000_000, starve) == 0
+    assert L.ddf_b200_take_fault() == 1
+    assert L.ddf_b200_take_fault() == 0
+    left = out.clone()
+    assert call(2_000_000_000, 0) == 0
+    assert L.ddf_b200_take_fault() == 0
+    check_close(out[:2], oracle_forward(x, cf, sf, 3, 1, 1, "mul"), torch.float16, "after a starved launch")
+    written = ~left.isnan()
+    assert torch.equal(left[written], out[written])
+    assert torch.equal(written, written[:, :1].expand_as(written))   # whole pixels
+    share = written.float().mean().item()
+    assert (share == 0) if starve == 1 else 0 < share < 1

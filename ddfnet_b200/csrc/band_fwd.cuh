@@ -35,7 +35,8 @@
 // NaN where the definition skips the tap: while the filters hold anything not below kBandFilterMax
 // in magnitude (so that cf * sf is finite too) a CTA takes a plain loop that skips those taps.  A thread takes it too
 // where x * sf may have left float's range although x * (cf * sf) does not (bfloat16 alone): where a result is not
-// finite.
+// finite, and, while a channel filter holds a value of kLargeCf or more, where one is below kBandSmall (x * sf below
+// 2^-126 is rounded, an error of up to 2^-150 |cf| a tap, which for results below 2^-60 may be more than 2^-24 of them).
 //
 // Every mbarrier wait is bounded by the plan's wait_cycles.  A thread whose wait ran out records a fault,
 // stays for the barriers of the others, and neither stores nor hands slots back: the producer's own wait
@@ -54,6 +55,7 @@ namespace ddf {
 constexpr int kBandSlots = 8;
 constexpr int kBandStage = 64;       // channels whose filters are staged together
 constexpr float kBandFilterMax = 1e18f;
+constexpr float kBandSmall = 8.6736173798840355e-19f;   // 2^-60
 constexpr uint32_t kBandGuard = 32;  // readable bytes before a slot's data (left halo of its first row)
 constexpr uint32_t kBandZero = 80;   // zeroed bytes after it
 constexpr uint32_t kBandDead = 2;    // bit of a compute thread's ring phase: one of its waits ran out
@@ -511,6 +513,8 @@ band_kernel(const __grid_constant__ BandPlan pl) {
         // Channel filters of the next units, one column of taps after the other; grad-x pairs window tap (i, j)
         // with the mirrored filter tap.
         int big = big_sf;
+        constexpr bool SMALL = MIX && std::is_same<T, __nv_bfloat16>::value;   // x * sf may lose what cf would bring back
+        int large = 0;
         {
             const T* cfp = reinterpret_cast<const T*>(pl.cf) + ((long long)rw.b * pl.C + c_lo) * KK;
             const int n = (c_hi - c_lo) * KK;
@@ -520,13 +524,21 @@ band_kernel(const __grid_constant__ BandPlan pl) {
                 const int w = pl.bwdx ? KK - 1 - t : t;
                 const float v = Elem<T>::load(cfp + e);
                 big |= !(fabsf(v) < kBandFilterMax);
+                if constexpr (SMALL) large |= fabsf(v) >= kLargeCf;
                 const uint32_t bits = __float_as_uint(v);
                 const uint32_t to = sbase + pl.off_cf + (uint32_t)((unit * G + plane) * CH + part) * CFB + (uint32_t)((w % K) * CFC);
                 if constexpr (MIX) sts32(to + (uint32_t)(4 * (w / K)), bits);
                 else sts64(to + (uint32_t)(8 * (w / K)), bits, bits);
             }
         }
-        const bool plain = band_sync_or(NW * 32, big);
+        bool plain = band_sync_or(NW * 32, big | large);
+        float usual = __int_as_float(0x7f800000);   // the sum of a thread's magnitudes below which its results stand
+        if constexpr (SMALL) {
+            if (plain) {   // rarely
+                plain = band_sync_or(NW * 32, big);
+                if (!plain) usual = 0.f;
+            }
+        }
 
         if constexpr (REG) {
             if (started) {
@@ -616,9 +628,14 @@ band_kernel(const __grid_constant__ BandPlan pl) {
                 }
             };
             // (2-byte values of float16 have products of three inside float's range)
-            auto overflowed = [](const float (&res)[PH]) {
-                return MIX && std::is_same<T, __nv_bfloat16>::value &&
-                       !(fabsf(res[0]) + fabsf(res[1]) + fabsf(res[2]) + fabsf(res[3]) < __int_as_float(0x7f800000));
+            auto out_of_range = [&](const float (&res)[PH]) {
+                if constexpr (!SMALL) return false;
+                const float sum = fabsf(res[0]) + fabsf(res[1]) + fabsf(res[2]) + fabsf(res[3]);
+                if (sum < usual) return false;
+                bool again = !(sum < __int_as_float(0x7f800000));
+#pragma unroll
+                for (int p = 0; p < PH; ++p) again |= p < rows_left && usual == 0.f && fabsf(res[p]) < kBandSmall;
+                return again;
             };
             if (plain) {
 #pragma unroll 1
@@ -640,7 +657,7 @@ band_kernel(const __grid_constant__ BandPlan pl) {
                     band_columns<0, T, K, D, S, MUL, MIX>(row, cmask, cf_s + (uint32_t)(ch * CFB), sfr, acc);
                     float res[PH];
                     unpack(acc, res);
-                    if (left > ch * G && overflowed(res)) exact(ch, res);  // (a missing channel holds anything)
+                    if (left > ch * G && out_of_range(res)) exact(ch, res);  // (a missing channel holds anything)
                     if (ch == CH - 1) hand_back();
                     finish(ch, res);
                 }
@@ -659,7 +676,7 @@ band_kernel(const __grid_constant__ BandPlan pl) {
 #pragma unroll
                 for (int ch = 0; ch < CH; ++ch) {
                     unpack(acc[ch], res[ch]);
-                    if (left > ch * G && overflowed(res[ch])) exact(ch, res[ch]);
+                    if (left > ch * G && out_of_range(res[ch])) exact(ch, res[ch]);
                 }
                 hand_back();
 #pragma unroll

@@ -238,13 +238,21 @@ struct RingPlane {
     }
 };
 
+// bfloat16, x * sf before cf: where |x * sf| < 2^-126 it is rounded to a multiple of 2^-149, an error of at most 2^-150 |cf|
+// a tap.  With |cf| < 2^8 that is, over 25 taps, less than 2^-137, an eighth of half the smallest bfloat16's step.  While there
+// are larger ones in a stage a thread forms every result again, cf * sf first: the limit that it compares the sum of its
+// results' magnitudes with is then 0, not infinity.  (To ask which results are small enough to have lost something takes the
+// rest a twentieth: (64,256,28x28) 49 us; so 46.5 to 47.4, as without any of it.)
+constexpr float kLargeCf = 256.f;
+
 // The same for k = 5, mul: the filter's tap rows come one after the other (its 25 values and the 50 words of the
 // spatial filter do not fit the registers together), and two pixels take the float filter value in one instruction.
 template <typename T, typename G, int K, int PW, int PH>
 __device__ __forceinline__ void ring_plane_rows(uint32_t tb, uint32_t zb, uint32_t rowsel,
                                                 const uint32_t (&lmask)[G::NLW > 0 ? G::NLW : 1],
                                                 const uint32_t (&rmask)[G::NRW > 0 ? G::NRW : 1],
-                                                const uint32_t (&sfw)[K * K][PW * PH / 2], uint32_t cfa, float (&res)[PW * PH]) {
+                                                const uint32_t (&sfw)[K * K][PW * PH / 2], uint32_t cfa, float usual,
+                                                float (&res)[PW * PH]) {
     constexpr int P = PW * PH;
     uint32_t w[G::NR][G::NWIN];
     RingPlane<T, G, K, 1, 1, PW, PH, DDF_B200_MUL>::template Rows<0>::load(tb, zb, rowsel, lmask, rmask, w);
@@ -279,9 +287,10 @@ __device__ __forceinline__ void ring_plane_rows(uint32_t tb, uint32_t zb, uint32
         f2_unpack(acc2[q], res[2 * q], res[2 * q + 1]);
         sum += fabsf(res[2 * q]) + fabsf(res[2 * q + 1]);
     }
-    // x * sf may have left float's range although x * (cf * sf) does not (not with float16's values): again, w first
+    // x * sf may have left float's range, upwards or downwards, although x * (cf * sf) does not (not with float16's
+    // values): again, w first
     if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-        if (!(sum < __int_as_float(0x7f800000))) {
+        if (!(sum < usual)) {
 #pragma unroll
             for (int pp = 0; pp < P; ++pp) res[pp] = 0.f;
 #pragma unroll
@@ -492,11 +501,13 @@ ring_kernel(const __grid_constant__ RingPlan pl) {
         }
         // Channel filters of the planes this warp's lanes will process in this stage: raw
         // 2-byte values -> the per-warp layout [pass][group][tap] the plane loop reads.
+        float usual = __int_as_float(0x7f800000);   // k = 5: 0 where one of them is kLargeCf or more
         {
             const unsigned long long st_first_plane = (unsigned long long)plane_lo + (unsigned long long)st * stage_planes;
             const uint32_t coff = (uint32_t)((st_first_plane * (KK * 2)) & 15ull);
             const uint32_t src = RSTAGE(slot) + pl.off_rawcf + coff;
             const int n = npass * (two_groups ? 2 : 1) * KK;
+            bool large = false;
             __syncwarp();
             for (int e = lane; e < n; e += 32) {
                 const int u = e / KK, t = e - u * KK;          // u = pass * groups + group
@@ -504,10 +515,12 @@ ring_kernel(const __grid_constant__ RingPlan pl) {
                 const int tt = BWDX ? KK - 1 - t : t;          // grad-x reads the filter mirrored
                 const uint32_t raw = lds16(src + 2u * (uint32_t)((pq * TG + g_lo + gi) * KK + t));
                 const uint32_t dst = cfw + (uint32_t)((pq * 2 + gi) * G::CFP);
+                if constexpr (K != 3) large |= fabsf(__uint_as_float(Mix<T>::f32_bits(raw))) >= kLargeCf;
                 if constexpr (K != 3) sts64(dst + (uint32_t)(tt / K * G::CFR + tt % K * 8), Mix<T>::f32_bits(raw), Mix<T>::f32_bits(raw));
                 else if constexpr (MODE == DDF_B200_MUL) sts32(dst + 4u * (uint32_t)tt, Mix<T>::f32_bits(raw));
                 else sts16(dst + 2u * (uint32_t)tt, raw);
             }
+            if constexpr (K != 3) usual = __any_sync(0xffffffffu, large) ? 0.f : usual;
             __syncwarp();
         }
 
@@ -570,7 +583,7 @@ ring_kernel(const __grid_constant__ RingPlan pl) {
             for (; run > 0; --run) {
                 float res[P];
                 if constexpr (K != 3) {
-                    ring_plane_rows<T, G, K, PW, PH>(tb, zb, rowsel, lmask, rmask, sfw, cfa, res);
+                    ring_plane_rows<T, G, K, PW, PH>(tb, zb, rowsel, lmask, rmask, sfw, cfa, usual, res);
                 } else {
                     // the plane's converted channel filter: KK floats (mul) or KK packed halves (add)
                     uint32_t c[G::CFS];

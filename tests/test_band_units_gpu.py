@@ -43,3 +43,23 @@ def test_inputs_near_the_types_limit(shape):
     want = oracle_forward(x, cf, sf, k, d, s, "mul")
     assert torch.isfinite(want).all() and torch.isfinite(out).all()
     assert (out - want).norm() <= 4e-3 * want.norm()
+
+
+@pytest.mark.parametrize("shape", [SHAPES[0], SHAPES[3], SHAPES[4], SHAPES[6]])
+@pytest.mark.parametrize("large,small", [(2.0 ** 55, 2.0 ** -100), (2.0 ** 20, 2.0 ** -118)])
+def test_small_factors_of_a_large_filter(shape, large, small):
+    """x * sf falls below float's range, x * (cf * sf) does not: held in the 2-norm as above.  Some channels have ordinary
+    filters, some samples none that are large."""
+    from ddfnet_b200 import ddf
+    B, C, H, W, k, d, s = shape
+    x, cf, sf, go = make_inputs(B, C, H, W, k, s, torch.bfloat16, 9)
+    x, go, sf = x * small, go * small, sf * (2.0 ** -5 / large)
+    cf = cf * large
+    cf[1::2, 1::3] = 0.25
+    dev = torch.device("cuda:0")
+    xd = x.to(dev).requires_grad_()
+    out = ddf(xd, cf.to(dev), sf.to(dev), k, d, s, "mul")
+    (gx,) = torch.autograd.grad(out, xd, go.to(dev))
+    for got, want in ((out, oracle_forward(x, cf, sf, k, d, s, "mul")), (gx, oracle_backward(go, x, cf, sf, k, d, s, "mul")[0])):
+        got = got.detach().cpu().double()
+        assert (got - want).norm() <= 4e-3 * want.norm()

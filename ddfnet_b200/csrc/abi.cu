@@ -502,7 +502,7 @@ int ddf_b200_backward(const void* go, const void* x, const void* cf, const void*
     const bool want = variant == DDF_B200_VARIANT_STREAM || stream_worthwhile(p, di->sm_count);
 
     // Decide the filter-gradient path first, so that a missing workspace is reported before
-    // anything has been launched.  Only the spatial-filter gradient uses the workspace.
+    // anything has been launched.  Of the plane-streaming form only the spatial-filter gradient uses the workspace.
     bool filters_stream = (gcf || gsf) && allow_stream && want && bwd_stream_supported(p);
     if (filters_stream && gsf) {
         const size_t need = bwd_stream_workspace(p, di->sm_count);

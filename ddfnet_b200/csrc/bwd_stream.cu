@@ -123,9 +123,9 @@ int ddf_b200_backward_noalloc(const void* go, const void* x, const void* cf, con
     rc = device_facts(&sm_count, &fault, &index);
     if (rc) return rc;
 
-    // The same kernel choice as ddf_b200_backward makes under AUTO, so that both entry
-    // points give bit-identical results.  Only the spatial-filter gradient uses scratch:
-    // refuse, before anything is launched, if it would need more than the array holds.
+    // The same kernel choice as ddf_b200_backward makes under AUTO with all the scratch it asks for, so that both entry
+    // points give bit-identical results, as far as the array goes.  Of the plane-streaming form only the spatial-filter
+    // gradient uses scratch: refuse, before anything is launched, if it would need more than the array holds.
     const bool streaming = (gcf || gsf) &&
                            ddf_b200_plan(B, C, H, W, k, d, s, combine, dtype, 1) == DDF_B200_VARIANT_STREAM;
     if (streaming && gsf && bwd_stream_workspace(p, sm_count) > kStaticScratchBytes)
@@ -139,29 +139,29 @@ int ddf_b200_backward_noalloc(const void* go, const void* x, const void* cf, con
     }
     if (!gcf && !gsf) return 0;
 
-    if (streaming) {
+    // Outside the streaming kernel's range, or where the band form is the faster one: the band kernel, whose grad-cf may
+    // take scratch too, where the array holds what it needs for one sample.
+    size_t band = 0, least = 0;
+    const bool band_fits = band_filters_workspace(p, sm_count, &band, &least) && least <= kStaticScratchBytes;
+    if (streaming && !(band_fits && band_cols_preferred(p, sm_count))) {
         void* scratch = nullptr;
         if (gsf) {
             rc = static_scratch_address(index, &scratch);
             if (rc) return rc;
         }
         int launches = 0;
-        rc = band_cols_preferred(p, sm_count)
-                 ? kNotHandled
-                 : bwd_stream_filters(p, go, x, cf, sf, gcf, gsf, scratch, sm_count, fault, index,
-                                      reinterpret_cast<cudaStream_t>(stream), &launches);
+        rc = bwd_stream_filters(p, go, x, cf, sf, gcf, gsf, scratch, sm_count, fault, index,
+                                reinterpret_cast<cudaStream_t>(stream), &launches);
         if (rc != kNotHandled) return rc;
     }
-    // Outside the streaming kernel's range, or where the band form is the faster one: the band kernel where the array holds its scratch for one sample,
-    // else the generic kernels, which use no scratch at all.
-    size_t band = 0, least = 0;
-    if (band_filters_workspace(p, sm_count, &band, &least) && least <= kStaticScratchBytes) {
+    if (band_fits) {
         void* scratch = nullptr;
         rc = static_scratch_address(index, &scratch);
         if (rc) return rc;
         return ddf_b200_backward(go, x, cf, sf, nullptr, gcf, gsf, scratch, kStaticScratchBytes, B, C, H, W, k, d, s,
                                  combine, dtype, DDF_B200_VARIANT_AUTO, stream);
     }
+    // the generic kernels, which use no scratch at all
     return ddf_b200_backward(go, x, cf, sf, nullptr, gcf, gsf, nullptr, 0, B, C, H, W, k, d, s,
                              combine, dtype, DDF_B200_VARIANT_GENERIC, stream);
 }

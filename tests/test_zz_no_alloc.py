@@ -100,6 +100,30 @@ def test_noalloc_small_problems_and_single_gradients():
     assert L.ddf_b200_take_fault() == 0
 
 
+@pytest.mark.parametrize("shape", [(1, 12288, 28, 30, 5, 1, 1), (1, 16384, 11, 50, 5, 1, 1)])
+def test_noalloc_keeps_the_plane_streaming_form(shape):
+    """Where AUTO prefers the tap columns but the array does not hold their scratch for one sample, the plane-streaming
+    form, whose scratch it holds, runs as it does in ddf_b200_backward."""
+    from ddfnet_b200 import _lib
+    L = _lib.load()
+    B, C, H, W, k, d, s = shape
+    limit = int(L.ddf_b200_backward_noalloc_limit())
+    assert L.ddf_b200_backward_workspace(*shape, 0, 1, _lib.VARIANT_AUTO) > limit
+    need = int(L.ddf_b200_backward_workspace(*shape, 0, 1, _lib.VARIANT_STREAM))
+    assert 0 < need <= limit
+    x, cf, sf, go = (t.to("cuda:0") for t in make_inputs(B, C, H, W, k, s, torch.float16, seed=43))
+    ws = torch.empty(need, dtype=torch.uint8, device="cuda:0")
+    stream = torch.cuda.current_stream().cuda_stream
+    ins = [t.data_ptr() for t in (go, x, cf, sf)]
+    got, want = ([torch.empty_like(t) for t in (x, cf, sf)] for _ in range(2))
+    assert L.ddf_b200_backward(*ins, *(t.data_ptr() for t in want), ws.data_ptr(), need, *shape, 0, 1, _lib.VARIANT_STREAM, stream) == 0
+    assert L.ddf_b200_backward_noalloc(*ins, *(t.data_ptr() for t in got), *shape, 0, 1, stream) == 0
+    torch.cuda.synchronize()
+    for name, g, w in zip(("grad_x", "grad_cf", "grad_sf"), got, want):
+        assert torch.equal(g, w), name
+    assert L.ddf_b200_take_fault() == 0
+
+
 def test_noalloc_refuses_problems_beyond_its_scratch():
     from ddfnet_b200 import _lib
     L = _lib.load()

@@ -139,11 +139,12 @@ int ddf_b200_backward_noalloc(const void* go, const void* x, const void* cf, con
     }
     if (!gcf && !gsf) return 0;
 
-    // Outside the streaming kernel's range, or where the band form is the faster one: the band kernel, whose grad-cf may
-    // take scratch too, where the array holds what it needs for one sample.
+    // Outside the streaming kernel's range, or where the band form is the faster one: the band kernel where the array holds
+    // what it needs for one sample.  Its grad-cf may take scratch too; the plane-streaming form's takes none, so that grad-cf
+    // alone leaves the array to other streams and has the bits of ddf_b200_backward without a workspace.
     size_t band = 0, least = 0;
     const bool band_fits = band_filters_workspace(p, sm_count, &band, &least) && least <= kStaticScratchBytes;
-    if (streaming && !(band_fits && band_cols_preferred(p, sm_count))) {
+    if (streaming && !(gsf && band_fits && band_cols_preferred(p, sm_count))) {
         void* scratch = nullptr;
         if (gsf) {
             rc = static_scratch_address(index, &scratch);

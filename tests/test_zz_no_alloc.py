@@ -124,6 +124,24 @@ def test_noalloc_keeps_the_plane_streaming_form(shape):
     assert L.ddf_b200_take_fault() == 0
 
 
+@pytest.mark.parametrize("shape", [(64, 64, 14, 14, 3, 1, 1), (64, 64, 14, 14, 5, 1, 1)])
+def test_noalloc_channel_filter_alone_takes_no_scratch(shape):
+    """Where AUTO prefers the tap columns: grad-cf alone is what ddf_b200_backward gives without a workspace."""
+    from ddfnet_b200 import _lib
+    L = _lib.load()
+    B, C, H, W, k, d, s = shape
+    assert L.ddf_b200_plan(*shape, 0, 1, 1) == _lib.VARIANT_STREAM
+    x, cf, sf, go = (t.to("cuda:0") for t in make_inputs(B, C, H, W, k, s, torch.float16, seed=44))
+    stream = torch.cuda.current_stream().cuda_stream
+    ins = [t.data_ptr() for t in (go, x, cf, sf)]
+    a, b = torch.empty_like(cf), torch.empty_like(cf)
+    assert L.ddf_b200_backward(*ins, None, a.data_ptr(), None, None, 0, *shape, 0, 1, _lib.VARIANT_AUTO, stream) == 0
+    assert L.ddf_b200_backward_noalloc(*ins, None, b.data_ptr(), None, *shape, 0, 1, stream) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(a, b)
+    assert L.ddf_b200_take_fault() == 0
+
+
 def test_noalloc_refuses_problems_beyond_its_scratch():
     from ddfnet_b200 import _lib
     L = _lib.load()

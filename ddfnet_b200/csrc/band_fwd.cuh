@@ -394,7 +394,9 @@ band_kernel(const __grid_constant__ BandPlan pl) {
 #pragma unroll
             for (int r = 0; r < NR; ++r) {
                 const int iy = y0 * S + D * (r - R);
-                rowoff[r] = (active && iy >= 0 && iy < pl.H)
+                // (a row that no pixel of the thread needs may not have been copied: odd heights at stride 2)
+                const bool needed = rows_left >= PH || r < S * (rows_left - 1) + K;
+                rowoff[r] = (active && needed && iy >= 0 && iy < pl.H)
                                 ? (uint32_t)pip * (uint32_t)plane_bytes + (uint32_t)(((iy - rw.iy_lo) * pl.W + x * S) * ES)
                                 : pl.zero_off + 16u;
                 pin(rowoff[r]);

@@ -13,9 +13,15 @@
 //
 // A thread owns four output pixels of one column, D rows apart (so neighbouring windows share rows at
 // every dilation).  Lanes of a warp own neighbouring columns: every shared load is conflict-free and
-// every store coalesced at any width and alignment, which vectors along x would not be.  One thread per position
-// fetches its pixels' k*k filter values when a band begins and leaves them in shared memory, laid out for its
-// own later loads; k = 3 takes them into registers from there, k = 5 a column of taps at a time, for two channels.
+// every store coalesced at any width and alignment, which vectors along x would not be.
+//
+// The filters of a thread's pixels when a band begins, in one of two ways.  Straight into the thread's registers (DIRECT),
+// every load in flight at once: the forward but for 2-byte mul at k = 3, and at k = 5 but for the two rules of band_launch.
+// Or by one thread per position to shared memory, laid out for its own later loads; k = 3 takes them into registers from
+// there, k = 5 a column of taps at a time, for two channels, at 96 registers a thread and not 168.  That way costs up to
+// 3 us at the start: us, forward, by way of shared memory alone -> as it is (and before there was that way):
+// (2,16,46x70) f32 k = 5 8.6 -> 5.4 (5.7), (3,24,56x56) bf16 add 5.7 -> 4.3 (4.8), (1,300,60x60) f32 9.0 -> 7.2 (8.2),
+// (2,64,29x31) f32 5.4 -> 3.7 (4.1), (7,96,48x29) f32 k = 5 add 17.5 -> 11.1 (13.6).
 //
 // Arithmetic.  2-byte types, mul: x * sf exact by the mixed-precision FMA from the 2-byte operands, then a float FMA
 // with cf (two-wide FMAs there wait for the pipe: 42.3 against 39.7 us at (2,128,200x280) bf16).  Float, add, and
@@ -23,12 +29,14 @@
 //
 // What bounds it: instruction issue (9 FMAs of 10 instructions at k = 5, 18 of 51 per output at k = 3 in mul).  Half
 // of what it issued before were products and selects that the compiler formed again in each pass (see pin); stores
-// under a predicate instead of a branch took another eighth.  us, forward / grad-x, before (filters in registers
-// from global memory, 80 to 168 registers) -> now: (2,256,200x300) f32 80.4 / 84.0 -> 76.4 / 78.7 and bf16
-// 84.9 / 89.3 -> 68.0 / 67.8, (4,128,50x67) f16 11.2 / 14.9 -> 10.1 / 11.5, (8,48,150x130) f16 add 25.9 / 30.4 ->
-// 24.8 / 25.6, k = 5 (8,96,75x101) f16 50.1 / 54.9 -> 35.3 / 37.9, f32 47.9 / 52.4 -> 43.1 / 41.7, and
-// (128,64,56x56) bf16 178 / 191 -> 139 / 139; (1,300,60x60) f32 8.3 / 11.4 -> 9.2 / 9.5.  Not kept: four channels a
-// unit (the same or slower), the filters of k = 3 out of shared memory in every pass.
+// under a predicate instead of a branch took another eighth.  Not all that is pinned stays in registers: -Xptxas -v shows
+// up to 132 bytes a thread spilled with MIX, 192 in grad-x and the normalised k = 5 without, 128 in the DIRECT forms (0 to 20 at
+// k = 3, stride 1).  us, forward / grad-x, before (a CTA of 80 to 168 registers a thread for both) -> now:
+// (2,256,200x300) f32 80.7 / 84.4 -> 67.6 / 79.0 and bf16 85.0 / 89.7 -> 69.5 / 69.7, (4,128,50x67) f16 11.4 / 15.0 ->
+// 10.5 / 11.9, (8,48,150x130) f16 add 26.1 / 30.7 -> 21.5 / 25.8, k = 5 (8,96,75x101) f16 50.4 / 55.1 -> 35.6 / 38.3, f32
+// 48.0 / 52.6 -> 37.8 / 42.6, and (128,64,56x56) bf16 178 / 191 -> 138 / 139; (1,300,60x60) f32 8.2 / 11.3 -> 7.2 / 9.5.
+// float32 at more than 288 columns is one CTA of ten compute warps an SM (96 registers), and the faster one all the same.
+// Not kept: four channels a unit (the same or slower), the filters of k = 3 out of shared memory in every pass.
 //
 // Zero padding.  Rows outside the plane are read from a zeroed spot of the slot (their offset is a
 // per-thread constant), columns outside are masked.  A zero times an infinite filter value would be
@@ -125,6 +133,16 @@ template <> struct Masked<__half> {
     template <int OFF> static __device__ __forceinline__ float at(uint32_t a, uint32_t m) { return Word<__half>::get(lds16i<OFF>(a) & m, 0); }
 };
 
+// An element's bits as they are loaded, and as a float's.
+template <typename T> struct Raw {
+    static __device__ __forceinline__ uint32_t load(const T* p) { return __ldg(reinterpret_cast<const uint16_t*>(p)); }
+    static __device__ __forceinline__ uint32_t f32_bits(uint32_t v) { return Mix<T>::f32_bits(v); }
+};
+template <> struct Raw<float> {
+    static __device__ __forceinline__ uint32_t load(const float* p) { return __float_as_uint(__ldg(p)); }
+    static __device__ __forceinline__ uint32_t f32_bits(uint32_t v) { return v; }
+};
+
 // Bytes of a channel's filter in shared memory: (c, c) pairs column by column, each column padded to
 // whole 16 bytes; SINGLE: plain floats.
 template <int K, bool SINGLE = false> constexpr int kBandCf = K * (SINGLE ? (K + 3) / 4 * 16 : (K + 1) / 2 * 16);
@@ -151,8 +169,8 @@ __device__ __forceinline__ bool band_sync_or(int n, int v) {
 template <int K> constexpr int kBandThreads = K == 3 ? 352 : 384;
 constexpr int kBandPixels = 4;  // rows a thread owns in its column
 // Registers of a thread: 24 warps of an SM, or 20 where 36 filter values (k = 3, float) or two channels' rows of a
-// 5 x 5 window are held.
-template <int K, bool MIX> constexpr int kBandRegs = K == 3 && MIX ? 80 : 96;
+// 5 x 5 window are held, or 12 where 100 filter values are (whole CTAs of them: one of 11 warps at 300 columns).
+template <int K, bool MIX, bool DIRECT = false> constexpr int kBandRegs = K == 5 && DIRECT ? 168 : K == 3 && MIX ? 80 : 96;
 
 // Stores v where pixel P is one of the first n; a predicate and no branch.
 template <int P>
@@ -240,9 +258,11 @@ __device__ __forceinline__ void band_columns_shared(const uint32_t (&row)[CH][NR
 }
 
 // MIX: 2-byte filters as they are, x * sf exact by the mixed-precision FMA; else float filters (float tensors, and
-// filters normalised here).  CH: channels a thread has of a unit.
-template <typename T, int K, int D, int S, int MODE, bool MIX, int CH>
-__global__ void __maxnreg__((kBandRegs<K, MIX>))
+// filters normalised here).  CH: channels a thread has of a unit.  DIRECT: the forward's filters of a thread's pixels come into
+// its registers straight from global memory, at k = 5 as they are (1) or normalised here (2: code for both in one kernel
+// takes (2,64,200x300) k = 5 add from 39 to 44 us).
+template <typename T, int K, int D, int S, int MODE, bool MIX, int CH, int DIRECT>
+__global__ void __maxnreg__((kBandRegs<K, MIX, DIRECT != 0>))
 band_kernel(const __grid_constant__ BandPlan pl) {
     constexpr int KK = K * K, R = (K - 1) / 2, ES = (int)sizeof(T);
     constexpr int PH = kBandPixels, NR = S * (PH - 1) + K;   // window rows of a thread, D input rows apart
@@ -250,7 +270,8 @@ band_kernel(const __grid_constant__ BandPlan pl) {
     constexpr int CFB = kBandCf<K, MIX>;
     constexpr int CFC = CFB / K;              // bytes of one tap column
     constexpr uint32_t SFB = PH * (MIX ? 2 : 4);   // bytes of a tap of a thread's pixels
-    constexpr bool REG = K == 3;              // the filters of a thread's pixels stay in registers
+    constexpr bool REG = K == 3 || DIRECT;    // the filters of a thread's pixels stay in registers
+    constexpr bool NORM = DIRECT && !MIX && (K == 3 || DIRECT == 2);
     static_assert(D == 1 || S == 1, "dilated windows are built at stride 1");
     static_assert(!MIX || (ES == 2 && MUL), "mixed-precision products take 2-byte factors; w = cf + sf is float");
 
@@ -405,9 +426,65 @@ band_kernel(const __grid_constant__ BandPlan pl) {
             // Spatial filters of the position's pixels, by one thread each.  Loads from clamped addresses and
             // values dropped after: a load behind a branch would wait for the one before.
             big_sf = 0;
-            if (owner && pip == 0) {
+            if constexpr (DIRECT) {
                 const T* sfb = reinterpret_cast<const T*>(pl.sf) + (long long)rw.b * KK * out_plane;
                 float sum_abs = 0.f;
+                const T* at[PH];
+#pragma unroll
+                for (int p = 0; p < PH; ++p) at[p] = p < rows_left ? sfb + (y0 + D * p) * pl.OW + x : sfb;
+#pragma unroll
+                for (int t = 0; t < KK; ++t) {
+                    uint32_t v[PH];
+#pragma unroll
+                    for (int p = 0; p < PH; ++p) {
+                        v[p] = Raw<T>::load(at[p]);
+                        at[p] += out_plane;
+                        if (p >= rows_left) v[p] = 0u;
+                        sum_abs += fabsf(__uint_as_float(Raw<T>::f32_bits(v[p])));
+                    }
+                    auto& to = sfr[(t % K) * K + t / K];
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        if constexpr (MIX) to[q] = v[2 * q] | (v[2 * q + 1] << 16);
+                        else to[q] = f2_pack(__uint_as_float(Raw<T>::f32_bits(v[q])), __uint_as_float(Raw<T>::f32_bits(v[q + 2])));
+                    }
+                }
+                if constexpr (NORM) {
+                    if (K == 5 || pl.norm) {
+                        sum_abs = 0.f;
+#pragma unroll
+                        for (int q = 0; q < 2; ++q) {
+                            unsigned long long sum2 = 0ull, var2 = 0ull;
+#pragma unroll
+                            for (int t = 0; t < KK; ++t) sum2 = f2_add(sum2, sfr[(t % K) * K + t / K][q]);
+                            float lo, hi;
+                            f2_unpack(sum2, lo, hi);
+                            const unsigned long long less2 = f2_pack(-(lo / (float)KK), -(hi / (float)KK));
+#pragma unroll
+                            for (int t = 0; t < KK; ++t) {
+                                auto& v2 = sfr[(t % K) * K + t / K][q];
+                                v2 = f2_add(v2, less2);
+                                var2 = f2_fma(v2, v2, var2);
+                            }
+                            f2_unpack(var2, lo, hi);
+                            const unsigned long long inv2 = f2_pack(pl.sf_scale / (sqrtf(lo / (float)(KK - 1)) + 1e-10f),
+                                                                    pl.sf_scale / (sqrtf(hi / (float)(KK - 1)) + 1e-10f));
+#pragma unroll
+                            for (int t = 0; t < KK; ++t) {
+                                auto& v2 = sfr[(t % K) * K + t / K][q];
+                                v2 = f2_mul(v2, inv2);
+                                f2_unpack(v2, lo, hi);
+                                sum_abs += fabsf(lo) + fabsf(hi);
+                            }
+                        }
+                    }
+                }
+                big_sf = !(sum_abs < kBandFilterMax);
+            } else if (owner && pip == 0) {
+                const T* sfb = reinterpret_cast<const T*>(pl.sf) + (long long)rw.b * KK * out_plane;
+                float sum_abs = 0.f;
+                // (The forward's branch stays where grad-x alone is launched, k = 3 without MIX: without it the compiler keeps
+                // others of the thread's constants in registers, and (2,256,200x300) f32 takes 82.5 us, not 78.6.)
                 if (!pl.bwdx) {
                     const T* at[PH];
                     bool ok[PH];
@@ -542,7 +619,7 @@ band_kernel(const __grid_constant__ BandPlan pl) {
             }
         }
 
-        if constexpr (REG) {
+        if constexpr (REG && !DIRECT) {
             if (started) {
 #pragma unroll
                 for (int t = 0; t < KK; ++t) {
@@ -611,7 +688,22 @@ band_kernel(const __grid_constant__ BandPlan pl) {
                 const uint32_t base = base_of(ch);
 #pragma unroll
                 for (int p = 0; p < PH; ++p) {
-                    float a = 0.f;
+                    float a = 0.f, mean = 0.f, inv = 1.f;
+                    const T* sfp = reinterpret_cast<const T*>(pl.sf) + (long long)rw.b * KK * out_plane + (y0 + p * D) * pl.OW + x;
+                    if constexpr (NORM) {
+                        if ((K == 5 || pl.norm) && p < rows_left) {
+                            float var = 0.f;
+#pragma unroll 1
+                            for (int t = 0; t < KK; ++t) mean += Elem<T>::load(sfp + t * out_plane);
+                            mean /= (float)KK;
+#pragma unroll 1
+                            for (int t = 0; t < KK; ++t) {
+                                const float v = Elem<T>::load(sfp + t * out_plane) - mean;
+                                var = fmaf(v, v, var);
+                            }
+                            inv = pl.sf_scale / (sqrtf(var / (float)(KK - 1)) + 1e-10f);
+                        }
+                    }
 #pragma unroll 1
                     for (int t = 0; t < KK; ++t) {  // t = column-major tap
                         const int col = t / K, k = t - col * K;
@@ -619,7 +711,9 @@ band_kernel(const __grid_constant__ BandPlan pl) {
                         if (p >= rows_left || iy < 0 || iy >= pl.H || ix < 0 || ix >= pl.W) continue;
                         const uint32_t sa = sf_s + (uint32_t)t * sf_tap;
                         float sv;
-                        if constexpr (MIX) sv = Word<T>::get(lds16(sa + 2u * p), 0);
+                        if constexpr (DIRECT)
+                            sv = (Elem<T>::load(sfp + (k * K + col) * out_plane) - mean) * inv;
+                        else if constexpr (MIX) sv = Word<T>::get(lds16(sa + 2u * p), 0);
                         else sv = ldsf(sa + 4u * (uint32_t)((p & 1) * 2 + (p >> 1)));
                         const float cv = ldsf(cf_s + (uint32_t)(ch * CFB + col * CFC + (MIX ? 4 : 8) * k));
                         const uint32_t at = base + (uint32_t)pip * (uint32_t)plane_bytes +
@@ -750,7 +844,7 @@ inline bool band_split(int B, int C, int OH, int OW, int D, int PH, int max_thre
 }
 
 // The launch of one instantiation; kNotHandled where it does not fit.
-template <typename T, int K, int D, int S, int MODE, bool MIX, int CH>
+template <typename T, int K, int D, int S, int MODE, bool MIX, int CH, int DIRECT>
 int band_launch_split(const BandArgs& a, const BandSplit& sp, cudaStream_t stream) {
     const Problem& p = a.p;
     constexpr int ES = (int)sizeof(T), R = (K - 1) / 2, PH = kBandPixels;
@@ -785,8 +879,8 @@ int band_launch_split(const BandArgs& a, const BandSplit& sp, cudaStream_t strea
         pl.stage_passes = stage / per_unit > 1 ? stage / per_unit : 1;
         if (pl.stage_passes > pl.passes) pl.stage_passes = pl.passes;
         pl.off_sf = round_up(pl.off_cf + (uint32_t)(pl.stage_passes * per_unit) * kBandCf<K, MIX>, 128);
-        pl.off_slot0 = round_up(pl.off_sf + (uint32_t)(K * K * sp.groups * p.OW * PH * (MIX ? 2 : 4)), 128);
-        const int fit = 4 * (65536 / 4 / 32 / kBandRegs<K, MIX>) / (sp.warps + 1);  // whole warps in each quarter of an SM
+        pl.off_slot0 = round_up(pl.off_sf + (DIRECT ? 0u : (uint32_t)(K * K * sp.groups * p.OW * PH * (MIX ? 2 : 4))), 128);
+        const int fit = 4 * (65536 / 4 / 32 / kBandRegs<K, MIX, DIRECT != 0>) / (sp.warps + 1);  // whole warps in each quarter of an SM
         for (ctas = fit < 1 ? 1 : fit < 4 ? fit : 4; ctas >= 1; --ctas) {
             const uint32_t budget = ctas == 1 ? kSmemBudget : (227u << 10) / (uint32_t)ctas - 1024u;
             if (pl.off_slot0 >= budget) continue;
@@ -799,7 +893,7 @@ int band_launch_split(const BandArgs& a, const BandSplit& sp, cudaStream_t strea
     const long long most = (long long)ctas * a.sm_count;
     const long long grid = units < most ? units : most;
     const uint32_t smem = pl.off_slot0 + (uint32_t)pl.n_slots * pl.slot_stride;
-    auto kern = band_kernel<T, K, D, S, MODE, MIX, CH>;
+    auto kern = band_kernel<T, K, D, S, MODE, MIX, CH, DIRECT>;
     static std::atomic<unsigned long long> opted_in{0};
     const unsigned long long bit = 1ull << (a.device & 63);
     if (!(opted_in.load(std::memory_order_acquire) & bit)) {
@@ -820,12 +914,34 @@ int band_launch(const BandArgs& a, cudaStream_t stream) {
     // Two channels a thread and unit share the waits and, at k = 5, the filters' way out of shared memory; one where
     // the units of two would not go evenly into the CTAs ((1,300,60x60) f32: two or three each, 9.3 us against 8.3).
     auto units = [&](int planes, int ch) { return (long long)p.B * sp.bands * ((p.C + planes * ch - 1) / (planes * ch)); };
+    // Filters straight into registers, us by way of shared memory against it.  Level at 50 units of one channel per SM for
+    // 2-byte mul at k = 5 ((8,96,75x101) f16 35.5 / 35.8; (1,135,135x162) f16 25.0 / 23.3, (128,64,56x56) bf16 138 / 152),
+    // whose filters take half the shared memory; at three for normalised ones at k = 5 ((8,61,24x37) f16 11.9 / 12.6,
+    // (2,40,40x45) bf16 add 9.3 / 7.3); the faster way at every size without MIX (k = 5 (2,64,200x300) bf16 add 46.7 / 39.0,
+    // (2,16,46x70) f32 8.6 / 5.4; k = 3 (2,256,200x300) f32 76.6 / 67.6, normalised 77.5 / 69.4).
+    const bool direct = !a.bwdx && (K == 3 ? !MIX : MIX ? units(sp.planes, 1) < 50ll * a.sm_count
+                                                         : !p.sf_norm || units(sp.planes, 1) < 3ll * a.sm_count);
     // fewer planes together while there are SMs without a unit
-    while (K == 3 && sp.planes > 1 && units(sp.planes, 1) < a.sm_count) sp.planes = (sp.planes + 1) / 2;
+    while ((K == 3 || direct) && sp.planes > 1 && units(sp.planes, 1) < a.sm_count) sp.planes = (sp.planes + 1) / 2;
     sp.warps = (sp.planes * sp.groups * p.OW + 31) / 32;
-    if constexpr (K == 3)
-        if (units(sp.planes, 2) < 6ll * a.sm_count) return band_launch_split<T, K, D, S, MODE, MIX, 1>(a, sp, stream);
-    return band_launch_split<T, K, D, S, MODE, MIX, 2>(a, sp, stream);
+    if constexpr (K == 5) {
+        if (direct) {
+            if constexpr (!MIX)
+                if (p.sf_norm) return band_launch_split<T, K, D, S, MODE, MIX, 1, 2>(a, sp, stream);
+            return band_launch_split<T, K, D, S, MODE, MIX, 1, 1>(a, sp, stream);
+        }
+        return band_launch_split<T, K, D, S, MODE, MIX, 2, 0>(a, sp, stream);
+    } else {
+        const bool one = units(sp.planes, 2) < 6ll * a.sm_count;
+        if constexpr (!MIX)
+            if (direct)
+                return one ? band_launch_split<T, K, D, S, MODE, MIX, 1, 1>(a, sp, stream)
+                           : band_launch_split<T, K, D, S, MODE, MIX, 2, 1>(a, sp, stream);
+        if constexpr (MIX || S == 1)
+            return one ? band_launch_split<T, K, D, S, MODE, MIX, 1, 0>(a, sp, stream)
+                       : band_launch_split<T, K, D, S, MODE, MIX, 2, 0>(a, sp, stream);
+        return kNotHandled;
+    }
 }
 
 // Defined once per element type in band_inst_<type>.cu.

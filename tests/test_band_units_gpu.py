@@ -63,3 +63,36 @@ def test_small_factors_of_a_large_filter(shape, large, small):
     for got, want in ((out, oracle_forward(x, cf, sf, k, d, s, "mul")), (gx, oracle_backward(go, x, cf, sf, k, d, s, "mul")[0])):
         got = got.detach().cpu().double()
         assert (got - want).norm() <= 4e-3 * want.norm()
+
+
+# (B, C, H, W, k, d, s), normalised in the kernel: at k = 5 straight into registers (few units a CTA) and by way of shared memory
+@pytest.mark.parametrize("shape", [(2, 37, 50, 67, 5, 1, 1), (3, 160, 50, 67, 5, 2, 1), (1, 43, 50, 67, 3, 1, 1), (6, 75, 50, 37, 3, 1, 2)])
+@pytest.mark.parametrize("dt", ["f32", "f16"])
+@pytest.mark.parametrize("mode", ["mul", "add"])
+def test_filters_normalised_in_the_kernel(shape, dt, mode):
+    """The last sample's channel filters are beyond what products with padding zeros may meet: tap by tap there."""
+    from ddfnet_b200.op import ddf_sfnorm, spatial_filter_norm
+    B, C, H, W, k, d, s = shape
+    x, cf, raw, _ = make_inputs(B, C, H, W, k, s, DTYPES[dt], 50 + sum(shape))
+    raw = raw + 0.4
+    big = dt == "f32" and mode == "mul"
+    if big:
+        cf[-1, 0] = 2e18
+    dev = torch.device("cuda:0")
+    out = ddf_sfnorm(x.to(dev), cf.to(dev), raw.to(dev), k, d, s, mode, 0.7).cpu()
+    want = oracle_forward(x, cf, spatial_filter_norm(raw.double(), k, 0.7), k, d, s, mode)
+    if big:
+        got = out[-1, 0].double()
+        assert (got - want[-1, 0]).norm() <= 1e-6 * want[-1, 0].norm()
+        out[-1, 0], want[-1, 0] = 0.0, 0.0
+    check_close(out, want, DTYPES[dt], f"sfnorm {shape} {dt} {mode}")
+
+
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
+def test_many_units_at_k5(dt):
+    """2-byte mul by way of shared memory: more than fifty units of a channel per SM."""
+    from ddfnet_b200 import ddf
+    x, cf, sf = make_inputs(2, 960, 200, 19, 5, 1, DTYPES[dt], 51, with_go=False)
+    dev = torch.device("cuda:0")
+    out = ddf(x.to(dev), cf.to(dev), sf.to(dev), 5, 1, 1, "mul")
+    check_close(out, oracle_forward(x, cf, sf, 5, 1, 1, "mul"), DTYPES[dt], f"forward {dt}")

@@ -281,17 +281,19 @@ static bool stream_worthwhile(const Problem& p, int sm_count) {
 
 // AUTO prefers the band forward and grad-x to the generic kernels except, us of both in a graph:
 //  - planes of one row, where most taps are padding, which the generic kernels skip: (16,64,1x100) f16 forward
-//    5.8 against 3.5, grad-x 8.3 against 4.1, (4096,64,1x7) f32 k = 5 155 against 30; and of one column, unless
-//    there are very many: (64,64,7x1) f32 1.2 times, but (64,64,300x1) f32 k = 5 18 against 31 (at 2^19 outputs
+//    5.0 against 3.1, grad-x 8.3 against 4.1, (4096,64,1x7) f32 k = 5 137 against 30; and of one column, unless
+//    there are very many: (64,64,7x1) f32 3.7 against 2.8, but (64,64,300x1) f32 k = 5 17 against 31 (at 2^19 outputs
 //    the two are level);
-//  - planes of fewer than nine pixels: (256,64,2x2) f16 5.1 against 3.9, (4096,2048,1x1) f32 k = 5 2916 against
-//    134; (256,16,3x3) f32 is 4.0 against 4.5 (k = 5, 3x3: 0.7 times for few samples, 1.6 at (8000,64));
+//  - planes of fewer than nine pixels: (256,64,2x2) f16 4.5 against 3.6, (1024,512,1x1) f32 k = 5 114 against
+//    8; (256,16,3x3) f32 is 3.7 against 4.1 (k = 5, 3x3: (16,16) 4.3 against 7.7, (8000,64) 356 against 227);
 //  - more samples than four CTAs per SM take at once, each with little work: a change of sample costs 2 to 3 us
-//    (k = 5: 4 to 7).  (4096,1,5x5) f16 15 against 5.2, (600,4,5x5) f32 5.6 against 4.7; with 162 outputs a sample
-//    ((2000,2,9x9) f32 k = 5) 0.87 times.
-// Elsewhere it wins from the smallest size on: (1,16,7x7) f16 3.6 against 3.9, (1,256,14x14) f16 3.7 against
-// 4.4, (2,64,29x31) f32 4.1 against 5.3, (1,16,33x31) f16 k = 5 5.3 against 7.8, (2,256,200x300) f32 80 against
-// 655.  The filter gradients win everywhere ((1,16,7x7) f16 7.7 against 11.3, (1,2048,1x1) f16 18 against 193).
+//    (k = 5: 4 to 7).  (4096,1,5x5) f16 16 against 4.7, (600,4,5x5) f32 5.1 against 4.3; with 162 outputs a sample
+//    ((2000,2,9x9) f32 k = 5) 14 against 18.
+// Elsewhere it wins from the smallest size on: (1,16,7x7) f16 2.8 against 4.0, (1,256,14x14) f16 3.6 against
+// 4.1, (2,64,29x31) f32 3.7 against 4.9, (1,80,36x41) f32 3.7 against 5.0, (2,24,56x56) f32 stride 2 3.9 against 4.0,
+// (1,16,33x31) f16 k = 5 4.8 against 7.7, (2,16,46x70) f32 k = 5 5.3 against 8.7, (2,256,200x300) f32 67 against
+// 653; not at (1,128,56x56) f16 stride 2 (5.2 against 4.6).  The filter gradients win everywhere ((1,16,7x7) f16 7.7
+// against 11.3, (1,2048,1x1) f16 18 against 193).
 static bool band_worthwhile(const Problem& p, int sm_count) {
     const long long pixels = (long long)p.OH * p.OW;
     if (p.OH == 1 || pixels < 9) return false;

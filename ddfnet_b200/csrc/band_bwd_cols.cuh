@@ -14,7 +14,7 @@
 // 14 and 7 columns the plane-streaming form) -> this one: (2,256,200x300) bf16 179 -> 131, (8,48,150x130) f16 add 86.7 -> 43.8,
 // (16,64,99x51) d = 2 bf16 52.9 -> 38.2, (4,128,50x67) f16 23.0 -> 19.3, k = 5 (128,64,56x56) bf16 804 -> 384,
 // (8,96,75x101) f16 207 -> 130, (64,512,14x14) bf16 167 -> 124, (64,512,7x7) bf16 123 -> 64.  Registers: 64 (k = 3)
-// and 96 leave room for 32 and 20 warps; k = 5 at 80 spills in its loop.  Not kept: scalar instead of two-wide sums
+// and 96 leave room for 32 and 20 warps; mul spills there, 84 and 64 bytes a thread loaded, k = 5 at 80 far more.  Not kept: scalar instead of two-wide sums
 // (154 at (2,256,200x300)).
 #pragma once
 
@@ -39,17 +39,16 @@ struct BandColsPlan {
     uint32_t off_red, part_stride;
 };
 
-template <typename T, int K, int D, int S, int MODE>
+template <typename T, int K, int D, int MODE>
 __global__ void __launch_bounds__(kColsThreads<K>, 1)
 band_cols_kernel(const __grid_constant__ BandColsPlan cp) {
     constexpr int KK = K * K, R = (K - 1) / 2, ES = (int)sizeof(T), PH = kColsPixels, CH = kColsCh;
-    constexpr int NR = S * (PH - 1) + K;
+    constexpr int NR = PH - 1 + K;
     constexpr int CFB = kBandCf<K>, CFC = CFB / K;
     constexpr bool MUL = MODE == DDF_B200_MUL;
     constexpr int SUMS = CH * K;                       // sums over lanes of a pass
     constexpr int LPS = 32 / SUMS >= 2 ? 2 : 1;        // lanes that share one
     static_assert(ES == 2 && SUMS * LPS <= 32, "2-byte types; one lane a sum at least");
-    static_assert(D == 1 || S == 1, "dilated windows are built at stride 1");
 
     const BandBwdPlan& pl = cp.p;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -88,8 +87,8 @@ band_cols_kernel(const __grid_constant__ BandColsPlan cp) {
     const int y_lo = band_row<D, PH>(band / cp.x_parts * pl.groups);
     const int y_next = y_lo + band_rows<D, PH>(pl.groups);
     int y_hi = y_next < pl.OH ? y_next : pl.OH;
-    int iy_lo = y_lo * S - R * D > 0 ? y_lo * S - R * D : 0;
-    const int iy_end = (y_hi - 1) * S + R * D + 1;
+    int iy_lo = y_lo - R * D > 0 ? y_lo - R * D : 0;
+    const int iy_end = y_hi + R * D;
     int iy_hi = iy_end < pl.H ? iy_end : pl.H;
     int go_row = y_lo;
     if (D > 1 && y_lo >= pl.OH) {  // the plane ends before this group: any row will do
@@ -141,7 +140,7 @@ band_cols_kernel(const __grid_constant__ BandColsPlan cp) {
     const int y0 = y_lo + band_row<D, PH>(grp);
     int rows_in = pos < pl.groups * pl.OW && y0 < pl.OH ? (pl.OH - y0 + D - 1) / D : 0;  // pixels inside the plane
     if (rows_in > PH) rows_in = PH;
-    const int ix = x * S + D * (j - R);
+    const int ix = x + D * (j - R);
     const int rows_left = ix >= 0 && ix < pl.W ? rows_in : 0;                            // and with this tap column
 
     // Rows no pixel of this thread needs, and pixels it does not have, read zeros.
@@ -149,8 +148,8 @@ band_cols_kernel(const __grid_constant__ BandColsPlan cp) {
     uint32_t rowbits = 0;
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
-        const int iy = y0 * S + D * (r - R);
-        const bool ok = rows_left > 0 && r <= S * (rows_left - 1) + K - 1 && iy >= 0 && iy < pl.H;
+        const int iy = y0 + D * (r - R);
+        const bool ok = rows_left > 0 && r < rows_left - 1 + K && iy >= 0 && iy < pl.H;
         rowbits |= ok ? 1u << r : 0u;
         rowoff[r] = ok ? (uint32_t)pip * (uint32_t)xplane + (uint32_t)(((iy - iy_lo) * pl.W + ix) * ES) : pl.zero_off + 16u;
         pin(rowoff[r]);
@@ -164,7 +163,7 @@ band_cols_kernel(const __grid_constant__ BandColsPlan cp) {
     // products with padding zeros, or of pixels outside the plane, in this thread / warp
     const bool edge = rows_left > 0 && (rowbits != (1u << NR) - 1u || rows_left < PH);
     const bool edge_warp = __any_sync(0xffffffffu, edge);
-    auto inside = [&](int k, int p) { return p < rows_left && ((rowbits >> (S * p + k)) & 1u) != 0u; };
+    auto inside = [&](int k, int p) { return p < rows_left && ((rowbits >> (p + k)) & 1u) != 0u; };
 
     if constexpr (MUL) {
         const T* cfp = reinterpret_cast<const T*>(pl.cf) + (long long)first_plane * KK;
@@ -247,8 +246,8 @@ band_cols_kernel(const __grid_constant__ BandColsPlan cp) {
                     if constexpr (MUL) c2 = lds64_pair(cf_s + 8u * k);
 #pragma unroll
                     for (int q = 0; q < 2; ++q) {
-                        prod2[q] = f2_pack(Mix<T>::fmaw(0, 0, v[S * 2 * q + k], g[2 * q], 0.f),
-                                           Mix<T>::fmaw(0, 0, v[S * (2 * q + 1) + k], g[2 * q + 1], 0.f));
+                        prod2[q] = f2_pack(Mix<T>::fmaw(0, 0, v[2 * q + k], g[2 * q], 0.f),
+                                           Mix<T>::fmaw(0, 0, v[2 * q + 1 + k], g[2 * q + 1], 0.f));
                         if constexpr (MUL) gsf2[k][q] = f2_fma(prod2[q], c2, gsf2[k][q]);
                         else gsf2[k][q] = f2_add(gsf2[k][q], prod2[q]);
                     }
@@ -276,7 +275,7 @@ band_cols_kernel(const __grid_constant__ BandColsPlan cp) {
                                     f2_unpack(sf2[k][p / 2], lo, hi);
                                     s = p & 1 ? hi : lo;
                                 }
-                                if (inside(k, p)) a = fmaf(Mix<T>::fmaw(0, 0, v[S * p + k], g[p], 0.f), s, a);
+                                if (inside(k, p)) a = fmaf(Mix<T>::fmaw(0, 0, v[p + k], g[p], 0.f), s, a);
                             }
                             sts32(mine + 4u * (uint32_t)(ch * K + k) * kColsRow, __float_as_uint(a));
                         }
@@ -383,7 +382,7 @@ struct BandColsLayout {
 inline bool band_cols_layout(const Problem& p, const BandColsSplit& s, BandColsLayout& l) {
     const int k = p.k, es = 2;
     const int out_rows = s.groups % p.d == 0 ? s.groups * kColsPixels : p.d * (kColsPixels - 1) + 1;
-    const long long rows = (long long)(out_rows - 1) * p.s + (k - 1) * p.d + 1;
+    const long long rows = (long long)(out_rows - 1) + (k - 1) * p.d + 1;
     const long long xrun = ((s.planes - 1) * (long long)p.H + (rows < p.H ? rows : p.H)) * p.W * es;
     const long long grun = ((s.planes - 1) * (long long)p.OH + (out_rows < p.OH ? out_rows : p.OH)) * p.OW * es;
     if (xrun > (32 << 10)) return false;
@@ -475,7 +474,7 @@ inline bool band_cols_split(const Problem& p, int sm_count, BandColsSplit& s) {
     return (long long)p.B * s.bands * s.chunks <= (1ll << 30);
 }
 
-template <typename T, int K, int D, int S, int MODE>
+template <typename T, int K, int D, int MODE>
 int band_cols_launch(const BandBwdArgs& a, const BandColsSplit& sp, cudaStream_t stream, int* launches) {
     constexpr int ES = (int)sizeof(T);
     const Problem& p = a.p;
@@ -505,7 +504,7 @@ int band_cols_launch(const BandBwdArgs& a, const BandColsSplit& sp, cudaStream_t
     pl.off_cf = l.off_cf; pl.off_part = l.off_part; pl.off_slot0 = l.off_slot0; pl.slot_stride = l.slot_stride;
     pl.zero_off = l.zero_off; pl.go_off = l.go_off; pl.n_slots = l.n_slots;
     cp.off_red = l.off_red; cp.part_stride = l.part_stride;
-    auto kern = band_cols_kernel<T, K, D, S, MODE>;
+    auto kern = band_cols_kernel<T, K, D, MODE>;
     static std::atomic<unsigned long long> opted_in{0};
     const unsigned long long bit = 1ull << (a.device & 63);
     if (!(opted_in.load(std::memory_order_acquire) & bit)) {

@@ -17,9 +17,9 @@
 // some 8 KB of distinct data in flight per SM and ran at a sixth of the memory's rate.  Pixels outside
 // the image are not read (zeros take their place).  The spatial filter is the same for all channels of a pixel: bias
 // and FilterNorm are applied once per pixel, by one thread, and the result is left in shared memory.
-// The sixteen layers of a ResNet-50 at 256 images of 224 x 224, float16: 822 -> 670 us.  Bound now by the 14 warps that an SM
-// holds at 128 registers (44 % of the issue slots), which meet at a barrier once per tile, and the FMA pipe (49 % of
-// the instructions are the FMAs).
+// The sixteen layers of a ResNet-50 at 256 images of 224 x 224, float16: 822 -> 670 us.  Bound now by the 16 warps that an SM
+// holds at 128 registers (stride 1 spills up to 36 bytes beyond them; at 64 channels 28 of 32 columns have pixels), which
+// meet at a barrier once per tile, and the FMA pipe.
 #include <atomic>
 
 #include "common.cuh"
@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(kNhwcThreads, 2) nhwc_forward_kernel(const __g
 
 // Partial sums of x over tiles of up to 196 pixels: partials[b][tile][c] (float), for the channel branch's
 // global average pool.  One CTA per (tile, sample).
-// A quarter of the image at least, so that small maps have CTAs enough for their loads to be in flight
+// A quarter of the image at most, so that small maps have CTAs enough for their loads to be in flight
 // (a tile is a CTA).  Float16, 256 images, us: (256,14x14) 10.5 -> 8.1, (512,14x14) 18.4 -> 11.9, (256,28x28) 24.3 -> 19.4,
 // (64,56x56) 26.7 -> 24.2.  Bound by the latency of the loads.
 constexpr int kPoolTile = 196;

@@ -121,3 +121,15 @@ def test_the_band_kernels_scratch_is_bounded(L):
         one = L.ddf_b200_backward_workspace(1, C, H, W, 5, 1, 1, 0, dtype, 0)
         need = L.ddf_b200_backward_workspace(B, C, H, W, 5, 1, 1, 0, dtype, 0)
         assert 0 < need <= max(256 << 20, one)
+
+
+@pytest.mark.parametrize("shape,cols", [((99, 456, 17, 22), False), ((51, 88, 26, 26), False), ((64, 256, 28, 28), False),
+                                        ((64, 512, 14, 14), True), ((99, 456, 17, 21), True)])
+def test_scratch_of_the_filter_gradients_form(shape, cols):
+    """Which form AUTO asks scratch for at k = 3, 2-byte types: the plane-streaming one where it measured faster.  (Shapes at
+    which the tap columns' need is the larger one.)"""
+    from ddfnet_b200 import _lib
+    L = _lib.load()
+    auto, stream = (int(L.ddf_b200_backward_workspace(*shape, 3, 1, 1, 0, 1, v)) for v in (_lib.VARIANT_AUTO, _lib.VARIANT_STREAM))
+    assert stream > 0
+    assert (auto == stream) is not cols

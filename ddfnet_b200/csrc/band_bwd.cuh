@@ -16,8 +16,8 @@
 // generic kernel's; Kahan sums and float partials gave 5.4e-8 (and 256 us instead of 300 at (2,256,200x300), now 280;
 // the generic kernels 3230).  For the 2-byte types the final rounding is 2^13 (f16) or 2^16 (bf16) times a
 // float's, and the sums are plain, over 64 channels at most before a compensated sum takes them: the error of
-// gsf against 64 bits is the generic kernel's to six digits (2.1e-4 f16, 1.66e-3 bf16; 77 drawn problems); Kahan's sum
-// took (2,256,200x300) bf16 from 180 to 265 us.
+// gsf against 64 bits is the generic kernel's to six digits (2.1e-4 f16, 1.66e-3 bf16; 77 drawn problems, on this form,
+// which they now take at stride 2 alone); Kahan's sum took (2,256,200x300) bf16 from 180 to 265 us.
 // gcf: the pixels of a warp are added as a tree, in plain float, the warps and bands compensated.  Error for
 // float against 64 bits 0.94 to 1.005 times the generic kernel's (which adds a thread's pixels compensated and
 // the threads plainly), for the 2-byte types the same to six digits.

@@ -10,12 +10,17 @@
 // grad-cf of a channel is a sum over lanes.  A warp leaves its lanes' values of four channels in shared memory
 // and adds them there, 16 bytes at a time: a third of the instructions of a butterfly of shuffles per channel.
 //
-// Bound by instruction issue: 98 a (channel, pixel) at k = 3, of which 36 are the arithmetic.  us, pixel form (band_bwd.cuh; at
+// Sums of gsf are plain over up to 64 channels; the pixel form's were at k = 5 over up to 24.  Relative error against 64 bits
+// over 76 problems (bands and whole planes, k = 3 and 5): gsf at most 1.0000001 times that form's, gcf the same to six digits;
+// at k = 5 290 of a million elements of gsf are not rounded as the exact value is, 244 there.  Not kept: chunks of 24
+// ((128,64,56x56) k = 5 384 -> 582 us), a second sum every 24 channels (4 to 12 % for a few of those elements).
+//
+// Bound by instruction issue: 90 a (channel, pixel) at k = 3, of which 36 are the arithmetic.  us, pixel form (band_bwd.cuh; at
 // 14 and 7 columns the plane-streaming form) -> this one: (2,256,200x300) bf16 179 -> 131, (8,48,150x130) f16 add 86.7 -> 43.8,
 // (16,64,99x51) d = 2 bf16 52.9 -> 38.2, (4,128,50x67) f16 23.0 -> 19.3, k = 5 (128,64,56x56) bf16 804 -> 384,
 // (8,96,75x101) f16 207 -> 130, (64,512,14x14) bf16 167 -> 124, (64,512,7x7) bf16 123 -> 64.  Registers: 64 (k = 3)
-// and 96 leave room for 32 and 20 warps; mul spills there, 84 and 64 bytes a thread loaded, k = 5 at 80 far more.  Not kept: scalar instead of two-wide sums
-// (154 at (2,256,200x300)).
+// and 96 leave room for 32 and 20 warps; mul spills there, 84 and 64 bytes a thread loaded, k = 5 at 80 far more.  Not kept:
+// scalar instead of two-wide sums (154 at (2,256,200x300)).
 #pragma once
 
 #include "band_bwd.cuh"

@@ -27,7 +27,8 @@
 // with cf (two-wide FMAs there wait for the pipe: 42.3 against 39.7 us at (2,128,200x280) bf16).  Float, add, and
 // filters normalised here: w = cf * sf (or cf + sf) and x * w, two pixels (p, p + 2) an instruction.
 //
-// What bounds it: instruction issue (9 FMAs of 10 instructions at k = 5, 18 of 51 per output at k = 3 in mul).  Half
+// What bounds it: instruction issue (38 instructions per output at k = 3 float32, 52 of which 18 are FMAs at 2-byte mul; at 300
+// columns half of the issue slots and two thirds of them are busy), and the latency of the few warps that fit.  Half
 // of what it issued before were products and selects that the compiler formed again in each pass (see pin); stores
 // under a predicate instead of a branch took another eighth.  Not all that is pinned stays in registers: -Xptxas -v shows
 // up to 132 bytes a thread spilled with MIX, 192 in grad-x and the normalised k = 5 without, 128 in the DIRECT forms (0 to 20 at

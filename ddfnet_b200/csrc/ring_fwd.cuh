@@ -242,7 +242,7 @@ struct RingPlane {
 // a tap.  With |cf| < 2^8 that is, over 25 taps, less than 2^-137, an eighth of half the smallest bfloat16's step.  While there
 // are larger ones in a stage a thread forms every result again, cf * sf first: the limit that it compares the sum of its
 // results' magnitudes with is then 0, not infinity.  (To ask which results are small enough to have lost something takes the
-// rest a twentieth: (64,256,28x28) 49 us; so 46.5 to 47.4, as without any of it.)
+// rest a twentieth: (64,256,28x28) 49 us; so it is 47.4, and 46.3 without any of it.)
 constexpr float kLargeCf = 256.f;
 
 // The same for k = 5, mul: the filter's tap rows come one after the other (its 25 values and the 50 words of the

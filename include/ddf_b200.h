@@ -251,10 +251,10 @@ int ddf_b200_backward(const void* go, const void* x, const void* cf, const void*
  * loads the library until the process exits.
  *
  *   - Problems of the plane-streaming kernels (ddf_b200_plan says STREAM) whose
- *     scratch need (what ddf_b200_backward_workspace reports) exceeds that limit
- *     are refused with DDF_B200_E_SCRATCH_LIMIT before anything is launched; any
- *     other problem runs, on the generic kernels where the array is too small for
- *     one sample.
+ *     scratch need there (what ddf_b200_backward_workspace reports for
+ *     DDF_B200_VARIANT_STREAM) exceeds that limit are refused with
+ *     DDF_B200_E_SCRATCH_LIMIT before anything is launched; any other problem runs, on
+ *     the generic kernels where the array is too small for one sample.
  *   - The call itself performs no cudaMalloc / cudaFree and uses no allocating
  *     library routine.
  *   - The first call on each device looks up the array's device address (one
